@@ -73,10 +73,83 @@ ZS_HD uint32_t rotr7(uint32_t x) {
   ZS_B3_G(v2, v7, v8, v13, m[s12], m[s13])                                                 \
   ZS_B3_G(v3, v4, v9, v14, m[s14], m[s15])
 
+#ifdef __CUDACC__
+// The first three words of hash2's prefix, kept from the compiler (see hash2).
+static __constant__ uint32_t kPairPrefix[3] = {0x2d67697au, 0x72617473u, 0x61703a6bu};
+#endif
+
+#ifdef __CUDA_ARCH__
+// The device's compression and what bounds it. A G is 14 operations: four xors and four
+// rotations, which only the ALU pipe executes (64 lanes per cycle and SM), and six
+// additions, which the FMA pipe (64 integer lanes too) executes as well when they have two
+// operands. Written plainly, a + b + m becomes one three-operand add on the ALU: 10 ALU
+// operations per G against 2 on the FMA pipe, and the hash kernels ran the ALU at 83-94 %.
+// add_fma keeps a + m out of it, as a * 1 + m with a 1 that the compiler cannot see (the
+// block's z extent: every launch of this library is one-dimensional), and the sum with b
+// is then a two-operand add: 8 ALU and 6 FMA operations per G. Measured on
+// one B200 over 148 x 16 CTAs of chained hashes: a compression of 16 unknown words 31.8 ->
+// 38.9 G/s, hash2 34.5 -> 38.9 G compressions/s (ALU bound of the 8: 41.6). Sending more
+// over (rotations as the halves of a wide product, c + d as a product) was slower in every
+// combination: a wide product takes two FMA slots and its halves an extra add.
+__device__ __forceinline__ uint32_t add_fma(uint32_t a, uint32_t m) {
+  uint32_t r;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(blockDim.z), "r"(m));
+  return r;
+}
+// ZX, ZY: the message word is zero.
+template <bool ZX, bool ZY>
+__device__ __forceinline__ void g_dev(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d, uint32_t mx, uint32_t my) {
+  a = ZX ? a + b : add_fma(a, mx) + b;
+  d = rotr16(d ^ a);
+  c = c + d;
+  b = rotr12(b ^ c);
+  a = ZY ? add_fma(a, b) : add_fma(a, my) + b;
+  d = rotr8(d ^ a);
+  c = c + d;
+  b = rotr7(b ^ c);
+}
+// Round R and those after it; ZERO: the set of message words known to be zero.
+template <uint32_t ZERO, int R>
+__device__ __forceinline__ void rounds_dev(uint32_t (&a)[4], uint32_t (&b)[4], uint32_t (&c)[4], uint32_t (&d)[4],
+                                           const uint32_t m[16]) {
+  if constexpr (R < 7) {
+    constexpr uint8_t s[7][16] = {{0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15},
+                                  {2, 6, 3, 10, 7, 0, 4, 13, 1, 11, 12, 5, 9, 14, 15, 8},
+                                  {3, 4, 10, 12, 13, 2, 7, 14, 6, 5, 9, 0, 11, 15, 8, 1},
+                                  {10, 7, 12, 9, 14, 3, 13, 15, 4, 0, 11, 2, 5, 8, 1, 6},
+                                  {12, 13, 9, 11, 15, 10, 14, 8, 7, 2, 5, 3, 0, 1, 6, 4},
+                                  {9, 14, 11, 5, 8, 12, 15, 1, 13, 3, 0, 10, 2, 6, 4, 7},
+                                  {11, 15, 5, 0, 1, 9, 8, 6, 14, 10, 2, 12, 3, 4, 7, 13}};
+#define ZS_B3_GD(i, j0, j1, j2, j3)                                                                             \
+  g_dev<((ZERO >> s[R][2 * i]) & 1) != 0, ((ZERO >> s[R][2 * i + 1]) & 1) != 0>(a[j0], b[j1], c[j2], d[j3],       \
+                                                                                m[s[R][2 * i]], m[s[R][2 * i + 1]]);
+    ZS_B3_GD(0, 0, 0, 0, 0)
+    ZS_B3_GD(1, 1, 1, 1, 1)
+    ZS_B3_GD(2, 2, 2, 2, 2)
+    ZS_B3_GD(3, 3, 3, 3, 3)
+    ZS_B3_GD(4, 0, 1, 2, 3)
+    ZS_B3_GD(5, 1, 2, 3, 0)
+    ZS_B3_GD(6, 2, 3, 0, 1)
+    ZS_B3_GD(7, 3, 0, 1, 2)
+#undef ZS_B3_GD
+    rounds_dev<ZERO, R + 1>(a, b, c, d, m);
+  }
+}
+#endif
+
 // Compression returning the 8-word chaining value (the first half of the output
 // state): cv <- compress(cv, m, counter = 0, block_len, flags)[0..8]. Every call on
-// this path uses counter 0 (single-chunk messages and parent nodes).
+// this path uses counter 0 (single-chunk messages and parent nodes). ZERO: the set of
+// message words that the caller knows to be zero (they cost nothing on the device).
+template <uint32_t ZERO = 0>
 ZS_HD void compress_cv(uint32_t cv[8], const uint32_t m[16], uint32_t block_len, uint32_t flags) {
+#ifdef __CUDA_ARCH__
+  uint32_t a[4] = {cv[0], cv[1], cv[2], cv[3]}, b[4] = {cv[4], cv[5], cv[6], cv[7]}, c[4] = {IV0, IV1, IV2, IV3},
+           d[4] = {0, 0, block_len, flags};
+  rounds_dev<ZERO, 0>(a, b, c, d, m);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) cv[i] = a[i] ^ c[i], cv[4 + i] = b[i] ^ d[i];
+#else
   uint32_t v0 = cv[0], v1 = cv[1], v2 = cv[2], v3 = cv[3], v4 = cv[4], v5 = cv[5], v6 = cv[6], v7 = cv[7];
   uint32_t v8 = IV0, v9 = IV1, v10 = IV2, v11 = IV3, v12 = 0, v13 = 0, v14 = block_len, v15 = flags;
   ZS_B3_ROUND(m, 0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15)
@@ -94,6 +167,7 @@ ZS_HD void compress_cv(uint32_t cv[8], const uint32_t m[16], uint32_t block_len,
   cv[5] = v5 ^ v13;
   cv[6] = v6 ^ v14;
   cv[7] = v7 ^ v15;
+#endif
 }
 
 // Full compression with a 64-bit counter and the 16-word output (host transcript).
@@ -175,7 +249,7 @@ ZS_HD void iv(uint32_t cv[8]) {
 ZS_HD void hash_qm31(const qm31& v, uint32_t out[8]) {
   uint32_t m[16] = {v.a.a, v.a.b, v.b.a, v.b.b, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   iv(out);
-  compress_cv(out, m, 16, CHUNK_START | CHUNK_END | ROOT);
+  compress_cv<0xfff0u>(out, m, 16, CHUNK_START | CHUNK_END | ROOT);
 }
 
 // hash2 (src/core/hash/hash.zig:17-25): Blake3("zig-stark:pair" || L || R), 78 bytes
@@ -184,9 +258,15 @@ ZS_HD void hash_qm31(const qm31& v, uint32_t out[8]) {
 ZS_HD void hash2(const uint32_t l[8], const uint32_t r[8], uint32_t out[8]) {
   // "zig-stark:pair" = 7a 69 67 2d 73 74 61 72 6b 3a 70 61 69 72
   uint32_t m[16];
+#ifdef __CUDA_ARCH__
+  // Opaque: an add of a known word becomes a three-operand add again (a compression of
+  // this block 35.7 G/s instead of 38.6).
+  m[0] = kPairPrefix[0], m[1] = kPairPrefix[1], m[2] = kPairPrefix[2];
+#else
   m[0] = 0x2d67697au;  // "zig-"
   m[1] = 0x72617473u;  // "star"
   m[2] = 0x61703a6bu;  // "k:pa"
+#endif
   // bytes 12,13 = "ir"; then L starts at byte 14 (2 bytes into word 3)
   m[3] = 0x00007269u | (l[0] << 16);
 #pragma unroll
@@ -205,7 +285,7 @@ ZS_HD void hash2(const uint32_t l[8], const uint32_t r[8], uint32_t out[8]) {
   m2[3] = r[7] >> 16;
 #pragma unroll
   for (int k = 4; k < 16; ++k) m2[k] = 0;
-  compress_cv(out, m2, 14, CHUNK_END | ROOT);
+  compress_cv<0xfff0u>(out, m2, 14, CHUNK_END | ROOT);
 }
 
 // Blake3 of a single-chunk message given as `nwords` little-endian u32 words

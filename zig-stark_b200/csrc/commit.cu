@@ -50,6 +50,10 @@ CommitPlan::CommitPlan(uint32_t C_, unsigned L_, unsigned B_, unsigned F_) : C(C
     layer_trees[i].log_n = L + B - i;
     alloc((void**)&layer_trees[i].words, DeviceTree::words_for(L + B - i) * sizeof(uint32_t));
   }
+  alloc((void**)&done, (F + 1) * sizeof(uint32_t));
+  ZS_CUDA(cudaMemsetAsync(done, 0, (F + 1) * sizeof(uint32_t), setup));
+  row_tree.done = done;
+  for (unsigned i = 0; i < F; ++i) layer_trees[i].done = done + 1 + i;
   alphas.assign(F, qzero());
   const char* env = std::getenv("ZS_NO_GRAPH");
   use_graph = !(env && env[0] == '1');
@@ -65,6 +69,7 @@ CommitPlan::~CommitPlan() {
   cudaFree(gammas);
   for (auto* p : layers) cudaFree(p);
   cudaFree(row_tree.words);
+  cudaFree(done);
   for (auto& t : layer_trees) cudaFree(t.words);
   small.reset();
   big.reset();

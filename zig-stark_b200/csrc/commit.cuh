@@ -25,6 +25,7 @@ struct CommitPlan {
   std::vector<qm31*> layers;    // F + 1 fold layers; layers[0] = g
   DeviceTree row_tree;
   std::vector<DeviceTree> layer_trees;  // trees of layers 0 .. F-1
+  uint32_t* done = nullptr;             // the trees' counters: row tree, then the layers
 
   CommitPlan(uint32_t C, unsigned L, unsigned B, unsigned F);
   ~CommitPlan();

@@ -1,12 +1,10 @@
 // Merkle trees on the device (src/core/merkle/merkle.zig:17-68).
 //
-// Two kinds of kernels, both without block-wide barriers so every lane stays busy:
-//   leaf kernels: one thread per leaf, one Blake3 compression chain in registers
-//     (hashQM31 = 1 compression, hashM31s of a 64-value row = 4);
-//   k_tree_up: one thread per 2^s consecutive digests of a level (s <= 3) folds them
-//     into its own s-level subtree with hash2 (= Blake3("zig-stark:pair" || L || R),
-//     two compressions), writing every node, because openings need all levels.
-// A tree over 2^22 leaves therefore takes one leaf launch and eight tree launches.
+// A leaf is one Blake3 compression (hashQM31) or a few (hashM31s of a row: 4 for 64
+// values), a node two (hash2 = Blake3("zig-stark:pair" || L || R), 78 bytes), each in one
+// thread's registers. Every node is written, because openings need all levels.
+//   k_row_leaves: one thread per row;
+//   k_tree: subtrees in CTAs, level by level, up to the root.
 #include <algorithm>
 
 #include "blake3.cuh"
@@ -29,49 +27,7 @@ __device__ __forceinline__ void get_digest(const uint32_t* tree_words, size_t di
   o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
 }
 
-// The subtree over CNT (2, 4 or 8) consecutive digests of `level0` starting at index
-// `first` (a multiple of CNT): digests arrive in order from `next(k, d)`, a stack of
-// pending left siblings merges them, and every new node is written.
-template <int CNT, typename Next>
-__device__ __forceinline__ void thread_subtree(Next&& next, uint32_t* tree_words, unsigned log_n, unsigned level0,
-                                               uint64_t first) {
-  const size_t N2 = (size_t)2 << log_n;
-  uint32_t stk[3][8];
-#pragma unroll
-  for (int k = 0; k < CNT; ++k) {
-    uint32_t cur[8];
-    next(k, cur);
-    int depth = __popc(k) ;  // pending left siblings before merging leaf k (k's set bits)
-#pragma unroll
-    for (int b = 0; (1 << (b + 1)) <= CNT; ++b) {
-      if (((k >> b) & 1) == 0) break;
-      --depth;
-      uint32_t o[8];
-      b3::hash2(stk[depth], cur, o);
-#pragma unroll
-      for (int w = 0; w < 8; ++w) cur[w] = o[w];
-      const unsigned lvl = level0 + b + 1;
-      put_digest(tree_words, (N2 - (N2 >> lvl)) + ((first + k) >> (b + 1)), cur);
-    }
-    if (k + 1 < CNT) {
-#pragma unroll
-      for (int w = 0; w < 8; ++w) stk[depth][w] = cur[w];
-    }
-  }
-}
 }  // namespace
-
-// hashQM31 leaves (src/m31/hash.zig:33-37).
-// blockIdx.y selects the tree of a set (its values `v_stride` elements after the previous).
-__global__ void __launch_bounds__(kThreads) k_qm31_leaves(const qm31* __restrict__ vals, size_t v_stride,
-                                                          TreeSet ts, uint64_t n) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint4 raw = __ldg(reinterpret_cast<const uint4*>(vals + blockIdx.y * v_stride) + i);
-  uint32_t o[8];
-  b3::hash_qm31(qmake(raw.x, raw.y, raw.z, raw.w), o);
-  put_digest(ts.words[blockIdx.y], i, o);
-}
 
 // Row leaves hashM31s(col_0[r], ..., col_{C-1}[r]) (src/m31/hash.zig:15-25), and
 // optionally g[r] = sum_c gammas[c] * col_c[r] with its hashQM31 leaf. The four
@@ -152,120 +108,181 @@ __global__ void __launch_bounds__(kThreads) k_row_leaves(const uint32_t* __restr
   }
 }
 
-// Levels level0+1 .. level0+log2(CNT): thread t folds digests [t*CNT, (t+1)*CNT) of level0.
-template <int CNT>
-__global__ void __launch_bounds__(kThreads) k_tree_up(TreeSet ts, unsigned log_n, unsigned level0) {
-  uint32_t* tree_words = ts.words[blockIdx.y];
-  const uint64_t count = ((uint64_t)1 << (log_n - level0)) / CNT;
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  const size_t N2 = (size_t)2 << log_n;
-  const uint32_t* src = tree_words + 8 * (N2 - (N2 >> level0));
-  const uint64_t first = t * CNT;
-  thread_subtree<CNT>([&](int k, uint32_t d[8]) { get_digest(src, first + k, d); }, tree_words, log_n, level0, first);
-}
+// The trees of one launch.
+struct TreeSet {
+  uint32_t* words[kTreeBatch];
+  uint32_t* done[kTreeBatch];
+  const qm31* vals[kTreeBatch];  // the leaves' values (LEAF)
+};
 
-// Subtrees of a tree in CTAs: CTA b takes the 2^levels <= kTopMax digests
-// [b 2^levels, (b + 1) 2^levels) of level `level0` and hashes the `levels` levels above
-// them in shared memory, one node per thread, a barrier between levels. These levels
-// are latency-bound (few nodes, each a chain of two compressions), so one launch
-// replaces one launch per level; with levels = log_n - level0 one CTA finishes the tree.
-constexpr unsigned kTopMax = 1024;
-__global__ void __launch_bounds__(kTopMax / 2) k_tree_block(TreeSet ts, unsigned log_n, unsigned level0,
-                                                            unsigned levels) {
-  __shared__ uint32_t s[kTopMax][8];
-  uint32_t* tree_words = ts.words[blockIdx.y];
+// Levels level0 + 1 .. level0 + levels over the 2^span digests [b 2^span, (b + 1) 2^span)
+// of level `level0` per CTA b (levels <= span), a barrier between levels; LEAF: the CTA
+// hashes those digests from the values first (hashQM31, level0 = 0). With `top` (levels =
+// span) the CTA that finishes the tree's last subtree goes on from the subtrees' roots to
+// the tree's root: each CTA counts itself in `done` after its root is visible, nobody
+// waits. All of a CTA's levels run through one loop with one copy of hash2: a copy is 26 KB
+// of instructions, and the seven copies of an earlier kernel (a 3-level subtree per
+// thread) ran at the rate of the instruction cache, not of the ALU.
+// Shared memory: the digests of the last level, two levels in turn.
+constexpr unsigned kTreeThreads = 256;
+template <bool LEAF>
+__global__ void __launch_bounds__(kTreeThreads, LEAF ? 4 : 3) k_tree(const __grid_constant__ TreeSet ts, unsigned log_n,
+                                                       unsigned level0, unsigned span, unsigned levels,
+                                                       unsigned top) {
+  extern __shared__ uint4 s_dig[];
+  uint32_t* words = ts.words[blockIdx.y];
   const size_t N2 = (size_t)2 << log_n;
-  uint32_t cnt = 1u << levels;
-  const uint32_t first = blockIdx.x << levels;  // first digest of this CTA at level0
-  const uint32_t* src = tree_words + 8 * (N2 - (N2 >> level0));
-  for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) get_digest(src, first + i, s[i]);
-  __syncthreads();
-  for (unsigned lvl = level0 + 1; lvl <= level0 + levels; ++lvl) {
-    cnt >>= 1;
-    uint32_t o[8];
-    const bool active = threadIdx.x < cnt;
-    if (active) {
-      b3::hash2(s[2 * threadIdx.x], s[2 * threadIdx.x + 1], o);
-      put_digest(tree_words, (N2 - (N2 >> lvl)) + (first >> (lvl - level0)) + threadIdx.x, o);
+  size_t cta = blockIdx.x;
+#pragma unroll 1
+  for (;;) {
+    uint32_t from = 0, to = 0;  // offsets of the two levels in s_dig, in digests
+#pragma unroll 1
+    for (unsigned l = 1; l <= levels; ++l) {
+      const uint32_t cnt = 1u << (span - l);
+      const size_t dst = (N2 - (N2 >> (level0 + l))) + (cta << (span - l));
+      const bool leaves = LEAF && level0 == 0 && l == 1;
+      // The children's digests (or their leaves' values) in `q`, loaded one node ahead: warps
+      // that all hash alike reach their loads together, and nothing else covers them.
+      const uint4* src =
+          leaves ? reinterpret_cast<const uint4*>(ts.vals[blockIdx.y]) + (cta << span)
+          : l == 1 ? reinterpret_cast<const uint4*>(words + 8 * ((N2 - (N2 >> level0)) + (cta << span)))
+                   : s_dig + 2 * from;
+      uint4 q[4];
+      auto load = [&](uint32_t e) {
+        if (leaves) {
+          q[0] = __ldg(src + 2 * e), q[1] = __ldg(src + 2 * e + 1);
+        } else if (l == 1) {  // past L1: other CTAs may have written them in this launch
+#pragma unroll
+          for (int k = 0; k < 4; ++k) q[k] = __ldcg(src + 4 * e + k);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) q[k] = src[4 * e + k];
+        }
+      };
+      if (threadIdx.x < cnt) load(threadIdx.x);
+#pragma unroll 1
+      for (uint32_t e = threadIdx.x; e < cnt; e += blockDim.x) {
+        uint32_t lc[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w};
+        uint32_t rc[8] = {q[2].x, q[2].y, q[2].z, q[2].w, q[3].x, q[3].y, q[3].z, q[3].w};
+        if (e + blockDim.x < cnt) load(e + blockDim.x);
+        uint32_t o[8];
+        if (leaves) {  // hash the two leaves first, the second into rc
+          const size_t leaf = (cta << span) + 2 * (size_t)e;
+          uint32_t v[4] = {lc[0], lc[1], lc[2], lc[3]};
+#pragma unroll 1
+          for (int k = 0; k < 2; ++k) {
+            b3::hash_qm31(qmake(v[0], v[1], v[2], v[3]), rc);
+            put_digest(words, leaf + k, rc);
+            if (k == 0) {
+#pragma unroll
+              for (int w = 0; w < 4; ++w) v[w] = lc[4 + w];
+#pragma unroll
+              for (int w = 0; w < 8; ++w) lc[w] = rc[w];
+            }
+          }
+        }
+        b3::hash2(lc, rc, o);
+        put_digest(words, dst + e, o);
+        if (l < levels) put_digest(reinterpret_cast<uint32_t*>(s_dig), to + e, o);
+      }
+      __syncthreads();
+      from = to;
+      to = to == 0 ? 1u << (span - 1) : 0;
     }
-    __syncthreads();  // every child is read before a parent overwrites it
-    if (active)
-      for (int w = 0; w < 8; ++w) s[threadIdx.x][w] = o[w];
+    if (!top || level0 + levels == log_n) return;
+    uint32_t& s_last = reinterpret_cast<uint32_t*>(s_dig)[0];  // the digests there are done with
+    if (threadIdx.x == 0) {  // wrote the subtree's root
+      __threadfence();
+      const uint32_t n_ctas = 1u << (log_n - level0 - levels);
+      const bool last = atomicAdd(ts.done[blockIdx.y], 1u) == n_ctas - 1;
+      if (last) {
+        *ts.done[blockIdx.y] = 0;
+        __threadfence();
+      }
+      s_last = last;
+    }
     __syncthreads();
+    const bool go_on = s_last != 0;
+    __syncthreads();  // read before the digests overwrite it
+    if (!go_on) return;
+    level0 += levels;
+    span = levels = log_n - level0;
+    cta = 0;
   }
 }
 
-static unsigned log2u(uint64_t x) {
-  unsigned l = 0;
-  while (((uint64_t)1 << l) < x) ++l;
-  return l;
-}
-
-static void launch_up(const TreeSet& ts, uint32_t count, unsigned log_n, unsigned lvl, unsigned s,
-                      cudaStream_t st) {
-  const uint64_t threads_total = ((uint64_t)1 << (log_n - lvl)) >> s;
-  const dim3 grid((unsigned)((threads_total + kThreads - 1) / kThreads), count);
-  switch (s) {
-    case 1: k_tree_up<2><<<grid, kThreads, 0, st>>>(ts, log_n, lvl); break;
-    case 2: k_tree_up<4><<<grid, kThreads, 0, st>>>(ts, log_n, lvl); break;
-    default: k_tree_up<8><<<grid, kThreads, 0, st>>>(ts, log_n, lvl); break;
+// The launches that take trees of 2^log_n leaves from level `level0` (its digests, or with
+// leaves to hash first) to their roots.
+namespace {
+struct TreeLaunch {
+  unsigned level0, span, levels, threads;
+  unsigned top_levels;  // levels that the last CTA adds
+  size_t smem() const {  // two levels in turn of the wider of the subtrees and the top
+    const unsigned w = levels < 2 && top_levels == 0 ? 0 : std::max(span, top_levels);
+    return w < 2 ? 0 : ((size_t)3 << (w - 2)) * 32;
   }
-}
+};
 
-// Three levels per launch while a level still gives every SM plenty of threads
-// (one thread chains 7 nodes = 14 compressions); above that one level per launch,
-// so the narrow top of the tree costs one hash2 of latency per level.
-static unsigned levels_per_launch(unsigned log_n, unsigned lvl) {
-  const unsigned remaining = log_n - lvl;
-  if (remaining >= 3 && remaining >= 3 + 15) return 3;  // >= 2^15 threads of 8-node subtrees
-  return 1;
-}
-
-static void finish_set(const TreeSet& ts, uint32_t count, unsigned log_n, unsigned from_level, cudaStream_t st) {
-  unsigned lvl = from_level;
-  while (lvl < log_n) {
-    const unsigned rem = log_n - lvl;
-    if (levels_per_launch(log_n, lvl) == 3) {  // wide levels: subtrees per thread
-      launch_up(ts, count, log_n, lvl, 3, st);
-      lvl += 3;
-      continue;
+// While the trees' digests fill the device a launch is bound by the ALU: it stops after
+// three or four levels, before a CTA's levels become narrower than its warps, and its
+// CTAs are the larger the more there are. From there on the levels are a chain of two
+// compressions each (1.3 us), so one launch takes 2^8 digests per CTA, one warp per
+// scheduler at its widest level, and its last CTA the levels above. Measured over spans of
+// 8..11, 2..11 levels and 128 or 256 threads, with leaves: one tree of 2^22 372 us (544 us
+// in narrow launches only, 562 us with three levels per thread), 2^20 116 us (126 us with
+// spans of 2^11), 2^18 53 us (60 us narrow), 2^14 27 us, 2^12 24.7 us; 32 trees of 2^17
+// 365 us (537 us narrow), 12 of 2^14 43 us (51 us narrow, 47 us with spans of 2^11).
+std::vector<TreeLaunch> plan_tree(unsigned log_n, unsigned level0, uint32_t count) {
+  std::vector<TreeLaunch> v;
+  while (level0 < log_n) {
+    const unsigned rem = log_n - level0;
+    const uint64_t digests = (uint64_t)count << rem;
+    TreeLaunch t{level0, 0, 0, 0, 0};
+    if (rem >= 13 && digests >= ((uint64_t)1 << 21)) {
+      t.span = 11, t.levels = 4, t.threads = 256;
+    } else if (rem >= 13 && digests >= ((uint64_t)1 << 20)) {
+      t.span = 10, t.levels = 4, t.threads = 256;
+    } else if (rem >= 13 && digests >= ((uint64_t)1 << 17)) {
+      t.span = 9, t.levels = 3, t.threads = 128;
+    } else {
+      t.span = t.levels = std::min(rem, 8u), t.threads = 128;
+      if (rem - t.levels <= 8) t.top_levels = rem - t.levels;
     }
-    const unsigned levels = rem < 10 ? rem : 10;  // narrow levels: subtrees per CTA
-    k_tree_block<<<dim3(1u << (rem - levels), count), kTopMax / 2, 0, st>>>(ts, log_n, lvl, levels);
-    lvl += levels;
+    v.push_back(t);
+    level0 += t.levels + t.top_levels;
+  }
+  return v;
+}
+
+void finish_set(const TreeSet& ts, uint32_t count, unsigned log_n, unsigned level0, bool leaves, cudaStream_t st) {
+  if (leaves && log_n == 0) throw Error(ZS_EGENERIC, "a tree of one leaf");
+  for (const TreeLaunch& t : plan_tree(log_n, level0, count)) {
+    const dim3 grid(1u << (log_n - t.level0 - t.span), count);
+    if (leaves && t.level0 == 0)
+      k_tree<true><<<grid, t.threads, t.smem(), st>>>(ts, log_n, t.level0, t.span, t.levels, t.top_levels > 0);
+    else
+      k_tree<false><<<grid, t.threads, t.smem(), st>>>(ts, log_n, t.level0, t.span, t.levels, t.top_levels > 0);
   }
   ZS_CUDA(cudaGetLastError());
 }
 
-static TreeSet single(const DeviceTree& tree) {
+TreeSet single(const DeviceTree& tree, const qm31* vals = nullptr) {
   TreeSet ts{};
-  ts.words[0] = tree.words;
+  ts.words[0] = tree.words, ts.done[0] = tree.done, ts.vals[0] = vals;
   return ts;
 }
+}  // namespace
 
 void tree_finish(DeviceTree& tree, unsigned from_level, cudaStream_t st) {
-  finish_set(single(tree), 1, tree.log_n, from_level, st);
+  finish_set(single(tree), 1, tree.log_n, from_level, false, st);
 }
 
 uint32_t tree_finish_launches(unsigned log_n, unsigned from_level) {
-  uint32_t k = 0;
-  for (unsigned lvl = from_level; lvl < log_n; ++k) {
-    const unsigned rem = log_n - lvl;
-    lvl += levels_per_launch(log_n, lvl) == 3 ? 3 : (rem < 10 ? rem : 10);
-  }
-  return k;
+  return (uint32_t)plan_tree(log_n, from_level, 1).size();
 }
 
 void build_qm31_tree(const qm31* d_values, DeviceTree& tree, cudaStream_t st) {
-  build_qm31_leaves(d_values, tree, st);
-  tree_finish(tree, 0, st);
-}
-
-void build_qm31_leaves(const qm31* d_values, DeviceTree& tree, cudaStream_t st) {
-  const uint64_t n = (uint64_t)1 << tree.log_n;
-  k_qm31_leaves<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(d_values, 0, single(tree), n);
-  ZS_CUDA(cudaGetLastError());
+  finish_set(single(tree, d_values), 1, tree.log_n, 0, true, st);
 }
 
 void build_qm31_trees(const qm31* d_values, size_t v_stride, DeviceTree* const* trees, uint32_t count,
@@ -276,13 +293,10 @@ void build_qm31_trees(const qm31* d_values, size_t v_stride, DeviceTree* const* 
     TreeSet ts{};
     for (uint32_t k = 0; k < c; ++k) {
       if (trees[t0 + k]->log_n != log_n) throw Error(ZS_EGENERIC, "build_qm31_trees: trees of different sizes");
-      ts.words[k] = trees[t0 + k]->words;
+      ts.words[k] = trees[t0 + k]->words, ts.done[k] = trees[t0 + k]->done;
+      ts.vals[k] = d_values + (size_t)(t0 + k) * v_stride;
     }
-    const uint64_t n = (uint64_t)1 << log_n;
-    k_qm31_leaves<<<dim3((unsigned)((n + kThreads - 1) / kThreads), c), kThreads, 0, st>>>(
-        d_values + (size_t)t0 * v_stride, v_stride, ts, n);
-    ZS_CUDA(cudaGetLastError());
-    finish_set(ts, c, log_n, 0, st);
+    finish_set(ts, c, log_n, 0, true, st);
   }
 }
 

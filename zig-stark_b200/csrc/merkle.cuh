@@ -12,7 +12,9 @@ namespace zs {
 struct DeviceTree {
   unsigned log_n = 0;
   uint32_t* words = nullptr;  // (2N - 1) * 8 words
-  bool owned = false;
+  // Finished subtrees of a launch in which the last one's CTA goes on to the top
+  // (k_tree): one word, zero before the tree's first launch and again after each.
+  uint32_t* done = nullptr;
   static size_t words_for(unsigned log_n) { return (((size_t)2 << log_n) - 1) * 8; }
   size_t level_offset(unsigned k) const {
     const size_t N2 = (size_t)2 << log_n;
@@ -26,20 +28,13 @@ struct DeviceTree {
 // Leaves hashQM31(values[i]) for 2^log_n QM31 values plus the whole tree.
 void build_qm31_tree(const qm31* d_values, DeviceTree& tree, cudaStream_t st);
 
-// Device tree pointers of a set of trees built by the same launches (blockIdx.y picks
-// the tree): small trees are latency-bound, so one launch per level range serves all.
+// Most trees that one launch builds (blockIdx.y picks the tree).
 constexpr uint32_t kTreeBatch = 64;
-struct TreeSet {
-  uint32_t* words[kTreeBatch];
-};
 // build_qm31_tree for `count` trees of one size: tree k over the values at
 // d_values + k * v_stride.
 void build_qm31_trees(const qm31* d_values, size_t v_stride, DeviceTree* const* trees, uint32_t count,
                       cudaStream_t st);
-// Leaves only (level 0) of build_qm31_tree.
-void build_qm31_leaves(const qm31* d_values, DeviceTree& tree, cudaStream_t st);
-// Completes levels above `from_level` (levels <= from_level must be written), three
-// levels per launch.
+// Completes the levels above `from_level` (levels <= from_level must be written).
 void tree_finish(DeviceTree& tree, unsigned from_level, cudaStream_t st);
 // Number of launches tree_finish makes.
 uint32_t tree_finish_launches(unsigned log_n, unsigned from_level);

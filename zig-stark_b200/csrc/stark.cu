@@ -420,11 +420,19 @@ Digest root_of(const DeviceTree& t, cudaStream_t st) {
 struct OwnedTree {
   DeviceTree t;
   cudaStream_t st;
-  OwnedTree(unsigned log_n, cudaStream_t s) : st(s) {
-    t.log_n = log_n;
+  OwnedTree(unsigned log_n, uint32_t* done, cudaStream_t s) : st(s) {
+    t.log_n = log_n, t.done = done;
     ZS_CUDA(cudaMallocAsync((void**)&t.words, DeviceTree::words_for(log_n) * sizeof(uint32_t), s));
   }
   ~OwnedTree() { cudaFreeAsync(t.words, st); }
+};
+
+// The counters of `count` trees (DeviceTree::done), zeroed on the stream.
+struct TreeCounters {
+  DevBuf<uint32_t> d;
+  TreeCounters(size_t count, cudaStream_t s) : d(count, s) {
+    ZS_CUDA(cudaMemsetAsync(d.p, 0, count * sizeof(uint32_t), s));
+  }
 };
 
 // Size-only tables (NTT twiddles, powers of FRI_OFFSET, fold tables) of sizes up to
@@ -689,8 +697,9 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   const NttTables& big = ntt_tables(lN, st, big_own);
   const qm31* offset_pows = offset_powers(tl, st, pows_own);
   DevBuf<qm31> vals((size_t)ncol * n, st), coeffs((size_t)ncol * n, st), cw((size_t)ncol * N, st);
+  TreeCounters done((size_t)ncol + 1 + L, st);  // the columns', the quotient's and the FRI layers' trees
   std::vector<std::unique_ptr<OwnedTree>> trees;
-  for (uint32_t j = 0; j < ncol; ++j) trees.push_back(std::make_unique<OwnedTree>(lN, st));
+  for (uint32_t j = 0; j < ncol; ++j) trees.push_back(std::make_unique<OwnedTree>(lN, done.d.p + j, st));
   {
     // Columns [pre | main] in groups: group g+1 is packed on the host and copied on a
     // copy stream while the LDE of group g runs on `st` and its trees on a side stream
@@ -863,7 +872,7 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
     k_quotient<<<(N + kT - 1) / kT, kT, 0, st>>>(cw.p, q.p, big.fwd, d_kc.p, zh_tab.p, per_tab.p);
   }
   ZS_CUDA(cudaGetLastError());
-  OwnedTree qtree(lN, st);
+  OwnedTree qtree(lN, done.d.p + ncol, st);
   build_qm31_tree(q.p, qtree.t, st);
   const Digest qroot = root_of(qtree.t, st);
   ch.absorb(qroot);
@@ -918,7 +927,7 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   std::unique_ptr<FoldTables> ftabs_own;
   const FoldTables& ftabs = fold_tables(lN, st, ftabs_own);
   std::vector<std::unique_ptr<OwnedTree>> ftrees;
-  for (unsigned i = 0; i < L; ++i) ftrees.push_back(std::make_unique<OwnedTree>(lN - i, st));
+  for (unsigned i = 0; i < L; ++i) ftrees.push_back(std::make_unique<OwnedTree>(lN - i, done.d.p + ncol + 1 + i, st));
   // The commit phase (fri.zig:195-227) runs without host round trips: per layer a
   // one-thread kernel absorbs the layer's root into the device copy of the transcript
   // and samples the folding challenge, which the fold reads from device memory. The
@@ -1109,8 +1118,9 @@ std::vector<uint8_t> commit_columns(const uint8_t* cols_b, size_t cols_len, unsi
   // trees of up to 1 GiB in all are built together, then their roots read back
   const size_t tree_bytes = DeviceTree::words_for(lN) * sizeof(uint32_t);
   const uint32_t per = (uint32_t)std::max<size_t>(1, std::min<size_t>(kTreeBatch, ((size_t)1 << 30) / tree_bytes));
+  TreeCounters done(std::min(per, C), st);
   std::vector<std::unique_ptr<OwnedTree>> trees;
-  for (uint32_t j = 0; j < std::min(per, C); ++j) trees.push_back(std::make_unique<OwnedTree>(lN, st));
+  for (uint32_t j = 0; j < std::min(per, C); ++j) trees.push_back(std::make_unique<OwnedTree>(lN, done.d.p + j, st));
   for (uint32_t c0 = 0; c0 < C; c0 += per) {
     const uint32_t c = std::min(per, C - c0);
     build_qm31_trees(cw.p + (size_t)c0 * N, N, tree_ptrs(trees, 0, c).data(), c, st);
