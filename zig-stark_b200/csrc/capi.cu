@@ -6,10 +6,12 @@
 #include <mutex>
 #include <new>
 #include <thread>
+#include <vector>
 
 #include "../../include/zs_m31.h"
 #include "circle.cuh"
 #include "commit.cuh"
+#include "staging.cuh"
 #include "stark.cuh"
 #include "verify.cuh"
 
@@ -143,13 +145,18 @@ int32_t zs_m31_commit_plan_results(zs_commit_plan* plan, void* stream, uint8_t* 
     if (!plan) throw Error(ZS_EMALFORMED, "null plan");
     CommitPlan& p = *plan->plan;
     cudaStream_t st = (cudaStream_t)stream;
-    if (lde_root) ZS_CUDA(cudaMemcpyAsync(lde_root, p.row_tree.root(), 32, cudaMemcpyDeviceToHost, st));
-    if (layer_roots)
-      for (unsigned i = 0; i < p.F; ++i)
-        ZS_CUDA(cudaMemcpyAsync(layer_roots + 32 * i, p.layer_trees[i].root(), 32, cudaMemcpyDeviceToHost, st));
-    if (final_layer)
-      ZS_CUDA(cudaMemcpyAsync(final_layer, p.layers[p.F], ((size_t)1 << (p.L + p.B - p.F)) * sizeof(qm31),
-                              cudaMemcpyDeviceToHost, st));
+    // The roots lie in one buffer; with a small final layer they come back through pinned
+    // memory with one wait (a pageable copy is a wait of its own, about 8 us each).
+    const size_t final_bytes = ((size_t)1 << (p.L + p.B - p.F)) * sizeof(qm31);
+    const bool final_small = final_bytes <= ((size_t)256 << 10);
+    if (final_layer && !final_small)
+      ZS_CUDA(cudaMemcpyAsync(final_layer, p.layers[p.F], final_bytes, cudaMemcpyDeviceToHost, st));
+    PinnedScope pinned(st);
+    std::vector<D2H> back;
+    if (lde_root) back.push_back({lde_root, p.roots, 32});
+    if (layer_roots && p.F > 0) back.push_back({layer_roots, p.roots + 8, (size_t)32 * p.F});
+    if (final_layer && final_small) back.push_back({final_layer, p.layers[p.F], final_bytes});
+    d2h_many(back.data(), back.size(), st);
     ZS_CUDA(cudaStreamSynchronize(st));
   });
 }

@@ -36,24 +36,36 @@ CommitPlan::CommitPlan(uint32_t C_, unsigned L_, unsigned B_, unsigned F_) : C(C
   small = std::make_unique<CircleDomain>(L, setup);
   big = std::make_unique<CircleDomain>(L + B, setup);
   tabs = std::make_unique<FoldTables>(L + B, setup);
-  auto alloc = [&](void** p, size_t bytes) { ZS_CUDA(cudaMallocAsync(p, bytes, setup)); };
-  alloc((void**)&trace, C * n * sizeof(uint32_t));
-  alloc((void**)&lde, C * N * sizeof(uint32_t));
-  alloc((void**)&scratch, lde_scratch_words(L, B, C) * sizeof(uint32_t));
-  alloc((void**)&gammas, C * sizeof(qm31));
   layers.resize(F + 1);
-  for (unsigned i = 0; i <= F; ++i) alloc((void**)&layers[i], (N >> i) * sizeof(qm31));
-  row_tree.log_n = L + B;
-  alloc((void**)&row_tree.words, DeviceTree::words_for(L + B) * sizeof(uint32_t));
   layer_trees.resize(F);
-  for (unsigned i = 0; i < F; ++i) {
-    layer_trees[i].log_n = L + B - i;
-    alloc((void**)&layer_trees[i].words, DeviceTree::words_for(L + B - i) * sizeof(uint32_t));
-  }
-  alloc((void**)&done, (F + 1) * sizeof(uint32_t));
+  // Every buffer of the plan lies in one allocation: a stream-ordered pool that keeps no
+  // memory maps each block anew, so a plan of forty small blocks took longer to make than
+  // one large one.
+  struct Part {
+    void** p;
+    size_t bytes;
+  };
+  std::vector<Part> parts = {{(void**)&trace, C * n * sizeof(uint32_t)},
+                             {(void**)&lde, C * N * sizeof(uint32_t)},
+                             {(void**)&scratch, lde_scratch_words(L, B, C) * sizeof(uint32_t)},
+                             {(void**)&gammas, C * sizeof(qm31)},
+                             {(void**)&row_tree.words, DeviceTree::words_for(L + B) * sizeof(uint32_t)},
+                             {(void**)&done, (F + 1) * sizeof(uint32_t)},
+                             {(void**)&roots, (F + 1) * 32}};
+  for (unsigned i = 0; i <= F; ++i) parts.push_back({(void**)&layers[i], (N >> i) * sizeof(qm31)});
+  for (unsigned i = 0; i < F; ++i)
+    parts.push_back({(void**)&layer_trees[i].words, DeviceTree::words_for(L + B - i) * sizeof(uint32_t)});
+  size_t total = 0;
+  for (const Part& q : parts) total += (q.bytes + 255) & ~(size_t)255;
+  ZS_CUDA(cudaMallocAsync((void**)&base, total, setup));
+  total = 0;
+  for (const Part& q : parts) *q.p = base + total, total += (q.bytes + 255) & ~(size_t)255;
   ZS_CUDA(cudaMemsetAsync(done, 0, (F + 1) * sizeof(uint32_t), setup));
-  row_tree.done = done;
-  for (unsigned i = 0; i < F; ++i) layer_trees[i].done = done + 1 + i;
+  row_tree.log_n = L + B, row_tree.done = done, row_tree.root_out = roots;
+  for (unsigned i = 0; i < F; ++i) {
+    DeviceTree& t = layer_trees[i];
+    t.log_n = L + B - i, t.done = done + 1 + i, t.root_out = roots + 8 * (1 + i);
+  }
   alphas.assign(F, qzero());
   const char* env = std::getenv("ZS_NO_GRAPH");
   use_graph = !(env && env[0] == '1');
@@ -63,14 +75,7 @@ CommitPlan::CommitPlan(uint32_t C_, unsigned L_, unsigned B_, unsigned F_) : C(C
 CommitPlan::~CommitPlan() {
   cudaDeviceSynchronize();
   drop_graph();
-  cudaFree(trace);
-  cudaFree(lde);
-  cudaFree(scratch);
-  cudaFree(gammas);
-  for (auto* p : layers) cudaFree(p);
-  cudaFree(row_tree.words);
-  cudaFree(done);
-  for (auto& t : layer_trees) cudaFree(t.words);
+  cudaFree(base);
   small.reset();
   big.reset();
   tabs.reset();
@@ -98,23 +103,52 @@ void CommitPlan::run_phase(int phase, const uint32_t* d_trace, cudaStream_t st) 
       circle_lde(d_trace, n, lde, N, C, L, B, *small, *big, scratch, st);
       break;
     case PHASE_ROW_TREE:
-      build_row_tree(lde, N, C, row_tree, gammas, layers[0], F > 0 ? &layer_trees[0] : nullptr, st);
+      build_row_leaves(lde, N, C, row_tree, gammas, layers[0], st);
+      tree_finish(row_tree, 0, st);
+      if (F > 0) build_qm31_tree(layers[0], layer_trees[0], st);
       break;
     case PHASE_FOLDS:
-      for (unsigned i = 0; i < F; ++i) {
-        const uint32_t half = (uint32_t)(N >> (i + 1));
-        fri_fold(layers[i], layers[i + 1], half, alphas[i], i, *tabs, i + 1 < F ? &layer_trees[i + 1] : nullptr, st);
+      for (unsigned i = 0; i < big_layers(); ++i) {
+        fold(i, st);
+        if (i + 1 < big_layers()) build_qm31_tree(layers[i + 1], layer_trees[i + 1], st);
       }
+      small_layers(1, st);
       break;
     default:
       throw Error(ZS_EMALFORMED, "unknown phase");
   }
 }
 
+// The layers of more than 2^kSmallTreeLog values: each has its own launches.
+unsigned CommitPlan::big_layers() const {
+  return std::min(F, L + B > kSmallTreeLog ? L + B - kSmallTreeLog : 0);
+}
+
+void CommitPlan::fold(unsigned i, cudaStream_t st) {
+  fri_fold(layers[i], layers[i + 1], 1u << (L + B - i - 1), alphas[i], nullptr, i, *tabs, st);
+}
+
+// The folds from layer big_layers() on and the trees of those layers: the folds of few
+// values in one CTA, the trees in one launch (their levels are chains of 1.3 us, whatever
+// the number of trees), from layer `first_tree` on.
+void CommitPlan::small_layers(unsigned first_tree, cudaStream_t st) {
+  unsigned i = big_layers();
+  std::vector<const qm31*> vals;
+  std::vector<DeviceTree*> trees;
+  for (unsigned k = std::max(i, first_tree); k < F; ++k) vals.push_back(layers[k]), trees.push_back(&layer_trees[k]);
+  for (; i < F && L + B - i > kChainLog; ++i) fold(i, st);
+  FoldChain fc{};
+  fc.first = i, fc.count = F - i, fc.log_size = L + B - i, fc.tables = tabs->tables;
+  for (unsigned k = 0; k < fc.count; ++k) fc.c[k] = qmul(alphas[i + k], tabs->offset_inv(i + k));
+  for (unsigned k = 0; k <= fc.count && fc.count; ++k) fc.layer[k] = layers[i + k];
+  fri_fold_chain(fc, st);
+  if (!trees.empty()) build_small_trees(vals.data(), trees.data(), (uint32_t)trees.size(), st);
+}
+
 // The step as a DAG: the LDE, the row leaves and the fold chain run on `st`; each
-// tree above its leaves (the row tree, the g tree, every committed fold layer's
-// tree) is finished on a side stream as soon as its leaves exist, so the narrow
-// tops of the trees overlap with each other and with the folds.
+// large tree (the row tree above its leaves, the large fold layers') is built on a side
+// stream as soon as its values exist, so the narrow tops of the trees overlap with each
+// other and with the folds.
 void CommitPlan::run_direct(const uint32_t* d_trace, cudaStream_t st) {
   const size_t n = (size_t)1 << L, N = (size_t)1 << (L + B);
   if (!d_trace) d_trace = trace;
@@ -167,27 +201,24 @@ void CommitPlan::run_host(const uint32_t* h_trace, cudaStream_t st) {
 // Everything after the LDE: row leaves with the gamma combination, the trees, the folds.
 void CommitPlan::after_lde(cudaStream_t st) {
   const size_t N = (size_t)1 << (L + B);
-  build_row_leaves(lde, N, C, row_tree, gammas, layers[0], F > 0 ? &layer_trees[0] : nullptr, st);
+  build_row_leaves(lde, N, C, row_tree, gammas, layers[0], st);
   unsigned side = 0;
   bool used[kSides] = {};
-  auto branch = [&](DeviceTree& t) {
+  auto branch = [&](auto&& build) {
     cudaEvent_t e = events[ev_used++];
     ZS_CUDA(cudaEventRecord(e, st));
     used[side % kSides] = true;
     cudaStream_t s = sides[side++ % kSides];
     ZS_CUDA(cudaStreamWaitEvent(s, e, 0));
-    tree_finish(t, 0, s);
+    build(s);
   };
   ev_used = 0;
-  branch(row_tree);
-  if (F > 0) branch(layer_trees[0]);
-  for (unsigned i = 0; i < F; ++i) {
-    const uint32_t half = (uint32_t)(N >> (i + 1));
-    const bool commit = i + 1 < F;
-    fri_fold(layers[i], layers[i + 1], half, alphas[i], i, *tabs, commit ? &layer_trees[i + 1] : nullptr, st,
-             /*finish_tree=*/false);
-    if (commit) branch(layer_trees[i + 1]);
+  branch([&](cudaStream_t s) { tree_finish(row_tree, 0, s); });
+  for (unsigned i = 0; i < big_layers(); ++i) {
+    branch([&](cudaStream_t s) { build_qm31_tree(layers[i], layer_trees[i], s); });
+    fold(i, st);
   }
+  small_layers(0, st);
   for (unsigned k = 0; k < kSides; ++k) {
     if (!used[k]) continue;  // only streams forked from `st` may join it (graph capture)
     cudaEvent_t e = events[ev_used++];
@@ -232,12 +263,15 @@ void CommitPlan::run(const uint32_t* d_trace, cudaStream_t st) {
 }
 
 uint32_t CommitPlan::launches() const {
-  // circle_lde: 3; row leaves: 1 + the row tree's and the g tree's tree_finish;
-  // each fold: 1 + the folded layer's tree_finish when it is committed.
+  // circle_lde: 3; row leaves: 1 and the row tree's; each large layer a fold and its tree's;
+  // then small_layers.
   const unsigned LB = L + B;
-  uint32_t k = 3 + 1 + tree_finish_launches(LB, 0);
-  if (F > 0) k += tree_finish_launches(LB, 0);
-  for (unsigned i = 0; i < F; ++i) k += 1 + (i + 1 < F ? tree_finish_launches(LB - i - 1, 0) : 0);
+  uint32_t k = 3 + 1 + tree_launches(LB);
+  for (unsigned i = 0; i < big_layers(); ++i) k += 1 + tree_launches(LB - i);
+  unsigned i = big_layers();
+  if (i < F) ++k;  // the trees
+  for (; i < F && LB - i > kChainLog; ++i) ++k;
+  if (i < F) ++k;  // the chain
   return k;
 }
 

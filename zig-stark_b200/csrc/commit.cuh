@@ -17,6 +17,7 @@ struct CommitPlan {
   cudaStream_t setup = nullptr;
   std::unique_ptr<CircleDomain> small, big;
   std::unique_ptr<FoldTables> tabs;
+  unsigned char* base = nullptr;  // the allocation that holds the buffers below
   uint32_t* trace = nullptr;    // C x 2^L, column-major
   uint32_t* lde = nullptr;      // C x 2^(L+B), column-major, natural order
   uint32_t* scratch = nullptr;  // circle_lde scratch
@@ -25,7 +26,8 @@ struct CommitPlan {
   std::vector<qm31*> layers;    // F + 1 fold layers; layers[0] = g
   DeviceTree row_tree;
   std::vector<DeviceTree> layer_trees;  // trees of layers 0 .. F-1
-  uint32_t* done = nullptr;             // the trees' counters: row tree, then the layers
+  uint32_t* done = nullptr;   // the trees' counters: row tree, then the layers
+  uint32_t* roots = nullptr;  // their roots, 8 words each, in the same order
 
   CommitPlan(uint32_t C, unsigned L, unsigned B, unsigned F);
   ~CommitPlan();
@@ -62,6 +64,9 @@ struct CommitPlan {
   const uint32_t* host_trace = nullptr;
   void drop_graph();
   void after_lde(cudaStream_t st);
+  unsigned big_layers() const;
+  void fold(unsigned i, cudaStream_t st);
+  void small_layers(unsigned first_tree, cudaStream_t st);
 };
 
 }  // namespace zs

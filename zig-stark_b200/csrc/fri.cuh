@@ -20,35 +20,46 @@ struct FoldTables {
 };
 
 // One fold (fri.zig:209-219): out[j] = (y0 + y1)/2 + alpha * (y0 - y1) / (2 D_layer[j]),
-// y0 = in[j], y1 = in[j + half], for j < half. When `next_tree` is given, also
-// writes the leaves hashQM31(out[j]) and, unless `finish_tree` is false (the caller
-// finishes it elsewhere), the rest of the folded layer's tree.
-void fri_fold(const qm31* d_in, qm31* d_out, uint32_t half, const qm31& alpha, unsigned layer,
-              const FoldTables& tabs, DeviceTree* next_tree, cudaStream_t st, bool finish_tree = true);
-// The same fold with the challenge read from device memory (written there by the
-// device transcript step that precedes it on `st`).
-void fri_fold(const qm31* d_in, qm31* d_out, uint32_t half, const qm31* d_alpha, unsigned layer,
-              const FoldTables& tabs, DeviceTree* next_tree, cudaStream_t st);
+// y0 = in[j], y1 = in[j + half], for j < half, with the challenge given or (`d_alpha`) read
+// from device memory.
+void fri_fold(const qm31* d_in, qm31* d_out, uint32_t half, const qm31& alpha, const qm31* d_alpha, unsigned layer,
+              const FoldTables& tabs, cudaStream_t st);
+
+// A chain of folds with given challenges, from a layer of at most 2^kChainLog values down,
+// in one CTA: each fold of so few values is a launch's latency otherwise.
+constexpr unsigned kChainLog = 12;
+struct FoldChain {
+  unsigned first, count;  // folds of layers first .. first + count - 1
+  unsigned log_size;      // log2 of layer `first`'s length
+  const qm31* tables;
+  qm31 c[kChainLog];                // alpha_i * offset_inv(i)
+  qm31* layer[kChainLog + 1];       // layer[0] is only read
+};
+void fri_fold_chain(const FoldChain& chain, cudaStream_t st);
 
 // The small layers of the commit phase in one CTA (fri.zig:195-227): for layers
-// first .. first + count - 1 (the first holding at most kTailMax values): commit the
-// layer (hashQM31 leaves and the whole tree), absorb its root into the device
-// transcript `ch` and sample the folding challenge, fold into the next layer. Every
-// step is a barrier apart, so the chain of small dependent steps costs no launches.
-constexpr uint32_t kTailMax = 1024;
-constexpr uint32_t kTailLayers = 16;
+// first .. first + count - 1 (the first holding at most kTailMax values): fold the layer
+// before into it, commit it (hashQM31 leaves and the whole tree), absorb its root into the
+// device transcript `ch` and sample the folding challenge; at the end the fold into the
+// layer after the last. Every step is a barrier apart, so the chain of small dependent
+// steps costs no launches.
+constexpr unsigned kTailLog = 9;
+constexpr uint32_t kTailMax = 1u << kTailLog;
+constexpr uint32_t kTailLayers = kTailLog + 1;
 struct FriTail {
   uint32_t first, count;  // absolute index of the first layer, layers handled
   unsigned log_size;      // log2 of the first layer's length
   const qm31* tables;     // FoldTables::tables
-  qm31 off_inv[kTailLayers];
-  qm31* layer[kTailLayers + 1];  // layer[c] has 2^(log_size - c) values; the last is only written
-  uint32_t* tree[kTailLayers];   // DeviceTree words of layer c
-  uint32_t* roots;               // 8 words per handled layer
-  qm31* alphas;                  // one per handled layer
+  qm31 off_inv[kTailLayers + 1];  // of layer first - 1 + c
+  // layer[c] is layer first - 1 + c; layer[0] may be null (first = 0); layer[count + 1],
+  // 2^(log_size - count) values, is only written
+  qm31* layer[kTailLayers + 2];
+  uint32_t* tree[kTailLayers];  // DeviceTree words of layer first + c
+  uint32_t* roots;              // 8 words per handled layer
+  qm31* alphas;                 // one per handled layer; alphas[-1] is layer first - 1's
 };
 struct Channel;
-// Launch with one CTA of kTailMax / 4 threads; `ft` and `ch` are in device memory.
+// `ft` and `ch` are in device memory.
 void fri_tail(const FriTail* ft, Channel* ch, cudaStream_t st);
 
 }  // namespace zs

@@ -96,9 +96,8 @@ struct FriParamsH {
 
 // Fiat-Shamir channel (channel.zig): one running Blake3 over
 // "zig-stark:channel" || separator || absorbed bytes; sample block k is
-// Blake3(state || "zig-stark:sample" || u64le(k)) and is absorbed back. Usable on the
-// host and, in one thread, on the device (the FRI commit phase runs its transcript
-// steps there); the layout is the same on both sides, so the state is copied across.
+// Blake3(state || "zig-stark:sample" || u64le(k)) and is absorbed back. The FRI commit
+// phase runs its transcript steps on the device (transcript.cuh), on a copy of this state.
 ZS_HD uint32_t m31_from_le(const uint8_t* b) {  // M31.fromBytes (m31.zig:97-100)
   const uint32_t r = (uint32_t)b[0] | ((uint32_t)b[1] << 8) | ((uint32_t)b[2] << 16) | ((uint32_t)b[3] << 24);
   return r >= P ? r % P : r;
@@ -106,35 +105,23 @@ ZS_HD uint32_t m31_from_le(const uint8_t* b) {  // M31.fromBytes (m31.zig:97-100
 
 struct Channel {
   Hasher h;
-  ZS_HD Channel(const void* sep, size_t n) {
+  Channel(const void* sep, size_t n) {
     h.update("zig-stark:channel", 17);
     h.update(sep, n);
   }
   void absorb(const Digest& d) { h.update(d.data(), 32); }
-  ZS_HD void absorb_bytes(const void* p, size_t n) { h.update(p, n); }
-  ZS_HD void absorb(const qm31& v) {
+  void absorb(const qm31& v) {
     const uint32_t w[4] = {v.a.a, v.a.b, v.b.a, v.b.b};
     uint8_t b[16];
     for (int i = 0; i < 4; ++i)
       for (int k = 0; k < 4; ++k) b[4 * i + k] = (uint8_t)(w[i] >> (8 * k));
     h.update(b, 16);
   }
-  // On the host a sample is drawn from a snapshot of the state (`scratch`, a local
-  // copy when null); on the device, in one thread, from the state itself extended by
-  // the suffix (Hasher::finalize_suffix), which copies no stack.
-  ZS_HD void sample_bytes(uint8_t* out, size_t len, Hasher* scratch = nullptr) {
+  // A sample is drawn from a snapshot of the state (`scratch`, a local copy when null).
+  void sample_bytes(uint8_t* out, size_t len, Hasher* scratch = nullptr) {
     uint64_t counter = 0;
     while (len) {
       uint8_t blk[32];
-#ifdef __CUDA_ARCH__
-      (void)scratch;
-      uint8_t suf[24];
-      copy_bytes(suf, "zig-stark:sample", 16);
-      for (int i = 0; i < 8; ++i) suf[16 + i] = (uint8_t)(counter >> (8 * i));
-      uint32_t o[8];
-      h.finalize_suffix(suf, 24, o);
-      for (int i = 0; i < 32; ++i) blk[i] = (uint8_t)(o[i / 4] >> (8 * (i % 4)));
-#else
       Hasher local;
       Hasher& snap = scratch ? *scratch : local;
       snap.snapshot_from(h);
@@ -143,7 +130,6 @@ struct Channel {
       for (int i = 0; i < 8; ++i) cb[i] = (uint8_t)(counter >> (8 * i));
       snap.update(cb, 8);
       snap.finalize(blk);
-#endif
       h.update(blk, 32);
       const size_t k = len < 32 ? len : 32;
       copy_bytes(out, blk, k);
@@ -152,7 +138,7 @@ struct Channel {
       ++counter;
     }
   }
-  ZS_HD qm31 sample_q(Hasher* scratch = nullptr) {
+  qm31 sample_q(Hasher* scratch = nullptr) {
     uint8_t b[16];
     sample_bytes(b, 16, scratch);
     return qmake(m31_from_le(b), m31_from_le(b + 4), m31_from_le(b + 8), m31_from_le(b + 12));
@@ -173,18 +159,6 @@ struct Channel {
     }
   }
 };
-
-#ifdef __CUDACC__
-// Block-cooperative copy of a transcript state between global and shared memory (the
-// single-thread transcript steps run on the shared copy: byte-wise state updates cost
-// far less there than in global memory).
-__device__ __forceinline__ void copy_state(void* dst, const void* src, size_t bytes) {
-  uint2* d = static_cast<uint2*>(dst);
-  const uint2* s = static_cast<const uint2*>(src);
-  for (size_t i = threadIdx.x; i < bytes / 8; i += blockDim.x) d[i] = s[i];
-}
-static_assert(sizeof(Channel) % 8 == 0, "the transcript state is copied in 8-byte words");
-#endif
 
 // Lagrange interpolation through (xs[i], ys[i]), the reference's own O(n^2)
 // algorithm (univariate.zig:79-139); used on <= 8 points (AIR constants, the FRI

@@ -9,28 +9,18 @@
 
 #include "blake3.cuh"
 #include "merkle.cuh"
+#include "transcript.cuh"
+#include "tree.cuh"
 
 namespace zs {
 
 namespace {
 constexpr unsigned kThreads = 256;
 
-__device__ __forceinline__ void put_digest(uint32_t* tree_words, size_t digest_index, const uint32_t o[8]) {
-  uint4* dst = reinterpret_cast<uint4*>(tree_words + 8 * digest_index);
-  dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-  dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-}
-__device__ __forceinline__ void get_digest(const uint32_t* tree_words, size_t digest_index, uint32_t o[8]) {
-  const uint4* src = reinterpret_cast<const uint4*>(tree_words + 8 * digest_index);
-  const uint4 a = src[0], b = src[1];
-  o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
-  o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
-}
-
 }  // namespace
 
 // Row leaves hashM31s(col_0[r], ..., col_{C-1}[r]) (src/m31/hash.zig:15-25), and
-// optionally g[r] = sum_c gammas[c] * col_c[r] with its hashQM31 leaf. The four
+// optionally g[r] = sum_c gammas[c] * col_c[r]. The four
 // coordinates of g accumulate unreduced 62-bit products in 64 bits (one wide
 // multiply-add each) with a Mersenne fold every four columns: after a fold the
 // accumulator is below 2^34, and four products below (p-1)^2 keep it below 2^64.
@@ -43,8 +33,7 @@ __device__ __forceinline__ uint32_t canon64(uint64_t x) {
 
 __global__ void __launch_bounds__(kThreads) k_row_leaves(const uint32_t* __restrict__ cols, size_t col_stride,
                                                          uint32_t C, uint32_t* tree_words, uint64_t n,
-                                                         const qm31* __restrict__ gammas, qm31* g_out,
-                                                         uint32_t* g_tree_words) {
+                                                         const qm31* __restrict__ gammas, qm31* g_out) {
   __shared__ uint4 sg[256];
   const bool comb = gammas != nullptr;
   if (comb)
@@ -100,96 +89,40 @@ __global__ void __launch_bounds__(kThreads) k_row_leaves(const uint32_t* __restr
   put_digest(tree_words, r, cv);
   if (!comb) return;
   const qm31 acc = qmake(canon64(acc0), canon64(acc1), canon64(acc2), canon64(acc3));
-  if (g_out) reinterpret_cast<uint4*>(g_out)[r] = make_uint4(acc.a.a, acc.a.b, acc.b.a, acc.b.b);
-  if (g_tree_words) {
-    uint32_t o[8];
-    b3::hash_qm31(acc, o);
-    put_digest(g_tree_words, r, o);
-  }
+  reinterpret_cast<uint4*>(g_out)[r] = u4_of(acc);
 }
 
-// The trees of one launch.
+// The trees of one launch: of one size, or (from their leaves, narrow) of several.
 struct TreeSet {
   uint32_t* words[kTreeBatch];
   uint32_t* done[kTreeBatch];
-  const qm31* vals[kTreeBatch];  // the leaves' values (LEAF)
+  const qm31* vals[kTreeBatch];    // the leaves' values (kValues)
+  uint32_t* root_out[kTreeBatch];  // where else the root goes (8 words), or null
+  uint8_t log_n[kTreeBatch];
 };
 
-// Levels level0 + 1 .. level0 + levels over the 2^span digests [b 2^span, (b + 1) 2^span)
-// of level `level0` per CTA b (levels <= span), a barrier between levels; LEAF: the CTA
-// hashes those digests from the values first (hashQM31, level0 = 0). With `top` (levels =
-// span) the CTA that finishes the tree's last subtree goes on from the subtrees' roots to
-// the tree's root: each CTA counts itself in `done` after its root is visible, nobody
-// waits. All of a CTA's levels run through one loop with one copy of hash2: a copy is 26 KB
-// of instructions, and the seven copies of an earlier kernel (a 3-level subtree per
-// thread) ran at the rate of the instruction cache, not of the ALU.
-// Shared memory: the digests of the last level, two levels in turn.
+// Levels level0 + 1 .. level0 + levels over the 2^span digests of CTA b's subtree
+// (cta_levels; a smaller tree takes one CTA). With `top` (levels = span) the CTA that
+// finishes the tree's last subtree goes on from the subtrees' roots to the tree's root:
+// each CTA counts itself in `done` after its root is visible, nobody waits. TX: the CTA
+// that has the root takes the transcript's step with it.
 constexpr unsigned kTreeThreads = 256;
-template <bool LEAF>
-__global__ void __launch_bounds__(kTreeThreads, LEAF ? 4 : 3) k_tree(const __grid_constant__ TreeSet ts, unsigned log_n,
-                                                       unsigned level0, unsigned span, unsigned levels,
-                                                       unsigned top) {
+template <int SRC, bool TX>
+__global__ void __launch_bounds__(kTreeThreads, SRC == kValues ? 4 : 3)
+    k_tree(const __grid_constant__ TreeSet ts, unsigned level0, unsigned span, unsigned levels, unsigned top,
+           const __grid_constant__ FoldSource f, const __grid_constant__ TranscriptStep tx) {
   extern __shared__ uint4 s_dig[];
   uint32_t* words = ts.words[blockIdx.y];
-  const size_t N2 = (size_t)2 << log_n;
+  const unsigned log_n = ts.log_n[blockIdx.y];
+  if (level0 + span > log_n) span = levels = log_n - level0;
   size_t cta = blockIdx.x;
+  if (cta >> (log_n - level0 - span)) return;  // the set has larger trees
+  qm31 fold_c = qzero();
+  if constexpr (SRC == kFold) fold_c = qmul(q_of(__ldcg(reinterpret_cast<const uint4*>(f.alpha))), f.off_inv);
 #pragma unroll 1
   for (;;) {
-    uint32_t from = 0, to = 0;  // offsets of the two levels in s_dig, in digests
-#pragma unroll 1
-    for (unsigned l = 1; l <= levels; ++l) {
-      const uint32_t cnt = 1u << (span - l);
-      const size_t dst = (N2 - (N2 >> (level0 + l))) + (cta << (span - l));
-      const bool leaves = LEAF && level0 == 0 && l == 1;
-      // The children's digests (or their leaves' values) in `q`, loaded one node ahead: warps
-      // that all hash alike reach their loads together, and nothing else covers them.
-      const uint4* src =
-          leaves ? reinterpret_cast<const uint4*>(ts.vals[blockIdx.y]) + (cta << span)
-          : l == 1 ? reinterpret_cast<const uint4*>(words + 8 * ((N2 - (N2 >> level0)) + (cta << span)))
-                   : s_dig + 2 * from;
-      uint4 q[4];
-      auto load = [&](uint32_t e) {
-        if (leaves) {
-          q[0] = __ldg(src + 2 * e), q[1] = __ldg(src + 2 * e + 1);
-        } else if (l == 1) {  // past L1: other CTAs may have written them in this launch
-#pragma unroll
-          for (int k = 0; k < 4; ++k) q[k] = __ldcg(src + 4 * e + k);
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) q[k] = src[4 * e + k];
-        }
-      };
-      if (threadIdx.x < cnt) load(threadIdx.x);
-#pragma unroll 1
-      for (uint32_t e = threadIdx.x; e < cnt; e += blockDim.x) {
-        uint32_t lc[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w};
-        uint32_t rc[8] = {q[2].x, q[2].y, q[2].z, q[2].w, q[3].x, q[3].y, q[3].z, q[3].w};
-        if (e + blockDim.x < cnt) load(e + blockDim.x);
-        uint32_t o[8];
-        if (leaves) {  // hash the two leaves first, the second into rc
-          const size_t leaf = (cta << span) + 2 * (size_t)e;
-          uint32_t v[4] = {lc[0], lc[1], lc[2], lc[3]};
-#pragma unroll 1
-          for (int k = 0; k < 2; ++k) {
-            b3::hash_qm31(qmake(v[0], v[1], v[2], v[3]), rc);
-            put_digest(words, leaf + k, rc);
-            if (k == 0) {
-#pragma unroll
-              for (int w = 0; w < 4; ++w) v[w] = lc[4 + w];
-#pragma unroll
-              for (int w = 0; w < 8; ++w) lc[w] = rc[w];
-            }
-          }
-        }
-        b3::hash2(lc, rc, o);
-        put_digest(words, dst + e, o);
-        if (l < levels) put_digest(reinterpret_cast<uint32_t*>(s_dig), to + e, o);
-      }
-      __syncthreads();
-      from = to;
-      to = to == 0 ? 1u << (span - 1) : 0;
-    }
-    if (!top || level0 + levels == log_n) return;
+    cta_levels<SRC>(words, log_n, level0, span, levels, cta, s_dig, ts.vals[blockIdx.y], f, fold_c);
+    if (!top || level0 + levels == log_n) break;
     uint32_t& s_last = reinterpret_cast<uint32_t*>(s_dig)[0];  // the digests there are done with
     if (threadIdx.x == 0) {  // wrote the subtree's root
       __threadfence();
@@ -208,6 +141,18 @@ __global__ void __launch_bounds__(kTreeThreads, LEAF ? 4 : 3) k_tree(const __gri
     level0 += levels;
     span = levels = log_n - level0;
     cta = 0;
+  }
+  if (level0 + levels != log_n) return;
+  const uint32_t* root = words + 8 * (((size_t)2 << log_n) - 2);
+  uint32_t* root_out = ts.root_out[blockIdx.y];
+  if (root_out && threadIdx.x < 8) root_out[threadIdx.x] = __ldcg(root + threadIdx.x);
+  if constexpr (TX) {
+    if (threadIdx.x >= 32) return;
+    __shared__ wtx::Shared s_tx;
+    wtx::load(s_tx, tx.ch);
+    const qm31 alpha = wtx::step(s_tx, root);
+    wtx::store(s_tx, tx.ch);
+    if (threadIdx.x == 0) *reinterpret_cast<uint4*>(tx.alpha) = u4_of(alpha);
   }
 }
 
@@ -232,6 +177,11 @@ struct TreeLaunch {
 // in narrow launches only, 562 us with three levels per thread), 2^20 116 us (126 us with
 // spans of 2^11), 2^18 53 us (60 us narrow), 2^14 27 us, 2^12 24.7 us; 32 trees of 2^17
 // 365 us (537 us narrow), 12 of 2^14 43 us (51 us narrow, 47 us with spans of 2^11).
+TreeLaunch plan_narrow(unsigned log_n, unsigned level0) {
+  const unsigned rem = log_n - level0, span = std::min(rem, 8u);
+  return {level0, span, span, 128, rem - span <= 8 ? rem - span : 0};
+}
+
 std::vector<TreeLaunch> plan_tree(unsigned log_n, unsigned level0, uint32_t count) {
   std::vector<TreeLaunch> v;
   while (level0 < log_n) {
@@ -245,8 +195,7 @@ std::vector<TreeLaunch> plan_tree(unsigned log_n, unsigned level0, uint32_t coun
     } else if (rem >= 13 && digests >= ((uint64_t)1 << 17)) {
       t.span = 9, t.levels = 3, t.threads = 128;
     } else {
-      t.span = t.levels = std::min(rem, 8u), t.threads = 128;
-      if (rem - t.levels <= 8) t.top_levels = rem - t.levels;
+      t = plan_narrow(log_n, level0);
     }
     v.push_back(t);
     level0 += t.levels + t.top_levels;
@@ -254,35 +203,50 @@ std::vector<TreeLaunch> plan_tree(unsigned log_n, unsigned level0, uint32_t coun
   return v;
 }
 
-void finish_set(const TreeSet& ts, uint32_t count, unsigned log_n, unsigned level0, bool leaves, cudaStream_t st) {
-  if (leaves && log_n == 0) throw Error(ZS_EGENERIC, "a tree of one leaf");
-  for (const TreeLaunch& t : plan_tree(log_n, level0, count)) {
+// All launches from level0 to the roots: the first from `src`, the last with the
+// transcript's step when `tx` is given.
+void finish_set(const TreeSet& ts, uint32_t count, unsigned log_n, unsigned level0, TreeSource src, cudaStream_t st,
+                const FoldSource& f = {}, const TranscriptStep* tx = nullptr) {
+  if (log_n == 0) throw Error(ZS_EGENERIC, "a tree of one leaf");
+  const std::vector<TreeLaunch> plan = plan_tree(log_n, level0, count);
+  for (const TreeLaunch& t : plan) {
     const dim3 grid(1u << (log_n - t.level0 - t.span), count);
-    if (leaves && t.level0 == 0)
-      k_tree<true><<<grid, t.threads, t.smem(), st>>>(ts, log_n, t.level0, t.span, t.levels, t.top_levels > 0);
-    else
-      k_tree<false><<<grid, t.threads, t.smem(), st>>>(ts, log_n, t.level0, t.span, t.levels, t.top_levels > 0);
+    const TreeSource from = &t == &plan.front() ? src : kDigests;
+    const bool with_tx = tx && &t == &plan.back();
+    auto* k = from == kFold     ? (with_tx ? k_tree<kFold, true> : k_tree<kFold, false>)
+              : from == kValues ? (with_tx ? k_tree<kValues, true> : k_tree<kValues, false>)
+                                : (with_tx ? k_tree<kDigests, true> : k_tree<kDigests, false>);
+    k<<<grid, t.threads, t.smem(), st>>>(ts, t.level0, t.span, t.levels, t.top_levels > 0, f,
+                                         tx ? *tx : TranscriptStep{});
   }
   ZS_CUDA(cudaGetLastError());
 }
 
+void add_tree(TreeSet& ts, uint32_t k, const DeviceTree& tree, const qm31* vals) {
+  ts.words[k] = tree.words, ts.done[k] = tree.done, ts.vals[k] = vals;
+  ts.root_out[k] = tree.root_out, ts.log_n[k] = (uint8_t)tree.log_n;
+}
+
 TreeSet single(const DeviceTree& tree, const qm31* vals = nullptr) {
   TreeSet ts{};
-  ts.words[0] = tree.words, ts.done[0] = tree.done, ts.vals[0] = vals;
+  add_tree(ts, 0, tree, vals);
   return ts;
 }
 }  // namespace
 
 void tree_finish(DeviceTree& tree, unsigned from_level, cudaStream_t st) {
-  finish_set(single(tree), 1, tree.log_n, from_level, false, st);
+  finish_set(single(tree), 1, tree.log_n, from_level, kDigests, st);
 }
 
-uint32_t tree_finish_launches(unsigned log_n, unsigned from_level) {
-  return (uint32_t)plan_tree(log_n, from_level, 1).size();
+uint32_t tree_launches(unsigned log_n) { return (uint32_t)plan_tree(log_n, 0, 1).size(); }
+
+void build_qm31_tree(const qm31* d_values, DeviceTree& tree, cudaStream_t st, const TranscriptStep* tx) {
+  finish_set(single(tree, d_values), 1, tree.log_n, 0, kValues, st, {}, tx);
 }
 
-void build_qm31_tree(const qm31* d_values, DeviceTree& tree, cudaStream_t st) {
-  finish_set(single(tree, d_values), 1, tree.log_n, 0, true, st);
+void build_fold_tree(const FoldSource& f, DeviceTree& tree, cudaStream_t st, const TranscriptStep* tx) {
+  if (f.half != 1u << tree.log_n) throw Error(ZS_EGENERIC, "fold and tree of different sizes");
+  finish_set(single(tree), 1, tree.log_n, 0, kFold, st, f, tx);
 }
 
 void build_qm31_trees(const qm31* d_values, size_t v_stride, DeviceTree* const* trees, uint32_t count,
@@ -293,31 +257,37 @@ void build_qm31_trees(const qm31* d_values, size_t v_stride, DeviceTree* const* 
     TreeSet ts{};
     for (uint32_t k = 0; k < c; ++k) {
       if (trees[t0 + k]->log_n != log_n) throw Error(ZS_EGENERIC, "build_qm31_trees: trees of different sizes");
-      ts.words[k] = trees[t0 + k]->words, ts.done[k] = trees[t0 + k]->done;
-      ts.vals[k] = d_values + (size_t)(t0 + k) * v_stride;
+      add_tree(ts, k, *trees[t0 + k], d_values + (size_t)(t0 + k) * v_stride);
     }
-    finish_set(ts, c, log_n, 0, true, st);
+    finish_set(ts, c, log_n, 0, kValues, st);
   }
 }
 
-void build_row_leaves(const uint32_t* d_cols, size_t col_stride, uint32_t C, DeviceTree& tree, const qm31* d_gammas,
-                      qm31* g_out, DeviceTree* g_tree, cudaStream_t st) {
-  if (C == 0 || C > 256) throw Error(ZS_EMALFORMED, "row leaves need 1..256 columns");
-  const uint64_t n = (uint64_t)1 << tree.log_n;
-  k_row_leaves<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(
-      d_cols, col_stride, C, tree.words, n, d_gammas, g_out, g_tree ? g_tree->words : nullptr);
+void build_small_trees(const qm31* const* d_values, DeviceTree* const* trees, uint32_t count, cudaStream_t st) {
+  for (uint32_t t0 = 0; t0 < count; t0 += kTreeBatch) {
+    const uint32_t c = std::min<uint32_t>(kTreeBatch, count - t0);
+    TreeSet ts{};
+    unsigned log_n = 0;
+    for (uint32_t k = 0; k < c; ++k) {
+      if (trees[t0 + k]->log_n > kSmallTreeLog || trees[t0 + k]->log_n == 0)
+        throw Error(ZS_EGENERIC, "build_small_trees: tree size");
+      add_tree(ts, k, *trees[t0 + k], d_values[t0 + k]);
+      log_n = std::max(log_n, trees[t0 + k]->log_n);
+    }
+    const TreeLaunch t = plan_narrow(log_n, 0);
+    k_tree<kValues, false><<<dim3(1u << (log_n - t.span), c), t.threads, t.smem(), st>>>(ts, 0, t.span, t.levels, 1,
+                                                                                       {}, {});
+  }
   ZS_CUDA(cudaGetLastError());
 }
 
-void build_row_tree(const uint32_t* d_cols, size_t col_stride, uint32_t C, DeviceTree& tree, const qm31* d_gammas,
-                    qm31* g_out, DeviceTree* g_tree, cudaStream_t st) {
+void build_row_leaves(const uint32_t* d_cols, size_t col_stride, uint32_t C, DeviceTree& tree, const qm31* d_gammas,
+                      qm31* g_out, cudaStream_t st) {
   if (C == 0 || C > 256) throw Error(ZS_EMALFORMED, "row leaves need 1..256 columns");
   const uint64_t n = (uint64_t)1 << tree.log_n;
-  k_row_leaves<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(
-      d_cols, col_stride, C, tree.words, n, d_gammas, g_out, g_tree ? g_tree->words : nullptr);
+  k_row_leaves<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(d_cols, col_stride, C, tree.words, n,
+                                                                               d_gammas, g_out);
   ZS_CUDA(cudaGetLastError());
-  tree_finish(tree, 0, st);
-  if (g_tree) tree_finish(*g_tree, 0, st);
 }
 
 // out[q * log_n * 8 ...] = siblings of indices[q], bottom-up.

@@ -15,6 +15,7 @@ struct DeviceTree {
   // Finished subtrees of a launch in which the last one's CTA goes on to the top
   // (k_tree): one word, zero before the tree's first launch and again after each.
   uint32_t* done = nullptr;
+  uint32_t* root_out = nullptr;  // where else the root goes when the tree is finished (8 words)
   static size_t words_for(unsigned log_n) { return (((size_t)2 << log_n) - 1) * 8; }
   size_t level_offset(unsigned k) const {
     const size_t N2 = (size_t)2 << log_n;
@@ -25,8 +26,28 @@ struct DeviceTree {
   const uint32_t* root() const { return level(log_n); }
 };
 
+// A fold as the source of a layer's values (fri.cuh): out[j], j < half, from `in` (2 half
+// values of layer `layer`), the challenge read from device memory.
+struct FoldSource {
+  const qm31* in;
+  qm31* out;
+  const qm31* alpha;
+  const qm31* tables;  // FoldTables::tables
+  qm31 off_inv;        // FoldTables::offset_inv(layer)
+  uint32_t half;
+  unsigned layer;
+};
+// A transcript step after a root: absorb it, sample a folding challenge.
+struct Channel;
+struct TranscriptStep {
+  Channel* ch;  // the transcript, in device memory
+  qm31* alpha;  // the challenge
+};
+
 // Leaves hashQM31(values[i]) for 2^log_n QM31 values plus the whole tree.
-void build_qm31_tree(const qm31* d_values, DeviceTree& tree, cudaStream_t st);
+void build_qm31_tree(const qm31* d_values, DeviceTree& tree, cudaStream_t st, const TranscriptStep* tx = nullptr);
+// The same over the outputs of a fold, which are stored as well.
+void build_fold_tree(const FoldSource& f, DeviceTree& tree, cudaStream_t st, const TranscriptStep* tx = nullptr);
 
 // Most trees that one launch builds (blockIdx.y picks the tree).
 constexpr uint32_t kTreeBatch = 64;
@@ -34,10 +55,14 @@ constexpr uint32_t kTreeBatch = 64;
 // d_values + k * v_stride.
 void build_qm31_trees(const qm31* d_values, size_t v_stride, DeviceTree* const* trees, uint32_t count,
                       cudaStream_t st);
+// Trees of several sizes up to 2^kSmallTreeLog, each over its own values: small trees are
+// chains of levels, so one launch takes the time of its largest.
+constexpr unsigned kSmallTreeLog = 14;
+void build_small_trees(const qm31* const* d_values, DeviceTree* const* trees, uint32_t count, cudaStream_t st);
 // Completes the levels above `from_level` (levels <= from_level must be written).
 void tree_finish(DeviceTree& tree, unsigned from_level, cudaStream_t st);
-// Number of launches tree_finish makes.
-uint32_t tree_finish_launches(unsigned log_n, unsigned from_level);
+// Number of launches that a tree from its leaves' digests or values takes.
+uint32_t tree_launches(unsigned log_n);
 
 // Opening path of leaf `index` (siblings bottom-up, merkle.zig:57-68), read back to
 // the host from a device tree. `out` receives log_n digests of 32 bytes.
@@ -49,12 +74,9 @@ void tree_open_many(const DeviceTree& tree, const uint64_t* d_indices, uint32_t 
 
 // Row leaves of C columns x 2^log_n M31 values (column c at d_cols + c * col_stride):
 // leaf r = hashM31s(col_0[r], ..., col_{C-1}[r]) (src/m31/hash.zig:15-25), C <= 256.
-// Also writes g[r] = sum_c gammas[c] * col_c[r] when `g_out` is not null, and, when
-// `g_tree` is not null, the tree over hashQM31(g[r]).
-void build_row_tree(const uint32_t* d_cols, size_t col_stride, uint32_t C, DeviceTree& tree, const qm31* d_gammas,
-                    qm31* g_out, DeviceTree* g_tree, cudaStream_t st);
-// The leaf level only of build_row_tree (and of the g tree); finish with tree_finish.
+// Also writes g[r] = sum_c gammas[c] * col_c[r] when `d_gammas` is not null. The leaf level
+// only; finish with tree_finish.
 void build_row_leaves(const uint32_t* d_cols, size_t col_stride, uint32_t C, DeviceTree& tree, const qm31* d_gammas,
-                      qm31* g_out, DeviceTree* g_tree, cudaStream_t st);
+                      qm31* g_out, cudaStream_t st);
 
 }  // namespace zs

@@ -147,8 +147,12 @@ struct Arena {
 };
 
 struct Slot {
-  Stager stager;
+  std::unique_ptr<Stager> stager_;  // 32 MB of pinned memory, made for the first large upload
   Arena arena;
+  Stager& stager() {
+    if (!stager_) stager_ = std::make_unique<Stager>();
+    return *stager_;
+  }
 };
 
 // Slots are created on demand and kept for the life of the process.
@@ -257,7 +261,7 @@ void host_copy(void* dst, const void* src, size_t bytes) {
 
 void upload_bytes(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   if (bytes == 0) return;
-  Stager* sg = (bytes < kSmall || !t_slot) ? nullptr : &t_slot->stager;
+  Stager* sg = (bytes < kSmall || !t_slot) ? nullptr : &t_slot->stager();
   if (!sg || !sg->ok) {
     ZS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
     return;
@@ -283,7 +287,7 @@ void upload_bytes(void* dst, const void* src, size_t bytes, cudaStream_t st) {
 
 void upload_low_words(uint32_t* dst, const uint8_t* const* cols, uint32_t C, size_t n, uint8_t* high,
                       cudaStream_t st) {
-  Stager* sg = t_slot ? &t_slot->stager : nullptr;
+  Stager* sg = t_slot ? &t_slot->stager() : nullptr;
   if (!sg || !sg->ok) throw Error(ZS_EGENERIC, "upload_low_words needs pinned staging");
   HostPool& pool = HostPool::get();
   const size_t parts = pool.width();
