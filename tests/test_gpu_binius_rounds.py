@@ -1,0 +1,37 @@
+"""Where the sum-check prover changes its launches: the last rounds in one CTA (by lookups
+and by table bytes) and the direct or table fold over GF(2^128), against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+REF = [([0, 1, 2], 1), ([0], 2)]
+WIDE_TERMS = [([0, 1, 2, 3, 4, 0], 9), ([4, 4], 1), ([], 7), ([2], 200), (list(range(5)) * 3, 255)]
+
+
+@pytest.mark.parametrize("level,k,m,terms", [
+    (3, 12, 3, REF), (3, 13, 3, REF), (3, 14, 3, REF), (3, 9, 5, WIDE_TERMS), (3, 11, 40, [([39], 1), ([0, 39], 5)]),
+    (3, 1, 1, [([0], 1)]), (3, 7, 1, [([], 3)]), (7, 5, 3, REF), (7, 6, 3, REF), (7, 7, 3, REF),
+    (7, 4, 5, WIDE_TERMS), (7, 8, 1, [([0], 1 << 100)])])
+def test_tail_rounds_match_oracle(orc, level, k, m, terms):
+    from zs_b200 import native
+    es = 1 if level == 3 else 16
+    rng = np.random.default_rng(900 + 13 * k + level + m)
+    tables = rng.bytes(m * (1 << k) * es)
+    seed = rng.bytes(3 * k) if k % 2 else None
+    got = native.binius_prove_combination(8 if level == 3 else 128, tables, k, m, terms, seed)
+    assert got == orc.binius_prove(level, tables, k, m, terms, seed)
+
+
+@pytest.mark.parametrize("m,length", [(3, 43690), (3, 43692), (1, 2), (7, 18726)])
+def test_fold128_either_way_matches_oracle(orc, m, length):
+    import torch
+    from zs_b200 import native
+    rng = np.random.default_rng(m + length)
+    cur = rng.bytes(m * length * 16)
+    r = int.from_bytes(rng.bytes(16), "little")
+    d_cur = torch.frombuffer(bytearray(cur), dtype=torch.uint8).to("cuda")
+    d_next = torch.zeros(m * (length // 2) * 16, dtype=torch.uint8, device="cuda")
+    d_scratch = torch.zeros(65536, dtype=torch.uint8, device="cuda")
+    native.binius_fold_device(128, d_cur.data_ptr(), length, m, r, d_next.data_ptr(), d_scratch.data_ptr())
+    torch.cuda.synchronize()
+    assert bytes(d_next.cpu().numpy()) == orc.binius_fold(7, cur, length, m, r)

@@ -33,18 +33,21 @@
 // coordinates of (a + b): a 16 x 256 table of r * (v X^byte k), built once per fold, turns
 // it into 16 lookups of 16 bytes.
 //
-// Prover. The tables go to the device once; each round is the values kernel, k_sc_step
-// (the coefficients from a Lagrange matrix built once per proof, then the SHA-256
-// transcript step in one thread, the challenge left in device memory) and the fold, which
-// reads the challenge there: the rounds run back to back and the host waits once.
+// Prover. The tables go to the device once; each round is the values kernel, whose last CTA
+// takes the step (the coefficients from a Lagrange matrix built once per proof, then the
+// SHA-256 transcript step, the challenge left in device memory), and the fold, which reads
+// the challenge there; the last rounds run in one CTA. The rounds run back to back and the
+// host waits once.
 #include <algorithm>
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/zs_binius.h"
 #include "common.cuh"
+#include "staging.cuh"
 
 namespace zs {
 namespace {
@@ -226,6 +229,26 @@ __device__ __forceinline__ g128 at_point128(const Tower& F, const g128& a, const
   else return gxor(a, F.s128(t, gxor(a, b)));
 }
 
+// The same at a point known at run time (uniform in a warp).
+__device__ __forceinline__ uint32_t at8(const Tower& F, uint32_t t, uint32_t a, uint32_t b) {
+  switch (t) {
+    case 0: return a;
+    case 1: return b;
+    case 2: return at_point8<2>(F, a, b);
+    case 3: return at_point8<3>(F, a, b);
+    default: return a ^ F.m8(t, a ^ b);
+  }
+}
+__device__ __forceinline__ g128 at128(const Tower& F, uint32_t t, const g128& a, const g128& b) {
+  switch (t) {
+    case 0: return a;
+    case 1: return b;
+    case 2: return at_point128<2>(F, a, b);
+    case 3: return at_point128<3>(F, a, b);
+    default: return gxor(a, F.s128(t, gxor(a, b)));
+  }
+}
+
 // prod[t] = (first factor at t), then prod[t] *= (next factor at t), for t < D.
 template <int D, int t = 0>
 __device__ __forceinline__ void first8(const Tower& F, uint32_t (&prod)[D], uint32_t a, uint32_t b) {
@@ -261,6 +284,187 @@ __device__ __forceinline__ g128 times_coef(const Tower& F, uint32_t kind, const 
   return kind == 0 ? v : kind == 1 ? F.s128((uint32_t)c.lo, v) : F.m128(c, v);
 }
 
+// ---- device: one round's transcript step of the combination prover ----------------
+// After a round's values are known: the round's coefficients by the Lagrange matrix
+// (sumcheck.zig:124-162), then the SHA-256 transcript step (sumcheck.zig:66-87) that
+// absorbs them and samples the next challenge. The CTA that finishes a round's values
+// takes the step, so the rounds of a proof run back to back on the device.
+
+__constant__ uint32_t kSha256K[64] = {
+    0x428a2f98, 0x71374491, 0xb5c0fbcf, 0xe9b5dba5, 0x3956c25b, 0x59f111f1, 0x923f82a4, 0xab1c5ed5,
+    0xd807aa98, 0x12835b01, 0x243185be, 0x550c7dc3, 0x72be5d74, 0x80deb1fe, 0x9bdc06a7, 0xc19bf174,
+    0xe49b69c1, 0xefbe4786, 0x0fc19dc6, 0x240ca1cc, 0x2de92c6f, 0x4a7484aa, 0x5cb0a9dc, 0x76f988da,
+    0x983e5152, 0xa831c66d, 0xb00327c8, 0xbf597fc7, 0xc6e00bf3, 0xd5a79147, 0x06ca6351, 0x14292967,
+    0x27b70a85, 0x2e1b2138, 0x4d2c6dfc, 0x53380d13, 0x650a7354, 0x766a0abb, 0x81c2c92e, 0x92722c85,
+    0xa2bfe8a1, 0xa81a664b, 0xc24b8b70, 0xc76c51a3, 0xd192e819, 0xd6990624, 0xf40e3585, 0x106aa070,
+    0x19a4c116, 0x1e376c08, 0x2748774c, 0x34b0bcb5, 0x391c0cb3, 0x4ed8aa4a, 0x5b9cca4f, 0x682e6ff3,
+    0x748f82ee, 0x78a5636f, 0x84c87814, 0x8cc70208, 0x90befffa, 0xa4506ceb, 0xbef9a3f7, 0xc67178f2};
+
+__device__ __forceinline__ uint32_t sha_rotr(uint32_t x, unsigned r) { return __funnelshift_r(x, x, r); }
+
+// One 64-byte block `m` of SHA-256 (FIPS 180-4) into the state `h`, both in shared memory,
+// by a converged warp: every lane computes the rounds (a chain that no other lane could
+// shorten), 16 to a pass of the loop with the message schedule in registers: 4,500 cycles
+// (8,000 with the additions sent to the FMA pipe: they lie on the chain). Unrolled over all 64 rounds and with the message picked
+// together byte by byte in one thread, a step took 26 us, most of it instruction fetches
+// and address arithmetic.
+__device__ __noinline__ void sha_block(uint32_t* h, const uint32_t* m) {
+  uint32_t w[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) w[i] = __byte_perm(m[i], 0, 0x0123);  // big-endian words
+  uint32_t v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = h[i];
+#pragma unroll 1
+  for (int q = 0; q < 64; q += 16) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if (q > 0) {
+        const uint32_t x = w[(i + 1) & 15], y = w[(i + 14) & 15];
+        w[i] += (sha_rotr(x, 7) ^ sha_rotr(x, 18) ^ (x >> 3)) + w[(i + 9) & 15] +
+                (sha_rotr(y, 17) ^ sha_rotr(y, 19) ^ (y >> 10));
+      }
+      // v rotates by one word per round: a = v[-i], ..., in place of moving eight words
+      const uint32_t a = v[(0 - i) & 7], bb = v[(1 - i) & 7], c = v[(2 - i) & 7], e = v[(4 - i) & 7],
+                     f = v[(5 - i) & 7], g = v[(6 - i) & 7];
+      const uint32_t t1 = v[(7 - i) & 7] + (sha_rotr(e, 6) ^ sha_rotr(e, 11) ^ sha_rotr(e, 25)) +
+                          ((e & f) ^ (~e & g)) + (kSha256K[q + i] + w[i]);
+      v[(3 - i) & 7] += t1;
+      v[(7 - i) & 7] = t1 + (sha_rotr(a, 2) ^ sha_rotr(a, 13) ^ sha_rotr(a, 22)) + ((a & bb) ^ (a & c) ^ (bb & c));
+    }
+  }
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) h[i] += v[i];
+  }
+  __syncwarp();
+}
+
+// What a step works on, in shared memory: the message to absorb (state || coefficients),
+// a hash block and the hash state.
+struct StepShared {
+  alignas(16) uint8_t msg[32 + kProveMaxPoints * 16];
+  alignas(16) uint8_t vals[kProveMaxPoints * 16];
+  uint8_t lag[kProveMaxPoints * kProveMaxPoints];
+  uint32_t blk[16], h[8];
+};
+
+// out[0..32) = SHA-256 of the n bytes at msg (shared or global memory), by a converged warp.
+__device__ __forceinline__ void sha256_warp(StepShared& s, const uint8_t* msg, uint64_t n, uint8_t* out) {
+  const uint32_t lane = threadIdx.x & 31;
+  constexpr uint32_t iv[8] = {0x6a09e667, 0xbb67ae85, 0x3c6ef372, 0xa54ff53a,
+                              0x510e527f, 0x9b05688c, 0x1f83d9ab, 0x5be0cd19};
+  if (lane == 0)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s.h[i] = iv[i];
+  const uint64_t blocks = (n + 9 + 63) / 64, end = 64 * blocks;
+  uint8_t* b = reinterpret_cast<uint8_t*>(s.blk);
+#pragma unroll 1
+  for (uint64_t at = 0; at < end; at += 64) {
+#pragma unroll
+    for (uint32_t i = lane; i < 64; i += 32) {
+      const uint64_t o = at + i;
+      uint8_t v = o < n ? msg[o] : o == n ? 0x80 : 0;
+      if (o >= end - 8) v = (uint8_t)((8 * n) >> (8 * (end - 1 - o)));
+      b[i] = v;
+    }
+    __syncwarp();
+    sha_block(s.h, s.blk);
+  }
+  out[lane] = (uint8_t)(s.h[lane >> 2] >> (24 - 8 * (lane & 3)));
+  __syncwarp();
+}
+
+// The device transcript: the SHA-256 state (32 bytes) and the last challenge (1 or 16
+// bytes), in device memory between rounds.
+struct ScTranscript {
+  uint8_t state[32];
+  uint8_t r[16];
+};
+
+// A round's step for the kernel that computes its values; tx null: values only.
+struct ScStep {
+  ScTranscript* tx;
+  uint32_t* done;      // finished CTAs of the round's launch: zero before and after
+  const uint8_t* lag;  // the n x n Lagrange matrix
+  const uint8_t* seed;
+  uint8_t* claimed;
+  uint8_t* rounds_out;
+  uint32_t n, round, seed_len;
+  int has_seed;
+};
+
+// Round `round`'s step by a converged warp, the values in s.vals and the Lagrange matrix in
+// s.lag; the state comes from the round before, in s.msg (`kept`) or device memory. The points 0..n-1 lie in
+// GF(2^8), so the Lagrange matrix does too, and a subfield scalar scales each byte
+// coordinate of a value: byte b of coefficient d is sum_i lag[i][d] * byte b of values[i],
+// one lane per byte. The first round also forms the claimed sum (values[0] + values[1])
+// and starts the transcript (from the seed, or from the claimed sum). The challenge is the
+// digest's last byte over GF(2^8), its last 16 bytes over GF(2^128).
+template <bool WIDE>
+__device__ __forceinline__ void sc_step(StepShared& s, const ScStep& st, uint32_t round, bool kept, const Tower& F) {
+  constexpr uint32_t ES = WIDE ? 16 : 1;
+  const uint32_t lane = threadIdx.x & 31, n = st.n;
+  if (round == 0) {
+    if (lane < ES) {  // one point: the sum of 2^k copies of a constant is 0
+      const uint8_t c = n >= 2 ? s.vals[lane] ^ s.vals[ES + lane] : 0;
+      s.msg[32 + lane] = c;
+      st.claimed[lane] = c;
+    }
+    __syncwarp();
+    if (st.has_seed)
+      sha256_warp(s, st.seed, st.seed_len, s.msg);
+    else
+      sha256_warp(s, s.msg + 32, ES, s.msg);
+  } else if (!kept) {
+    s.msg[lane] = __ldcg(st.tx->state + lane);
+  }
+  for (uint32_t e = lane; e < n * ES; e += 32) {
+    const uint32_t d = e / ES, b = e % ES;
+    uint32_t c = 0;
+#pragma unroll 4
+    for (uint32_t i = 0; i < n; ++i) c ^= F.m8(s.lag[i * n + d], s.vals[ES * i + b]);
+    s.msg[32 + e] = (uint8_t)c;
+    st.rounds_out[(size_t)round * n * ES + e] = (uint8_t)c;
+  }
+  __syncwarp();
+  sha256_warp(s, s.msg, 32 + n * ES, s.msg);
+  st.tx->state[lane] = s.msg[lane];
+  if (lane < ES) st.tx->r[lane] = s.msg[32 - ES + lane];
+  __syncwarp();
+}
+
+// The end of a values kernel: the CTA's accumulators (`words` words in shared memory) go to
+// `out`; with a step to take, the CTA that is the last to do so takes it and clears `out`
+// for the next round.
+template <bool WIDE>
+__device__ __forceinline__ void finish_values(const uint32_t* s_acc, uint32_t words, uint32_t* out, const ScStep& st,
+                                              const Tower& F) {
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < words; k += blockDim.x)
+    if (s_acc[k]) atomicXor(out + k, s_acc[k]);
+  if (!st.tx) return;
+  __shared__ StepShared s;
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(st.done, 1u) == gridDim.x * gridDim.y - 1;
+    if (s_last) *st.done = 0;
+  }
+  __syncthreads();
+  if (!s_last || threadIdx.x >= 32) return;
+  __threadfence();
+  for (uint32_t k = threadIdx.x; k < words; k += 32) {
+    reinterpret_cast<uint32_t*>(s.vals)[k] = __ldcg(out + k);
+    out[k] = 0;
+  }
+  for (uint32_t k = threadIdx.x; k < st.n * st.n; k += 32) s.lag[k] = __ldg(st.lag + k);
+  __syncwarp();
+  sc_step<WIDE>(s, st, st.round, false, F);
+}
+
 // GF(2^8) round; out: (dmax + 1) bytes packed four to a word (little-endian: byte t is
 // values[t]). D > 0: the D = dmax + 1 points in registers, every row once. D = 0: one
 // point per pass, points t = blockIdx.y, blockIdx.y + gridDim.y, ... (a grid of dmax + 1
@@ -268,7 +472,8 @@ __device__ __forceinline__ g128 times_coef(const Tower& F, uint32_t kind, const 
 template <int D>
 __global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* __restrict__ cur, uint32_t len, uint32_t half,
                                                        uint32_t dmax, const __grid_constant__ Terms tm,
-                                                       const uint8_t* __restrict__ gT, uint32_t* __restrict__ out) {
+                                                       const uint8_t* __restrict__ gT, uint32_t* __restrict__ out,
+                                                       const __grid_constant__ ScStep step) {
   extern __shared__ uint4 smem_b[];
   uint8_t* s_T = reinterpret_cast<uint8_t*>(smem_b);
   uint32_t* s_acc = reinterpret_cast<uint32_t*>(s_T + 65536);
@@ -337,7 +542,7 @@ __global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* __restrict
           uint32_t prod = tm.coef[k];
           for (uint32_t j = j0; j < j1; ++j) {
             const uint8_t* p = cur + (size_t)tm.idx[j] * len + 2 * (size_t)rest;
-            const uint32_t a = p[0], v = a ^ F.m8(t, a ^ p[1]);
+            const uint32_t v = at8(F, t, p[0], p[1]);
             prod = (j == j0 && tm.kind[k] == 0) ? v : F.m8(prod, v);
           }
           acc ^= prod;
@@ -346,9 +551,15 @@ __global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* __restrict
       warp_xor_into(acc << (8 * (t & 3)), s_acc + (t >> 2));
     }
   }
-  __syncthreads();
-  for (uint32_t k = threadIdx.x; k < words; k += blockDim.x)
-    if (s_acc[k]) atomicXor(out + k, s_acc[k]);
+  finish_values<false>(s_acc, words, out, step, F);
+}
+
+// 16 little-endian bytes
+__device__ __forceinline__ g128 load_challenge(const uint8_t* r) {
+  g128 v{0, 0};
+#pragma unroll
+  for (int b = 7; b >= 0; --b) v.lo = (v.lo << 8) | r[b], v.hi = (v.hi << 8) | r[8 + b];
+  return v;
 }
 
 __device__ __forceinline__ g128 load_g128(const uint4* p) {
@@ -360,7 +571,8 @@ __device__ __forceinline__ g128 load_g128(const uint4* p) {
 template <int D>
 __global__ void __launch_bounds__(kBThreads, (D >= 1 && D <= 4) ? 2 : 1) k_values128(const uint4* __restrict__ cur, uint32_t len, uint32_t half,
                                                          uint32_t dmax, const __grid_constant__ Terms tm,
-                                                         const uint8_t* __restrict__ gT, uint32_t* __restrict__ out) {
+                                                         const uint8_t* __restrict__ gT, uint32_t* __restrict__ out,
+                                                         const __grid_constant__ ScStep step) {
   extern __shared__ uint4 smem_b[];
   uint8_t* s_T = reinterpret_cast<uint8_t*>(smem_b);
   uint32_t* s_acc = reinterpret_cast<uint32_t*>(s_T + 65536);
@@ -414,7 +626,7 @@ __global__ void __launch_bounds__(kBThreads, (D >= 1 && D <= 4) ? 2 : 1) k_value
           g128 prod = c;
           for (uint32_t j = j0; j < j1; ++j) {
             const uint4* p = cur + (size_t)tm.idx[j] * len + 2 * (size_t)rest;
-            const g128 a = load_g128(p), v = gxor(a, F.s128(t, gxor(a, load_g128(p + 1))));
+            const g128 v = at128(F, t, load_g128(p), load_g128(p + 1));
             prod = j == j0 ? times_coef(F, kind, c, v) : F.m128(prod, v);
           }
           acc = gxor(acc, prod);
@@ -423,9 +635,7 @@ __global__ void __launch_bounds__(kBThreads, (D >= 1 && D <= 4) ? 2 : 1) k_value
       warp_xor_into128(acc, s_acc + 4 * t);
     }
   }
-  __syncthreads();
-  for (uint32_t k = threadIdx.x; k < words; k += blockDim.x)
-    if (s_acc[k]) atomicXor(out + k, s_acc[k]);
+  finish_values<true>(s_acc, words, out, step, F);
 }
 
 // next[f][rest] = a + r (a + b) over GF(2^8); grid.y runs over the tables.
@@ -449,9 +659,9 @@ __global__ void __launch_bounds__(kBThreads) k_fold8(const uint8_t* __restrict__
 __global__ void __launch_bounds__(kBThreads) k_mul_table128(uint64_t r_lo, uint64_t r_hi, const uint8_t* __restrict__ d_r,
                                                             const uint8_t* __restrict__ gT, uint4* __restrict__ R) {
   extern __shared__ uint4 smem_b[];
-  if (d_r) {  // the challenge in device memory: 16 little-endian bytes
-    r_lo = r_hi = 0;
-    for (int b = 7; b >= 0; --b) r_lo = (r_lo << 8) | d_r[b], r_hi = (r_hi << 8) | d_r[8 + b];
+  if (d_r) {
+    const g128 r = load_challenge(d_r);
+    r_lo = r.lo, r_hi = r.hi;
   }
   uint8_t* s_T = reinterpret_cast<uint8_t*>(smem_b);
   load_table(s_T, gT);
@@ -485,134 +695,143 @@ __global__ void __launch_bounds__(kBThreads) k_fold128(const uint4* __restrict__
   }
 }
 
-// ---- device: one round's transcript step of the combination prover ----------------
-// After a round's values are on the device: the round's coefficients by the Lagrange
-// matrix (sumcheck.zig:124-162), then the SHA-256 transcript step (sumcheck.zig:66-87)
-// that absorbs them and samples the next challenge, so the rounds of a proof run back to
-// back on the device with no trip to the host between them.
-
-__constant__ uint32_t kSha256K[64] = {
-    0x428a2f98, 0x71374491, 0xb5c0fbcf, 0xe9b5dba5, 0x3956c25b, 0x59f111f1, 0x923f82a4, 0xab1c5ed5,
-    0xd807aa98, 0x12835b01, 0x243185be, 0x550c7dc3, 0x72be5d74, 0x80deb1fe, 0x9bdc06a7, 0xc19bf174,
-    0xe49b69c1, 0xefbe4786, 0x0fc19dc6, 0x240ca1cc, 0x2de92c6f, 0x4a7484aa, 0x5cb0a9dc, 0x76f988da,
-    0x983e5152, 0xa831c66d, 0xb00327c8, 0xbf597fc7, 0xc6e00bf3, 0xd5a79147, 0x06ca6351, 0x14292967,
-    0x27b70a85, 0x2e1b2138, 0x4d2c6dfc, 0x53380d13, 0x650a7354, 0x766a0abb, 0x81c2c92e, 0x92722c85,
-    0xa2bfe8a1, 0xa81a664b, 0xc24b8b70, 0xc76c51a3, 0xd192e819, 0xd6990624, 0xf40e3585, 0x106aa070,
-    0x19a4c116, 0x1e376c08, 0x2748774c, 0x34b0bcb5, 0x391c0cb3, 0x4ed8aa4a, 0x5b9cca4f, 0x682e6ff3,
-    0x748f82ee, 0x78a5636f, 0x84c87814, 0x8cc70208, 0x90befffa, 0xa4506ceb, 0xbef9a3f7, 0xc67178f2};
-
-// SHA-256 (FIPS 180-4) of the message prefix || body in one thread. Each 64-byte block's
-// words are assembled from the message bytes (and the padding, computed on the fly), and
-// the 64 rounds are unrolled so the message schedule stays in registers.
-__device__ __forceinline__ uint32_t sha_rotr(uint32_t x, unsigned r) { return __funnelshift_r(x, x, r); }
-
-__device__ void sha256_dev(const uint8_t* prefix, uint32_t plen, const uint8_t* body, uint32_t blen,
-                           uint8_t out[32]) {
-  uint32_t h[8] = {0x6a09e667, 0xbb67ae85, 0x3c6ef372, 0xa54ff53a, 0x510e527f, 0x9b05688c, 0x1f83d9ab, 0x5be0cd19};
-  const uint64_t len = (uint64_t)plen + blen;
-  const uint64_t nblocks = (len + 9 + 63) / 64;
-  const uint64_t bits = len * 8;
-  auto byte_at = [&](uint64_t i) -> uint32_t {
-    if (i < plen) return prefix[i];
-    if (i < len) return body[i - plen];
-    if (i == len) return 0x80;
-    const uint64_t end = nblocks * 64;
-    if (i >= end - 8) return (uint32_t)(bits >> (8 * (end - 1 - i))) & 0xff;
-    return 0;
-  };
-  for (uint64_t blk = 0; blk < nblocks; ++blk) {
-    uint32_t w[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const uint64_t o = blk * 64 + 4 * i;
-      w[i] = byte_at(o) << 24 | byte_at(o + 1) << 16 | byte_at(o + 2) << 8 | byte_at(o + 3);
-    }
-    uint32_t a = h[0], b = h[1], c = h[2], d = h[3], e = h[4], f = h[5], g = h[6], hh = h[7];
-#pragma unroll
-    for (int i = 0; i < 64; ++i) {
-      if (i >= 16) {
-        const uint32_t x = w[(i - 15) & 15], y = w[(i - 2) & 15];
-        w[i & 15] += (sha_rotr(x, 7) ^ sha_rotr(x, 18) ^ (x >> 3)) + w[(i - 7) & 15] +
-                     (sha_rotr(y, 17) ^ sha_rotr(y, 19) ^ (y >> 10));
-      }
-      const uint32_t t1 =
-          hh + (sha_rotr(e, 6) ^ sha_rotr(e, 11) ^ sha_rotr(e, 25)) + ((e & f) ^ (~e & g)) + kSha256K[i] + w[i & 15];
-      const uint32_t t2 = (sha_rotr(a, 2) ^ sha_rotr(a, 13) ^ sha_rotr(a, 22)) + ((a & b) ^ (a & c) ^ (b & c));
-      hh = g, g = f, f = e, e = d + t1, d = c, c = b, b = a, a = t1 + t2;
-    }
-    h[0] += a, h[1] += b, h[2] += c, h[3] += d, h[4] += e, h[5] += f, h[6] += g, h[7] += hh;
+// The fold with each product taken in full (121 lookups of a byte, against 16 of 16 bytes
+// in a table that costs a launch of its own): the cheaper one for few elements.
+__global__ void __launch_bounds__(kBThreads) k_fold128_direct(const uint4* __restrict__ cur, uint32_t len,
+                                                              uint32_t half, uint64_t r_lo, uint64_t r_hi,
+                                                              const uint8_t* __restrict__ d_r,
+                                                              const uint8_t* __restrict__ gT,
+                                                              uint4* __restrict__ next) {
+  extern __shared__ uint4 smem_b[];
+  uint8_t* s_T = reinterpret_cast<uint8_t*>(smem_b);
+  load_table(s_T, gT);
+  g128 r{r_lo, r_hi};
+  if (d_r) r = load_challenge(d_r);
+  __syncthreads();
+  const Tower F{s_T};
+  const uint4* src = cur + (size_t)blockIdx.y * len;
+  uint4* dst = next + (size_t)blockIdx.y * half;
+  for (uint32_t rest = blockIdx.x * blockDim.x + threadIdx.x; rest < half; rest += gridDim.x * blockDim.x) {
+    const g128 a = load_g128(src + 2 * (size_t)rest), b = load_g128(src + 2 * (size_t)rest + 1);
+    const g128 o = gxor(a, F.m128(r, gxor(a, b)));
+    dst[rest] = make_uint4((uint32_t)o.lo, (uint32_t)(o.lo >> 32), (uint32_t)o.hi, (uint32_t)(o.hi >> 32));
   }
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) out[4 * i + j] = (uint8_t)(h[i] >> (24 - 8 * j));
 }
 
-// The device transcript: the SHA-256 state (32 bytes) and the last challenge (1 or 16
-// bytes), in device memory between rounds.
-struct ScTranscript {
-  uint8_t state[32];
-  uint8_t r[16];
-};
-
-// Round `round`'s step. The points 0..n-1 lie in GF(2^8), so the Lagrange matrix `lag`
-// (n x n bytes) does too, and coefficient d = sum_i values[i] * lag[i][d] takes products by
-// a subfield scalar (one lookup over GF(2^8), 16 independent ones over GF(2^128)); one lane
-// per coefficient, the product table in global memory. The coefficients go to rounds_out;
-// the first round also forms the claimed sum (values[0] + values[1]) and starts the
-// transcript (from `seed`, or from the claimed sum); then thread 0 absorbs the
-// coefficients and samples the challenge (the digest's last byte over GF(2^8), its last
-// 16 bytes over GF(2^128)).
+// The last rounds of a proof in one CTA: the tables (m of `len` elements each, in `cur`)
+// come to shared memory and stay there, and each round is its values, the step and the
+// fold, a barrier apart; a round of few rows is otherwise three launches and as many loads
+// of the product table. A warp takes 32 rows (or 128) at one point at a time.
+// Shared memory: the product table, the tables, half as much for their folds.
+constexpr unsigned kTailThreads = 512;
+constexpr size_t kTailBytes = (size_t)64 << 10;  // of tables
 template <bool WIDE>
-__global__ void __launch_bounds__(64) k_sc_step(const uint8_t* __restrict__ vals, const uint8_t* __restrict__ lag,
-                                                uint32_t n, uint32_t round, const uint8_t* __restrict__ gT,
-                                                const uint8_t* __restrict__ seed, uint32_t seed_len, int has_seed,
-                                                ScTranscript* __restrict__ tx, uint8_t* __restrict__ claimed,
-                                                uint8_t* __restrict__ rounds_out) {
-  constexpr uint32_t ES = WIDE ? 16 : 1;
-  __shared__ uint8_t s_msg[32 + kProveMaxPoints * 16];  // the absorbed message: state || coefficients
-  const Tower F{gT};
-  for (uint32_t d = threadIdx.x; d < n; d += blockDim.x) {
-    uint8_t* out = s_msg + 32 + ES * d;
-    if constexpr (WIDE) {
-      uint64_t lo = 0, hi = 0;
-      for (uint32_t i = 0; i < n; ++i) {
-        const uint32_t c = lag[(size_t)i * n + d];
-        const uint8_t* v = vals + 16 * i;
-        uint64_t vlo = 0, vhi = 0;
+__global__ void __launch_bounds__(kTailThreads) k_sc_tail(const void* __restrict__ cur, uint32_t len, uint32_t m,
+                                                          uint32_t rounds, const __grid_constant__ Terms tm,
+                                                          const uint8_t* __restrict__ gT,
+                                                          const __grid_constant__ ScStep step) {
+  using E = typename std::conditional<WIDE, g128, uint8_t>::type;
+  constexpr uint32_t W = WIDE ? 4 : 1;
+  extern __shared__ uint4 smem_b[];
+  __shared__ StepShared s;
+  __shared__ uint32_t s_acc[kProveMaxPoints * W];
+  uint8_t* s_T = reinterpret_cast<uint8_t*>(smem_b);
+  load_table(s_T, gT);
+  const Tower F{s_T};
+  E* tab = reinterpret_cast<E*>(s_T + 65536);
+  E* nxt = reinterpret_cast<E*>(s_T + 65536 + (((size_t)m * len * sizeof(E) + 15) & ~(size_t)15));
+  // whole 16-byte words: the buffers are rounded up to them
+  for (uint32_t k = threadIdx.x; k < (m * len * sizeof(E) + 15) / 16; k += blockDim.x)
+    reinterpret_cast<uint4*>(tab)[k] = __ldcg(static_cast<const uint4*>(cur) + k);
+  const uint32_t n = step.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (uint32_t k = threadIdx.x; k < n * n; k += blockDim.x) s.lag[k] = step.lag[k];
+#pragma unroll 1
+  for (uint32_t i = 0; i < rounds; ++i, len >>= 1) {
+    const uint32_t half = len >> 1;
+    for (uint32_t k = threadIdx.x; k < n * W; k += blockDim.x) s_acc[k] = 0;
+    __syncthreads();
+    auto values = [&](auto rows_c) {
+      constexpr int kRows = decltype(rows_c)::value;  // rows per lane
+      const uint32_t groups = (half + 32 * kRows - 1) / (32 * kRows);
+#pragma unroll 1
+      for (uint32_t item = warp; item < groups * n; item += warps) {
+        const uint32_t t = item % n, rest = (item / n) * (32 * kRows) + lane;
+        E acc{};
+        for (uint32_t k = 0; k < tm.nterms; ++k) {
+          const uint32_t j0 = tm.off[k], j1 = tm.off[k + 1], kind = tm.kind[k];
+          if constexpr (WIDE) {
+            const uint64_t* cf = reinterpret_cast<const uint64_t*>(tm.coef + 16 * k);
+            const g128 c{cf[0], cf[1]};
+            if (rest < half) {
+              g128 prod = c;
+              for (uint32_t j = j0; j < j1; ++j) {
+                const g128* p = tab + (size_t)tm.idx[j] * len + 2 * rest;
+                const g128 v = at128(F, t, p[0], p[1]);
+                prod = j == j0 ? times_coef(F, kind, c, v) : F.m128(prod, v);
+              }
+              acc = gxor(acc, prod);
+            }
+          } else {
+            uint32_t prod[kRows];
 #pragma unroll
-        for (int b = 7; b >= 0; --b) vlo = (vlo << 8) | v[b], vhi = (vhi << 8) | v[8 + b];
-        lo ^= F.s64(c, vlo);
-        hi ^= F.s64(c, vhi);
+            for (int r = 0; r < kRows; ++r) prod[r] = tm.coef[k];
+            for (uint32_t j = j0; j < j1; ++j) {
+              const uint8_t* p = tab + (size_t)tm.idx[j] * len + 2 * rest;
+#pragma unroll
+              for (int r = 0; r < kRows; ++r) {
+                const bool in = rest + 32 * r < half;
+                const uint32_t v = at8(F, t, in ? p[64 * r] : 0, in ? p[64 * r + 1] : 0);
+                prod[r] = (j == j0 && kind == 0) ? v : F.m8(prod[r], v);
+              }
+            }
+#pragma unroll
+            for (int r = 0; r < kRows; ++r)
+              if (rest + 32 * r < half) acc ^= (uint8_t)prod[r];
+          }
+        }
+        if constexpr (WIDE)
+          warp_xor_into128(acc, s_acc + 4 * t);
+        else
+          warp_xor_into(acc, s_acc + t);
       }
-#pragma unroll
-      for (int b = 0; b < 8; ++b) out[b] = (uint8_t)(lo >> (8 * b)), out[8 + b] = (uint8_t)(hi >> (8 * b));
-    } else {
-      uint32_t acc = 0;
-      for (uint32_t i = 0; i < n; ++i) acc ^= F.m8(lag[(size_t)i * n + d], vals[i]);
-      out[0] = (uint8_t)acc;
-    }
-    for (uint32_t b = 0; b < ES; ++b) rounds_out[((size_t)round * n + d) * ES + b] = out[b];
-  }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  if (round == 0) {
-    uint8_t h[16];
-    for (uint32_t b = 0; b < ES; ++b) {  // one point: the sum of 2^k copies of a constant is 0
-      h[b] = n >= 2 ? (uint8_t)(vals[b] ^ vals[ES + b]) : 0;
-      claimed[b] = h[b];
-    }
-    if (has_seed)
-      sha256_dev(seed, seed_len, nullptr, 0, s_msg);
+    };
+    // over GF(2^8) four rows per lane while there are as many: byte lookups are latency otherwise
+    if (!WIDE && half > 64)
+      values(std::integral_constant<int, 4>{});
     else
-      sha256_dev(h, ES, nullptr, 0, s_msg);
-  } else {
-    for (int b = 0; b < 32; ++b) s_msg[b] = tx->state[b];
+      values(std::integral_constant<int, 1>{});
+    __syncthreads();
+    if (warp == 0) {
+      for (uint32_t k = lane; k < n * W; k += 32) {
+        if constexpr (WIDE)
+          reinterpret_cast<uint32_t*>(s.vals)[k] = s_acc[k];
+        else
+          s.vals[k] = (uint8_t)s_acc[k];
+      }
+      __syncwarp();
+      sc_step<WIDE>(s, step, step.round + i, i > 0, F);  // leaves the challenge at the digest's end
+    }
+    __syncthreads();
+    if (i + 1 == rounds) break;
+    const uint8_t* d = s.msg + (WIDE ? 16 : 31);
+    if constexpr (WIDE) {
+      const g128 r = load_challenge(d);
+      for (uint32_t k = threadIdx.x; k < m * half; k += blockDim.x) {
+        const g128 a = tab[2 * k], b = tab[2 * k + 1];  // table f's rows follow table f - 1's
+        nxt[k] = gxor(a, F.m128(r, gxor(a, b)));
+      }
+    } else {
+      const uint32_t r = d[0];
+      for (uint32_t k = threadIdx.x; k < m * half; k += blockDim.x) {
+        const uint32_t a = tab[2 * k], b = tab[2 * k + 1];
+        nxt[k] = (uint8_t)(a ^ F.m8(r, a ^ b));
+      }
+    }
+    __syncthreads();
+    E* const old = tab;
+    tab = nxt;
+    nxt = old;
   }
-  uint8_t st[32];
-  sha256_dev(s_msg, 32 + n * ES, nullptr, 0, st);
-  for (int b = 0; b < 32; ++b) tx->state[b] = st[b];
-  for (uint32_t b = 0; b < ES; ++b) tx->r[b] = WIDE ? st[16 + b] : st[31];
 }
 
 // ---- host: argument checks and launches -------------------------------------------
@@ -660,6 +879,7 @@ const void* const kValues128[kRegPoints + 1] = {
     (const void*)k_values128<3>, (const void*)k_values128<4>, (const void*)k_values128<5>,
     (const void*)k_values128<6>, (const void*)k_values128<7>, (const void*)k_values128<8>};
 constexpr size_t kValuesSmem = 65536 + 16 * (kMaxPoint + 1);
+constexpr size_t kTailSmem = 65536 + kTailBytes + kTailBytes / 2 + 32;
 
 // Per device, set up on first use: the product table, the SM count, the kernels' shared
 // memory limits and how many CTAs of each fit on an SM.
@@ -690,6 +910,9 @@ const DeviceState& device_state(cudaStream_t st) {
     }
     ZS_CUDA(cudaFuncSetAttribute(k_mul_table128, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
     ZS_CUDA(cudaFuncSetAttribute(k_fold128, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
+    ZS_CUDA(cudaFuncSetAttribute(k_fold128_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
+    for (const void* fn : {(const void*)k_sc_tail<false>, (const void*)k_sc_tail<true>})
+      ZS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));
     uint8_t* t = nullptr;
     ZS_CUDA(cudaMalloc(&t, 65536));
     ZS_CUDA(cudaMemcpyAsync(t, host_tower().T.data(), 65536, cudaMemcpyHostToDevice, st));
@@ -699,14 +922,16 @@ const DeviceState& device_state(cudaStream_t st) {
   return d;
 }
 
-// Zeroes d_out and accumulates one round's values into it, asynchronously on `st`. With
+// Accumulates one round's values into d_out, asynchronously on `st`, and takes the round's
+// step when one is given (d_out is zero before and after then; it is zeroed here
+// otherwise). With
 // enough rows to give every SM a CTA, each thread takes all points of its rows (up to
 // eight; one point per pass beyond that); with fewer rows, the points get CTAs of their
 // own (a grid of dmax + 1 rows), so that small rounds still spread over the GPU.
 void values_async(bool wide, const void* d_cur, size_t len, size_t half, size_t dmax, const Terms& tm, void* d_out,
-                  cudaStream_t st) {
+                  const ScStep& step, cudaStream_t st) {
   const size_t words = wide ? 4 * (dmax + 1) : (dmax + 4) / 4;
-  ZS_CUDA(cudaMemsetAsync(d_out, 0, words * 4, st));
+  if (!step.tx) ZS_CUDA(cudaMemsetAsync(d_out, 0, words * 4, st));
   if (half == 0) return;
   const DeviceState& ds = device_state(st);
   const int D = dmax + 1 <= (size_t)kRegPoints ? (int)dmax + 1 : 0;
@@ -725,11 +950,12 @@ void values_async(bool wide, const void* d_cur, size_t len, size_t half, size_t 
   uint32_t L = (uint32_t)len, H = (uint32_t)half, M = (uint32_t)dmax;
   const uint8_t* T = ds.table;
   uint32_t* out = static_cast<uint32_t*>(d_out);
-  void* args[] = {&cur, &L, &H, &M, const_cast<Terms*>(&tm), &T, &out};
+  void* args[] = {&cur, &L, &H, &M, const_cast<Terms*>(&tm), &T, &out, const_cast<ScStep*>(&step)};
   ZS_CUDA(cudaLaunchKernel(wide ? kValues128[kd] : kValues8[kd], grid, dim3(kBThreads), args, 65536 + 4 * words,
                            st));
 }
 
+constexpr size_t kDirectFold = (size_t)1 << 16;  // elements up to which the direct fold is used
 // next (m tables of len / 2) = fold of cur (m tables of len) at r, asynchronously on `st`.
 // r_mul: a 64 KB device buffer for the GF(2^128) multiply table.
 void fold_async(bool wide, const void* d_cur, size_t len, size_t m, u128 r, const uint8_t* d_r, void* d_next,
@@ -743,6 +969,10 @@ void fold_async(bool wide, const void* d_cur, size_t len, size_t m, u128 r, cons
   if (!wide) {
     k_fold8<<<grid, kBThreads, 0, st>>>(static_cast<const uint8_t*>(d_cur), (uint32_t)len, (uint32_t)half,
                                         (uint32_t)r, d_r, ds.table, static_cast<uint8_t*>(d_next));
+  } else if (m * half <= kDirectFold) {
+    k_fold128_direct<<<grid, kBThreads, 65536, st>>>(static_cast<const uint4*>(d_cur), (uint32_t)len, (uint32_t)half,
+                                                     (uint64_t)r, (uint64_t)(r >> 64), d_r, ds.table,
+                                                     static_cast<uint4*>(d_next));
   } else {
     k_mul_table128<<<4096 / kBThreads, kBThreads, 65536, st>>>((uint64_t)r, (uint64_t)(r >> 64), d_r, ds.table, r_mul);
     k_fold128<<<grid, kBThreads, 65536, st>>>(static_cast<const uint4*>(d_cur), (uint32_t)len, (uint32_t)half,
@@ -794,7 +1024,7 @@ int32_t hook_values(bool wide, const uint8_t* cur_flat, size_t len, size_t m, co
     DevMem<uint4> d_cur((m * len * es + 15) / 16, st);
     DevMem<uint32_t> d_out(words, st);
     if (m * len) ZS_CUDA(cudaMemcpyAsync(d_cur.p, cur_flat, m * len * es, cudaMemcpyHostToDevice, st));
-    values_async(wide, d_cur.p, len, half, dmax, tm, d_out.p, st);
+    values_async(wide, d_cur.p, len, half, dmax, tm, d_out.p, {}, st);
     std::vector<uint32_t> h(words);
     ZS_CUDA(cudaMemcpyAsync(h.data(), d_out.p, words * 4, cudaMemcpyDeviceToHost, st));
     ZS_CUDA(cudaStreamSynchronize(st));
@@ -838,6 +1068,19 @@ std::vector<std::vector<u128>> lagrange_matrix(const HostTower& ht, unsigned lev
   return lag;
 }
 
+// Table lookups per row of a round (its values at `pts` points and the folds of the m tables).
+uint64_t tail_row_cost(bool wide, size_t m, const Terms& tm, size_t pts) {
+  const uint64_t mul = wide ? 121 : 1, scale = wide ? 16 : 1;
+  uint64_t c = m * mul;
+  for (uint32_t k = 0; k < tm.nterms; ++k) {
+    const uint64_t f = tm.off[k + 1] - tm.off[k];
+    c += pts * (f == 0 ? 1 : (f - 1) * mul + (tm.kind[k] == 0 ? 0 : tm.kind[k] == 1 ? scale : mul));
+    for (size_t t = 4; t < pts; ++t) c += f * scale;
+  }
+  return c;
+}
+constexpr uint64_t kTailCost = (uint64_t)3 << 14;
+
 int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, size_t m, const uint8_t* coeffs,
                           size_t nterms, const uint32_t* indices, size_t n_indices, const uint32_t* offsets,
                           const uint8_t* seed, size_t seed_len, int32_t has_seed, uint8_t* claimed_out,
@@ -872,49 +1115,66 @@ int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, 
 
     cudaStream_t st = (cudaStream_t)stream;
     retain_pool_memory();
+    PinnedScope pinned(st);
     const size_t words = wide ? 4 * (dmax + 1) : (dmax + 4) / 4;
     DevMem<uint4> d_a((m * n * es + 15) / 16, st), d_b((m * (n / 2) * es + 15) / 16, st);
-    DevMem<uint32_t> d_vals(words, st);
-    DevMem<uint4> d_rmul(wide ? 4096 : 0, st);
-    // the device transcript's inputs and outputs: the Lagrange matrix, the seed, the
-    // state and challenge, the claimed sum and every round's coefficients
+    DevMem<uint4> d_rmul(wide && m * (n / 2) > kDirectFold ? 4096 : 0, st);
     const size_t pts = dmax + 1;
     std::vector<uint8_t> lag_b(pts * pts);  // GF(2^8) entries: the points lie in GF(2^8)
     for (size_t a = 0; a < pts; ++a)
       for (size_t d = 0; d < pts; ++d) lag_b[a * pts + d] = (uint8_t)lag[a][d];
-    DevMem<uint8_t> d_lag(lag_b.size(), st), d_seed(has_seed ? seed_len : 0, st), d_claimed(es, st),
-        d_rounds(k * pts * es, st);
-    DevMem<ScTranscript> d_tx(1, st);
-    ZS_CUDA(cudaMemcpyAsync(d_lag.p, lag_b.data(), lag_b.size(), cudaMemcpyHostToDevice, st));
-    if (has_seed && seed_len) ZS_CUDA(cudaMemcpyAsync(d_seed.p, seed, seed_len, cudaMemcpyHostToDevice, st));
+    // One block for the device transcript's inputs and outputs: the values' accumulators and
+    // the counter (zero between rounds), the state and challenge, the Lagrange matrix, the
+    // seed, the claimed sum and every round's coefficients.
+    size_t at = 0;
+    auto part = [&](size_t bytes) {
+      const size_t o = at;
+      at += (bytes + 15) & ~(size_t)15;
+      return o;
+    };
+    const size_t o_vals = part(words * 4), o_done = part(4), o_tx = part(sizeof(ScTranscript)),
+                 o_lag = part(lag_b.size()), o_seed = part(has_seed ? seed_len : 0), o_claimed = part(es),
+                 o_rounds = part(k * pts * es);
+    DevMem<uint4> d_aux(at / 16, st);
+    uint8_t* const aux = reinterpret_cast<uint8_t*>(d_aux.p);
+    ZS_CUDA(cudaMemsetAsync(aux, 0, o_tx, st));
+    h2d_small(aux + o_lag, lag_b.data(), lag_b.size(), st);
+    if (has_seed && seed_len) ZS_CUDA(cudaMemcpyAsync(aux + o_seed, seed, seed_len, cudaMemcpyHostToDevice, st));
     ZS_CUDA(cudaMemcpyAsync(d_a.p, tables, m * n * es, cudaMemcpyHostToDevice, st));
     const uint8_t* T = device_state(st).table;
+    ScStep step{};
+    step.tx = reinterpret_cast<ScTranscript*>(aux + o_tx);
+    step.done = reinterpret_cast<uint32_t*>(aux + o_done);
+    step.lag = aux + o_lag, step.seed = aux + o_seed, step.claimed = aux + o_claimed, step.rounds_out = aux + o_rounds;
+    step.n = (uint32_t)pts, step.seed_len = (uint32_t)seed_len, step.has_seed = has_seed ? 1 : 0;
 
-    // every round on the device, back to back: values, the transcript step, the fold
+    // every round on the device, back to back: values with the transcript step, the fold;
+    // the last ones in one CTA
+    const uint64_t row_cost = tail_row_cost(wide, m, tm, pts);
     void* cur = d_a.p;
     void* nxt = d_b.p;
     size_t len = n;
     for (size_t i = 0; i < k; ++i) {
       const size_t half = len / 2;
-      values_async(wide, cur, len, half, dmax, tm, d_vals.p, st);
-      const uint8_t* vb = reinterpret_cast<const uint8_t*>(d_vals.p);
-      if (wide)
-        k_sc_step<true><<<1, 64, 0, st>>>(vb, d_lag.p, (uint32_t)pts, (uint32_t)i, T, d_seed.p, (uint32_t)seed_len,
-                                          has_seed ? 1 : 0, d_tx.p, d_claimed.p, d_rounds.p);
-      else
-        k_sc_step<false><<<1, 64, 0, st>>>(vb, d_lag.p, (uint32_t)pts, (uint32_t)i, T, d_seed.p, (uint32_t)seed_len,
-                                           has_seed ? 1 : 0, d_tx.p, d_claimed.p, d_rounds.p);
-      ZS_CUDA(cudaGetLastError());
+      step.round = (uint32_t)i;
+      if (m * len * es <= kTailBytes && half * row_cost <= kTailCost) {
+        const size_t smem = 65536 + ((m * len * es + 15) & ~(size_t)15) + ((m * half * es + 15) & ~(size_t)15);
+        if (wide)
+          k_sc_tail<true><<<1, kTailThreads, smem, st>>>(cur, (uint32_t)len, (uint32_t)m, (uint32_t)(k - i), tm, T, step);
+        else
+          k_sc_tail<false><<<1, kTailThreads, smem, st>>>(cur, (uint32_t)len, (uint32_t)m, (uint32_t)(k - i), tm, T, step);
+        ZS_CUDA(cudaGetLastError());
+        break;
+      }
+      values_async(wide, cur, len, half, dmax, tm, aux + o_vals, step, st);
       if (i + 1 < k) {
-        fold_async(wide, cur, len, m, 0, reinterpret_cast<const uint8_t*>(d_tx.p) + offsetof(ScTranscript, r), nxt,
-                   d_rmul.p, st);
+        fold_async(wide, cur, len, m, 0, aux + o_tx + offsetof(ScTranscript, r), nxt, d_rmul.p, st);
         std::swap(cur, nxt);
       }
       len = half;
     }
-    ZS_CUDA(cudaMemcpyAsync(claimed_out, d_claimed.p, es, cudaMemcpyDeviceToHost, st));
-    ZS_CUDA(cudaMemcpyAsync(rounds_out, d_rounds.p, k * pts * es, cudaMemcpyDeviceToHost, st));
-    ZS_CUDA(cudaStreamSynchronize(st));
+    const D2H back[2] = {{claimed_out, aux + o_claimed, es}, {rounds_out, aux + o_rounds, k * pts * es}};
+    d2h_many(back, 2, st);
   });
 }
 
@@ -948,7 +1208,7 @@ extern "C" int32_t zs_binius_sumcheck_values_device(uint32_t field_bits, const v
       throw zs::Error(zs::ZS_EMALFORMED, "misaligned buffer");
     zs::check_rows(len, half, dmax);
     const zs::Terms tm = zs::pack_terms(wide, m, coeffs, nterms, indices, n_indices, offsets);
-    zs::values_async(wide, d_cur, len, half, dmax, tm, d_out, (cudaStream_t)stream);
+    zs::values_async(wide, d_cur, len, half, dmax, tm, d_out, {}, (cudaStream_t)stream);
   });
 }
 
