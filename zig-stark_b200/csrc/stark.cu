@@ -460,21 +460,12 @@ const FoldTables& fold_tables(unsigned dlog, cudaStream_t st, std::unique_ptr<Fo
   return cached_table<FoldTables>(dlog, [&](cudaStream_t s) { return new FoldTables(dlog, s); });
 }
 
-// FRI_OFFSET^k for k < 2^log_n.
-struct OffsetPowers {
-  qm31* p = nullptr;
-  OffsetPowers(unsigned log_n, cudaStream_t s) {
-    ZS_CUDA(cudaMallocAsync(&p, sizeof(qm31) << log_n, s));
-    qm31_powers(q_fri_offset(), p, 1u << log_n, s);
-  }
-};
-const qm31* offset_powers(unsigned log_n, cudaStream_t st, std::unique_ptr<DevBuf<qm31>>& own) {
+const OffsetTable& offset_table(unsigned log_n, cudaStream_t st, std::unique_ptr<OffsetTable>& own) {
   if (log_n > kCacheLog) {
-    own = std::make_unique<DevBuf<qm31>>((size_t)1 << log_n, st);
-    qm31_powers(q_fri_offset(), own->p, 1u << log_n, st);
-    return own->p;
+    own = std::make_unique<OffsetTable>(log_n, st);
+    return *own;
   }
-  return cached_table<OffsetPowers>(log_n, [&](cudaStream_t s) { return new OffsetPowers(log_n, s); }).p;
+  return cached_table<OffsetTable>(log_n, [&](cudaStream_t s) { return new OffsetTable(log_n, s); });
 }
 
 // The roots of trees[a, b), read back with one wait.
@@ -669,10 +660,10 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   // ---- LDE of preprocessed and main columns ------------------------------------
   const uint32_t ncol = n_pre + m_total;  // [pre | main | acc]
   std::unique_ptr<NttTables> small_own, big_own;
-  std::unique_ptr<DevBuf<qm31>> pows_own;
+  std::unique_ptr<OffsetTable> offset_own;
   const NttTables& small = ntt_tables(tl, st, small_own);
   const NttTables& big = ntt_tables(lN, st, big_own);
-  const qm31* offset_pows = offset_powers(tl, st, pows_own);
+  const OffsetTable& offset_pows = offset_table(tl, st, offset_own);
   DevBuf<qm31> vals((size_t)ncol * n, st), coeffs((size_t)ncol * n, st), cw((size_t)ncol * N, st);
   TreeCounters done((size_t)ncol + 1 + L, st);  // the columns', the quotient's and the FRI layers' trees
   std::vector<std::unique_ptr<OwnedTree>> trees;
@@ -1084,10 +1075,10 @@ std::vector<uint8_t> commit_columns(const uint8_t* cols_b, size_t cols_len, unsi
   out.u64(C);
   if (C == 0) return out.out;
   std::unique_ptr<NttTables> small_own, big_own;
-  std::unique_ptr<DevBuf<qm31>> pows_own;
+  std::unique_ptr<OffsetTable> offset_own;
   const NttTables& small = ntt_tables(trace_log, st, small_own);
   const NttTables& big = ntt_tables(lN, st, big_own);
-  const qm31* offset_pows = offset_powers(trace_log, st, pows_own);
+  const OffsetTable& offset_pows = offset_table(trace_log, st, offset_own);
   DevBuf<qm31> vals((size_t)C * n, st), coeffs((size_t)C * n, st), cw((size_t)C * N, st);
   upload_columns(cols, vals.p, n, st);
   lde_qm31(vals.p, n, coeffs.p, n, cw.p, N, C, small, big, offset_pows, st);
