@@ -22,9 +22,15 @@ constexpr unsigned kThreads = 256;
 // Row leaves hashM31s(col_0[r], ..., col_{C-1}[r]) (src/m31/hash.zig:15-25), and
 // optionally g[r] = sum_c gammas[c] * col_c[r]. The four
 // coordinates of g accumulate unreduced 62-bit products in 64 bits (one wide
-// multiply-add each) with a Mersenne fold every four columns: after a fold the
-// accumulator is below 2^34, and four products below (p-1)^2 keep it below 2^64.
+// multiply-add each). p 2^32 is a multiple of p, so where the high word has reached p it can
+// be taken off there: one ALU operation (a minimum) after every second product, where a
+// Mersenne fold of 64 bits takes five after every fourth. After it the high word is at most
+// p + 1, and two products of words below p keep the sum below 2^64.
 __device__ __forceinline__ uint64_t fold64(uint64_t x) { return (x & P) + (x >> 31); }
+__device__ __forceinline__ uint64_t fold_high(uint64_t x) {
+  const uint32_t hi = (uint32_t)(x >> 32);
+  return (uint64_t)umin32(hi, hi - P) << 32 | (uint32_t)x;
+}
 __device__ __forceinline__ uint32_t canon64(uint64_t x) {
   x = fold64(fold64(x));  // < 2^31 + 8
   const uint32_t s = (uint32_t)x;
@@ -73,11 +79,11 @@ __global__ void __launch_bounds__(kThreads) k_row_leaves(const uint32_t* __restr
           acc2 += (uint64_t)g.z * v;
           acc3 += (uint64_t)g.w * v;
         }
-        if ((k & 3) == 3) {
-          acc0 = fold64(acc0);
-          acc1 = fold64(acc1);
-          acc2 = fold64(acc2);
-          acc3 = fold64(acc3);
+        if (k & 1) {
+          acc0 = fold_high(acc0);
+          acc1 = fold_high(acc1);
+          acc2 = fold_high(acc2);
+          acc3 = fold_high(acc3);
         }
       }
     }
