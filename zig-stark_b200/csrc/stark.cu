@@ -394,22 +394,45 @@ Digest root_of(const DeviceTree& t, cudaStream_t st) {
   return d;
 }
 
-struct OwnedTree {
-  DeviceTree t;
-  cudaStream_t st;
-  OwnedTree(unsigned log_n, uint32_t* done, cudaStream_t s) : st(s) {
-    t.log_n = log_n, t.done = done;
-    ZS_CUDA(cudaMallocAsync((void**)&t.words, DeviceTree::words_for(log_n) * sizeof(uint32_t), s));
+// The trees of a proof's columns (one size), in one allocation with their counters: a wide
+// proof has hundreds, and a stream-ordered allocation and free takes 2-3 us of the host's
+// time each (1.9 ms of a 387-column proof).
+struct OwnedTrees {
+  std::vector<DeviceTree> t;
+  OwnedTrees(uint32_t count, unsigned log_n, cudaStream_t s)
+      : t(count), words((size_t)count * tree_words(log_n), s), done(count, s) {
+    ZS_CUDA(cudaMemsetAsync(done.p, 0, count * sizeof(uint32_t), s));
+    for (uint32_t j = 0; j < count; ++j) {
+      t[j].log_n = log_n;
+      t[j].words = words.p + (size_t)j * tree_words(log_n);
+      t[j].done = done.p + j;
+    }
   }
-  ~OwnedTree() { cudaFreeAsync(t.words, st); }
+  static size_t tree_words(unsigned log_n) { return (DeviceTree::words_for(log_n) + 63) & ~(size_t)63; }
+
+ private:
+  DevBuf<uint32_t> words, done;
 };
 
-// The counters of `count` trees (DeviceTree::done), zeroed on the stream.
-struct TreeCounters {
-  DevBuf<uint32_t> d;
-  TreeCounters(size_t count, cudaStream_t s) : d(count, s) {
-    ZS_CUDA(cudaMemsetAsync(d.p, 0, count * sizeof(uint32_t), s));
+// The trees of the FRI layers (2^log_n leaves and down), likewise.
+struct LayerTrees {
+  std::vector<DeviceTree> t;
+  LayerTrees(uint32_t count, unsigned log_n, cudaStream_t s) : t(count), words(offset(count, log_n), s), done(count, s) {
+    ZS_CUDA(cudaMemsetAsync(done.p, 0, count * sizeof(uint32_t), s));
+    for (uint32_t i = 0; i < count; ++i) {
+      t[i].log_n = log_n - i;
+      t[i].words = words.p + offset(i, log_n);
+      t[i].done = done.p + i;
+    }
   }
+
+ private:
+  static size_t offset(uint32_t i, unsigned log_n) {  // of layer i's tree
+    size_t o = 0;
+    for (uint32_t k = 0; k < i; ++k) o += OwnedTrees::tree_words(log_n - k);
+    return o;
+  }
+  DevBuf<uint32_t> words, done;
 };
 
 // Size-only tables (NTT twiddles, powers of FRI_OFFSET, fold tables) of sizes up to
@@ -469,19 +492,18 @@ const OffsetTable& offset_table(unsigned log_n, cudaStream_t st, std::unique_ptr
 }
 
 // The roots of trees[a, b), read back with one wait.
-std::vector<Digest> roots_of(const std::vector<std::unique_ptr<OwnedTree>>& trees, uint32_t a, uint32_t b,
-                             cudaStream_t st) {
+std::vector<Digest> roots_of(const std::vector<DeviceTree>& trees, uint32_t a, uint32_t b, cudaStream_t st) {
   std::vector<Digest> out(b - a);
   std::vector<D2H> c;
-  for (uint32_t j = a; j < b; ++j) c.push_back({out[j - a].data(), trees[j]->t.root(), 32});
+  for (uint32_t j = a; j < b; ++j) c.push_back({out[j - a].data(), trees[j].root(), 32});
   d2h_many(c.data(), c.size(), st);
   return out;
 }
 
 // The DeviceTree pointers of trees[a, b).
-std::vector<DeviceTree*> tree_ptrs(const std::vector<std::unique_ptr<OwnedTree>>& trees, uint32_t a, uint32_t b) {
+std::vector<DeviceTree*> tree_ptrs(std::vector<DeviceTree>& trees, uint32_t a, uint32_t b) {
   std::vector<DeviceTree*> v;
-  for (uint32_t j = a; j < b; ++j) v.push_back(&trees[j]->t);
+  for (uint32_t j = a; j < b; ++j) v.push_back(&trees[j]);
   return v;
 }
 
@@ -665,9 +687,8 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   const NttTables& big = ntt_tables(lN, st, big_own);
   const OffsetTable& offset_pows = offset_table(tl, st, offset_own);
   DevBuf<qm31> vals((size_t)ncol * n, st), coeffs((size_t)ncol * n, st), cw((size_t)ncol * N, st);
-  TreeCounters done((size_t)ncol + 1 + L, st);  // the columns', the quotient's and the FRI layers' trees
-  std::vector<std::unique_ptr<OwnedTree>> trees;
-  for (uint32_t j = 0; j < ncol; ++j) trees.push_back(std::make_unique<OwnedTree>(lN, done.d.p + j, st));
+  OwnedTrees owned(ncol + 1, lN, st);  // the columns' and the quotient's
+  std::vector<DeviceTree>& trees = owned.t;
   {
     // Columns [pre | main] in groups: group g+1 is packed on the host and copied on a
     // copy stream while the LDE of group g runs on `st` and its trees on a side stream
@@ -840,9 +861,9 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
     k_quotient<<<(N + kT - 1) / kT, kT, 0, st>>>(cw.p, q.p, big.fwd, d_kc.p, zh_tab.p, per_tab.p);
   }
   ZS_CUDA(cudaGetLastError());
-  OwnedTree qtree(lN, done.d.p + ncol, st);
-  build_qm31_tree(q.p, qtree.t, st);
-  const Digest qroot = root_of(qtree.t, st);
+  DeviceTree& qtree = trees[ncol];
+  build_qm31_tree(q.p, qtree, st);
+  const Digest qroot = root_of(qtree, st);
   ch.absorb(qroot);
   proof.digest(qroot);
 
@@ -887,15 +908,16 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   h2d_small(d_dc.p, &dc, sizeof(dc), st);
   DevBuf<qm31> d_ge(ge.size(), st);
   h2d_small(d_ge.p, ge.data(), ge.size() * sizeof(qm31), st);
-  std::vector<std::unique_ptr<DevBuf<qm31>>> layers;
-  layers.push_back(std::make_unique<DevBuf<qm31>>(N, st));
-  k_deep<<<(N + kT - 1) / kT, kT, 0, st>>>(cw.p, q.p, big.fwd, d_dc.p, d_ge.p, layers[0]->p);
+  DevBuf<qm31> layer_mem((size_t)2 * N, st);  // layer i holds N >> i values after the layers before it
+  std::vector<qm31*> layers(L + 1);
+  for (unsigned i = 0; i <= L; ++i) layers[i] = layer_mem.p + ((size_t)2 * N - ((size_t)2 * N >> i));
+  k_deep<<<(N + kT - 1) / kT, kT, 0, st>>>(cw.p, q.p, big.fwd, d_dc.p, d_ge.p, layers[0]);
   ZS_CUDA(cudaGetLastError());
 
   std::unique_ptr<FoldTables> ftabs_own;
   const FoldTables& ftabs = fold_tables(lN, st, ftabs_own);
-  std::vector<std::unique_ptr<OwnedTree>> ftrees;
-  for (unsigned i = 0; i < L; ++i) ftrees.push_back(std::make_unique<OwnedTree>(lN - i, done.d.p + ncol + 1 + i, st));
+  LayerTrees fri_owned(L, lN, st);
+  std::vector<DeviceTree>& ftrees = fri_owned.t;
   // The commit phase (fri.zig:195-227) runs without host round trips: the CTA that finishes
   // a layer's tree absorbs the root into the device copy of the transcript and samples the
   // folding challenge, and the next layer's launch folds with it, hashes and builds its
@@ -913,16 +935,15 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
     h2d_small(d_ch.p, &ch, sizeof(Channel), st);
     DevBuf<qm31> d_alpha(L, st);
     DevBuf<uint32_t> d_roots((size_t)8 * L, st);
-    for (unsigned i = 0; i < L; ++i) layers.push_back(std::make_unique<DevBuf<qm31>>(N >> (i + 1), st));
     for (unsigned i = 0; i < tail; ++i) {
       const TranscriptStep tx{d_ch.p, d_alpha.p + i};
-      ftrees[i]->t.root_out = d_roots.p + 8 * i;
+      ftrees[i].root_out = d_roots.p + 8 * i;
       if (i == 0) {
-        build_qm31_tree(layers[0]->p, ftrees[0]->t, st, &tx);
+        build_qm31_tree(layers[0], ftrees[0], st, &tx);
       } else {
-        const FoldSource f{layers[i - 1]->p, layers[i]->p, d_alpha.p + i - 1, ftabs.tables, ftabs.offset_inv(i - 1),
+        const FoldSource f{layers[i - 1], layers[i], d_alpha.p + i - 1, ftabs.tables, ftabs.offset_inv(i - 1),
                            N >> i, i - 1};
-        build_fold_tree(f, ftrees[i]->t, st, &tx);
+        build_fold_tree(f, ftrees[i], st, &tx);
       }
     }
     DevBuf<FriTail> d_tail(1, st);
@@ -930,26 +951,26 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
       FriTail ft{};
       ft.first = tail, ft.count = L - tail, ft.log_size = lN - tail, ft.tables = ftabs.tables;
       for (unsigned c = 0; c <= ft.count + 1; ++c)
-        ft.layer[c] = tail + c > 0 ? layers[tail + c - 1]->p : nullptr;
+        ft.layer[c] = tail + c > 0 ? layers[tail + c - 1] : nullptr;
       for (unsigned c = 0; c <= ft.count; ++c)
         ft.off_inv[c] = tail + c > 0 ? ftabs.offset_inv(tail + c - 1) : qzero();
-      for (unsigned c = 0; c < ft.count; ++c) ft.tree[c] = ftrees[tail + c]->t.words;
+      for (unsigned c = 0; c < ft.count; ++c) ft.tree[c] = ftrees[tail + c].words;
       ft.roots = d_roots.p + 8 * tail;
       ft.alphas = d_alpha.p + tail;
       h2d_small(d_tail.p, &ft, sizeof(ft), st);
       fri_tail(d_tail.p, d_ch.p, st);
     } else {
-      fri_fold(layers[L - 1]->p, layers[L]->p, N >> L, qzero(), d_alpha.p + L - 1, L - 1, ftabs, st);
+      fri_fold(layers[L - 1], layers[L], N >> L, qzero(), d_alpha.p + L - 1, L - 1, ftabs, st);
     }
     std::vector<uint32_t> words((size_t)8 * L);
     const D2H back[3] = {{&ch, d_ch.p, sizeof(Channel)},  // the transcript continues on the host
                          {words.data(), d_roots.p, words.size() * sizeof(uint32_t)},
-                         {last.data(), layers[L]->p, rem * sizeof(qm31)}};
+                         {last.data(), layers[L], rem * sizeof(qm31)}};
     d2h_many(back, 3, st);
     for (unsigned i = 0; i < L; ++i)
       for (int b = 0; b < 32; ++b) froots[i][b] = (uint8_t)(words[8 * i + b / 4] >> (8 * (b % 4)));
   } else {
-    d2h_small(last.data(), layers[L]->p, rem * sizeof(qm31), st);
+    d2h_small(last.data(), layers[L], rem * sizeof(qm31), st);
   }
   std::vector<qm31> xs(rem);
   {
@@ -984,10 +1005,10 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   // 2^(lN-i-1), then their two paths
   for (unsigned i = 0; i < L; ++i) {
     const unsigned ml = lN - (i + 1);
-    want(0, layers[i]->p, 4, kQLow, ml, kQValue);
-    want(0, layers[i]->p, 4, kQHigh, ml, kQValue);
-    want_path(0, ftrees[i]->t, kQLow, ml);
-    want_path(0, ftrees[i]->t, kQHigh, ml);
+    want(0, layers[i], 4, kQLow, ml, kQValue);
+    want(0, layers[i], 4, kQHigh, ml, kQValue);
+    want_path(0, ftrees[i], kQLow, ml);
+    want_path(0, ftrees[i], kQHigh, ml);
   }
   // STARK reveals, per query: the values (columns at p0, columns at p0 + shift, the
   // quotient, preprocessed columns), then their paths in the same order
@@ -995,10 +1016,10 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   for (uint32_t j = 0; j < m_total; ++j) want(1, cw.p + (size_t)(n_pre + j) * N, 4, kQShift, lN, kQValue);
   want(1, q.p, 4, kQP0, lN, kQValue);
   for (uint32_t j = 0; j < n_pre; ++j) want(1, cw.p + (size_t)j * N, 4, kQP0, lN, kQValue);
-  for (uint32_t j = 0; j < m_total; ++j) want_path(1, trees[n_pre + j]->t, kQP0, lN);
-  for (uint32_t j = 0; j < m_total; ++j) want_path(1, trees[n_pre + j]->t, kQShift, lN);
-  want_path(1, qtree.t, kQP0, lN);
-  for (uint32_t j = 0; j < n_pre; ++j) want_path(1, trees[j]->t, kQP0, lN);
+  for (uint32_t j = 0; j < m_total; ++j) want_path(1, trees[n_pre + j], kQP0, lN);
+  for (uint32_t j = 0; j < m_total; ++j) want_path(1, trees[n_pre + j], kQShift, lN);
+  want_path(1, qtree, kQP0, lN);
+  for (uint32_t j = 0; j < n_pre; ++j) want_path(1, trees[j], kQP0, lN);
   const uint32_t nq = (uint32_t)sp.num_queries;
   const size_t off = (size_t)nq * (sec_words[0] + sec_words[1]);
   std::vector<uint32_t> gathered(off);
@@ -1085,9 +1106,8 @@ std::vector<uint8_t> commit_columns(const uint8_t* cols_b, size_t cols_len, unsi
   // trees of up to 1 GiB in all are built together, then their roots read back
   const size_t tree_bytes = DeviceTree::words_for(lN) * sizeof(uint32_t);
   const uint32_t per = (uint32_t)std::max<size_t>(1, std::min<size_t>(kTreeBatch, ((size_t)1 << 30) / tree_bytes));
-  TreeCounters done(std::min(per, C), st);
-  std::vector<std::unique_ptr<OwnedTree>> trees;
-  for (uint32_t j = 0; j < std::min(per, C); ++j) trees.push_back(std::make_unique<OwnedTree>(lN, done.d.p + j, st));
+  OwnedTrees owned(std::min(per, C), lN, st);
+  std::vector<DeviceTree>& trees = owned.t;
   for (uint32_t c0 = 0; c0 < C; c0 += per) {
     const uint32_t c = std::min(per, C - c0);
     build_qm31_trees(cw.p + (size_t)c0 * N, N, tree_ptrs(trees, 0, c).data(), c, st);
