@@ -676,7 +676,8 @@ __device__ __forceinline__ void mid_order(unsigned K, unsigned M, unsigned G, ui
   }
 }
 
-// KC, MC, GC: the compile-time layout of mid_order (0, 0, 0: K, M and G at run time);
+// KC, MC, GC: the compile-time layout of mid_order (0, 0, 0: K, M and G at run time: the
+// plain transforms, and LDEs outside k_mid_one's and k_mid_two's sizes);
 // 10, 10, 8 (the 2^20-row LDE) runs the LDE mode in the register-direct layouts of
 // k_low10, with 1/n applied by the last inverse chunk.
 template <unsigned KC = 0, unsigned MC = 0, unsigned GC = 0>
@@ -789,6 +790,106 @@ __global__ void __launch_bounds__(kMidThreads, 3) k_mid(const uint32_t* __restri
   }
 }
 
+// The middle pass of the LDE for M = L - K <= 5: one chunk, the 2^M values of one low
+// position per thread and no shared memory. All positions share the chunk's twiddles.
+template <int M>
+__global__ void __launch_bounds__(kMidThreads) k_mid_one(const uint32_t* __restrict__ in, size_t in_stride,
+                                                         uint32_t* __restrict__ out, size_t out_stride, unsigned L,
+                                                         unsigned B, const uint32_t* __restrict__ ITW_small,
+                                                         const uint32_t* __restrict__ TW_big) {
+  const unsigned K = L - M;
+  const uint32_t n = 1u << L, l = blockIdx.x * kMidThreads + threadIdx.x;
+  const uint32_t* src = in + (size_t)blockIdx.y * in_stride + l;
+  uint32_t* dst = out + (size_t)blockIdx.y * out_stride + l;
+  uint32_t v[1 << M];
+#pragma unroll
+  for (int m = 0; m < (1 << M); ++m) v[m] = __ldg(src + ((size_t)m << K));
+  chunk_layers<M, true, 0>(v, ITW_small, n, K, 0);
+  const unsigned inv_n_shift = (31 - L) % 31;  // 1/n = 2^(31 - L) mod p
+#pragma unroll
+  for (int m = 0; m < (1 << M); ++m) v[m] = mshl(v[m], inv_n_shift);
+#pragma unroll 1
+  for (uint32_t q = 0; q < (1u << B); ++q) {
+    uint32_t w[1 << M];
+#pragma unroll
+    for (int m = 0; m < (1 << M); ++m) w[m] = v[m];
+    chunk_layers<M, false, 0>(w, TW_big, n << B, K, q);
+    uint32_t* dq = dst + (size_t)q * n;
+#pragma unroll
+    for (int m = 0; m < (1 << M); ++m) dq[(size_t)m << K] = w[m];
+  }
+}
+
+// The same for M = RA + RB in two chunks (RA the lower layers'), K >= 5: a CTA takes G
+// consecutive low positions, lanes along them on both sides, so that the chunk of the low
+// layers moves its values between registers and global memory directly and shared memory only
+// carries the transpose between the chunks. Value hi of position g sits at
+// G (hi + hi / 2^RA) + g: the row of padding puts the 32 / G chunks of a warp on distinct
+// banks on the low side, where they are 2^RA rows apart, and they are adjacent rows on the
+// high side. With unequal chunks a thread takes two of the smaller one's. The scaled inverse
+// values stay in the thread's own slots of the first buffer; each quarter goes through the
+// second.
+template <int RA, int RB>
+struct MidTwo {
+  static constexpr int V = 1 << (RA > RB ? RA : RB), SA = V >> RA, SB = V >> RB;
+  static constexpr uint32_t G = (kMidThreads * V) >> (RA + RB), C = kMidThreads / G;
+  static constexpr uint32_t words = G * ((1u << (RA + RB)) + (1u << RB));
+};
+template <int RA, int RB>
+__global__ void __launch_bounds__(kMidThreads, RA == 5 ? 3 : 4)
+    k_mid_two(const uint32_t* __restrict__ in, size_t in_stride, uint32_t* __restrict__ out, size_t out_stride,
+              unsigned L, unsigned B, const uint32_t* __restrict__ ITW_small, const uint32_t* __restrict__ TW_big) {
+  using T = MidTwo<RA, RB>;
+  constexpr uint32_t G = T::G;
+  extern __shared__ uint32_t sm[];
+  uint32_t *s_in = sm, *s_q = sm + T::words;
+  const unsigned K = L - RA - RB;
+  const uint32_t n = 1u << L, g = threadIdx.x % G, r = threadIdx.x / G;
+  const size_t io = (size_t)blockIdx.x * G + g;
+  const uint32_t* src = in + (size_t)blockIdx.y * in_stride + io;
+  uint32_t* dst = out + (size_t)blockIdx.y * out_stride + io;
+  auto at = [&](uint32_t hi) { return G * (hi + (hi >> RA)) + g; };
+  uint32_t v[T::V];
+  // low side: chunk a = r + C s of values hi = a 2^RA + m; high side: b = r + C s of m 2^RA + b
+  auto low = [&](auto&& f) {
+#pragma unroll
+    for (int s = 0; s < T::SA; ++s)
+#pragma unroll
+      for (int m = 0; m < (1 << RA); ++m) f(v[s << RA | m], ((r + T::C * s) << RA) + m);
+  };
+  auto high = [&](auto&& f) {
+#pragma unroll
+    for (int s = 0; s < T::SB; ++s)
+#pragma unroll
+      for (int m = 0; m < (1 << RB); ++m) f(v[s << RB | m], ((uint32_t)m << RA) + r + T::C * s);
+  };
+  low([&](uint32_t& x, uint32_t hi) { x = __ldg(src + ((size_t)hi << K)); });
+#pragma unroll
+  for (int s = 0; s < T::SA; ++s) chunk_layers<RA, true, 0>(v + (s << RA), ITW_small, n, K, r + T::C * s);
+  low([&](uint32_t& x, uint32_t hi) { s_in[at(hi)] = x; });
+  __syncthreads();
+  high([&](uint32_t& x, uint32_t hi) { x = s_in[at(hi)]; });
+#pragma unroll
+  for (int s = 0; s < T::SB; ++s) chunk_layers<RB, true, 0>(v + (s << RB), ITW_small, n, K + RA, 0);
+  const unsigned inv_n_shift = (31 - L) % 31;  // 1/n = 2^(31 - L) mod p
+  high([&](uint32_t& x, uint32_t hi) { s_in[at(hi)] = mshl(x, inv_n_shift); });
+#pragma unroll 1
+  for (uint32_t q = 0; q < (1u << B); ++q) {
+    high([&](uint32_t& x, uint32_t hi) { x = s_in[at(hi)]; });
+#pragma unroll
+    for (int s = 0; s < T::SB; ++s) chunk_layers<RB, false, 0>(v + (s << RB), TW_big, n << B, K + RA, q);
+    high([&](uint32_t& x, uint32_t hi) { s_q[at(hi)] = x; });
+    __syncthreads();
+    low([&](uint32_t& x, uint32_t hi) { x = s_q[at(hi)]; });
+#pragma unroll
+    for (int s = 0; s < T::SA; ++s)
+      chunk_layers<RA, false, 0>(v + (s << RA), TW_big, n << B, K, (q << RB) + r + T::C * s);
+    uint32_t* dq = dst + (size_t)q * n;
+    low([&](uint32_t& x, uint32_t hi) { dq[(size_t)hi << K] = x; });
+    __syncthreads();  // s_q is rewritten by the next quarter
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Host launch helpers
 // ---------------------------------------------------------------------------
@@ -836,6 +937,21 @@ void launch_low(const uint32_t* src, size_t src_stride, uint32_t* dst, size_t ds
                                                                   tw);
   }
 }
+template <int M>
+void launch_mid_one(const uint32_t* in, size_t in_stride, uint32_t* out, size_t out_stride, uint32_t C, unsigned L,
+                    unsigned B, const uint32_t* itw, const uint32_t* tw, cudaStream_t st) {
+  k_mid_one<M><<<dim3((1u << (L - M)) / kMidThreads, C), kMidThreads, 0, st>>>(in, in_stride, out, out_stride, L, B,
+                                                                               itw, tw);
+}
+template <int RA, int RB>
+void launch_mid_two(const uint32_t* in, size_t in_stride, uint32_t* out, size_t out_stride, uint32_t C, unsigned L,
+                    unsigned B, const uint32_t* itw, const uint32_t* tw, cudaStream_t st) {
+  using T = MidTwo<RA, RB>;
+  constexpr size_t sb = 2 * T::words * sizeof(uint32_t);
+  if (sb > 48 * 1024) set_smem((const void*)k_mid_two<RA, RB>, sb);
+  k_mid_two<RA, RB><<<dim3((1u << (L - RA - RB)) / T::G, C), kMidThreads, sb, st>>>(in, in_stride, out, out_stride, L,
+                                                                                  B, itw, tw);
+}
 // The middle pass (k_mid) over C columns of a size-2^L transform split at K.
 void launch_mid(const uint32_t* in, size_t in_stride, uint32_t* out, size_t out_stride, uint32_t C, unsigned L,
                 unsigned K, unsigned B, const uint32_t* itw, const uint32_t* tw, int mode, cudaStream_t st) {
@@ -844,6 +960,23 @@ void launch_mid(const uint32_t* in, size_t in_stride, uint32_t* out, size_t out_
   const unsigned G = pick_groups(M, ngroups, kGroupWords / 2);
   size_t sb = smem_bytes(M, G, 2);
   const dim3 grid(ngroups / G, C);
+  // Register chunks for every LDE of up to 2^10 rows above the split (run-time layouts took
+  // 85 us of a 37 x 2^15 commit's middle pass, these 21 us); 2^20 rows keep the compile-time
+  // layout below, whose two thread mappings came out 4 % faster than k_mid_two<5, 5>.
+  if (mode == MID_LDE && K >= 8 && M >= 1 && M <= 10 && !(K == 10 && M == 10)) {
+    auto* f = M == 1   ? launch_mid_one<1>
+              : M == 2 ? launch_mid_one<2>
+              : M == 3 ? launch_mid_one<3>
+              : M == 4 ? launch_mid_one<4>
+              : M == 5 ? launch_mid_one<5>
+              : M == 6 ? launch_mid_two<3, 3>
+              : M == 7 ? launch_mid_two<4, 3>
+              : M == 8 ? launch_mid_two<4, 4>
+              : M == 9 ? launch_mid_two<5, 4>
+                       : launch_mid_two<5, 5>;
+    f(in, in_stride, out, out_stride, C, L, B, itw, tw, st);
+    return;
+  }
   if (K == 10 && M == 10 && G == 8) {  // the 2^20 -> 2^22 LDE: compile-time layout
     sb = std::max(sb, 2 * kBatch10Words * sizeof(uint32_t));
     set_smem((const void*)k_mid<10, 10, 8>, sb);
