@@ -38,16 +38,6 @@ void ensure_device() {
   if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0) throw Error(ZS_EDEVICE, "no CUDA device");
 }
 
-struct DeviceBuffer {
-  void* p = nullptr;
-  explicit DeviceBuffer(size_t bytes) { ZS_CUDA(cudaMalloc(&p, bytes ? bytes : 4)); }
-  ~DeviceBuffer() { cudaFree(p); }
-  template <typename T>
-  T* as() const {
-    return reinterpret_cast<T*>(p);
-  }
-};
-
 int32_t circle_transform(const uint32_t* in, uint32_t n_columns, uint32_t ox, uint32_t oy, uint32_t sx, uint32_t sy,
                          uint32_t log_half, uint32_t* out, bool inverse) {
   return guarded([&] {
@@ -58,14 +48,24 @@ int32_t circle_transform(const uint32_t* in, uint32_t n_columns, uint32_t ox, ui
     const unsigned lg = log_half + 1;
     const size_t n = (size_t)1 << lg;
     cudaStream_t st = nullptr;
+    thread_stream(0, &st);  // the calling thread's stream on the current device
+    retain_some_pool_memory();
+    PinnedScope pinned(st);
+    const size_t words = n * n_columns;
+    struct Buffers {  // input, output, scratch
+      uint32_t* p = nullptr;
+      cudaStream_t st;
+      Buffers(size_t w, cudaStream_t s) : st(s) { ZS_CUDA(cudaMallocAsync((void**)&p, 3 * w * 4, s)); }
+      ~Buffers() { cudaFreeAsync(p, st); }
+    } buf(words, st);
     CircleDomain dom(lg, cpoint{ox, oy}, cpoint{sx, sy}, st);
-    DeviceBuffer a(n * n_columns * 4), b(n * n_columns * 4), s(n * n_columns * 4);
-    ZS_CUDA(cudaMemcpy(a.p, in, n * n_columns * 4, cudaMemcpyHostToDevice));
+    upload_bytes(buf.p, in, words * 4, st);
     if (inverse)
-      circle_ifft(a.as<uint32_t>(), b.as<uint32_t>(), n_columns, dom, s.as<uint32_t>(), st);
+      circle_ifft(buf.p, buf.p + words, n_columns, dom, buf.p + 2 * words, st);
     else
-      circle_fft(a.as<uint32_t>(), b.as<uint32_t>(), n_columns, dom, s.as<uint32_t>(), st);
-    ZS_CUDA(cudaMemcpy(out, b.p, n * n_columns * 4, cudaMemcpyDeviceToHost));
+      circle_fft(buf.p, buf.p + words, n_columns, dom, buf.p + 2 * words, st);
+    ZS_CUDA(cudaMemcpyAsync(out, buf.p + words, words * 4, cudaMemcpyDeviceToHost, st));
+    ZS_CUDA(cudaStreamSynchronize(st));
   });
 }
 

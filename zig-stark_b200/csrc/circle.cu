@@ -15,7 +15,7 @@
 // [0, n/2), layer i >= 1 the 2^(lg-1-i) words after it. The inverse table holds the
 // elementwise M31 inverses. Both tables store each twiddle doubled (2t < 2^32), the
 // form the butterflies' multiply takes (mmul2). Tables are generated on the device
-// once per domain.
+// once per domain (k_twiddles).
 //
 // Each transform is split into HBM passes over groups held in shared memory: the
 // butterflies of layers [0, K) connect elements inside aligned runs of 2^K
@@ -25,6 +25,8 @@
 // five layers; for groups of 2^10 the chunks next to global memory load and store
 // their registers directly, and shared memory carries only the transpose between them. Every butterfly is the reference's exact M31 butterfly with the
 // reference's twiddle, so outputs are bit-identical.
+#include <algorithm>
+
 #include "circle.cuh"
 
 namespace zs {
@@ -33,59 +35,63 @@ namespace zs {
 // Twiddle tables
 // ---------------------------------------------------------------------------
 
-// Tree levels t = 0 .. lg-2: level t holds x(D^t(P_r)) for r < 2^(lg-2-t) in
-// bit-reversed order, P_r = offset + r*step of the half coset (circle.zig:69-82).
-__global__ void k_tw_tree(unsigned lg, cpoint offset, cpoint step, uint32_t* TW) {
+// A domain's tables, one thread per entry of the line layers. Entry r (bit-reversed) of tree
+// level t = 0 .. lg-2 is x(D^t(P_r)), P_r = offset + r*step of the half coset and D the
+// doubling (circle.zig:69-82); the threads of level 0 also write its circle layer,
+// (f0, f1) -> [f1, -f1, -f0, f0] (circle.zig:96-106). Every entry is computed on its own, a
+// chain of about lg doublings (and 60 products for the inverse), so that one launch makes all
+// levels of both tables of up to two domains; a launch per step (levels, circle layer,
+// inverses, doubling) took eight for the allocation-free LDE, half of its time.
+// lg = 1, 2: the reference's closed forms (circle.zig:210-220, 290-319) as the same flat
+// table: layer 0 = [y] or [y, -y], layer 1 = [x].
+struct TwJob {
+  unsigned lg;
+  cpoint offset, step;
+  uint32_t *tw, *itw;  // null: not wanted
+};
+__global__ void k_twiddles(const __grid_constant__ TwJob j0, const __grid_constant__ TwJob j1) {
+  const TwJob& j = blockIdx.y ? j1 : j0;
+  const unsigned lg = j.lg;
   const uint32_t half = 1u << (lg - 1);
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= (1u << (lg - 2))) return;
-  cpoint pt = padd(offset, pmul(step, r));
-  for (unsigned t = 0; t + 2 <= lg; ++t) {
-    if (r >= (1u << (lg - 2 - t))) break;
-    const uint32_t off = half - (1u << (lg - 1 - t));
-    TW[half + off + bitrev(r, lg - 2 - t)] = pt.x;
-    pt = pdbl(pt);
+  const uint32_t off = blockIdx.x * blockDim.x + threadIdx.x;
+  auto put = [&](uint32_t i, uint32_t x, uint32_t inv) {  // stored doubled (see mmul2)
+    if (j.tw) j.tw[i] = x << 1;
+    if (j.itw) j.itw[i] = inv << 1;
+  };
+  if (off >= half) return;
+  if (off == half - 1) {  // the reference's padding slot
+    put(2 * half - 1, 1, 1);
+    if (lg <= 2) {
+      const uint32_t yi = minv(j.offset.y);
+      put(0, j.offset.y, yi);
+      if (lg == 2) put(1, mneg(j.offset.y), mneg(yi));
+    }
+    return;
   }
-  if (r == 0) TW[2 * half - 1] = 1;  // the reference's padding slot
-}
-
-// Circle layer from the first tree level: (f0, f1) -> [f1, -f1, -f0, f0] (circle.zig:96-106).
-__global__ void k_tw_circle_layer(unsigned lg, uint32_t* TW) {
-  const uint32_t half = 1u << (lg - 1);
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= (half >> 2)) return;
-  const uint32_t f0 = TW[half + 2 * k], f1 = TW[half + 2 * k + 1];
-  TW[4 * k] = f1;
-  TW[4 * k + 1] = mneg(f1);
-  TW[4 * k + 2] = mneg(f0);
-  TW[4 * k + 3] = f0;
-}
-
-// lg = 1, 2: the reference's closed forms (circle.zig:210-220, 290-319) written as
-// the same flat table: layer 0 = [y] or [y, -y], layer 1 = [x].
-__global__ void k_tw_small(unsigned lg, cpoint p0, uint32_t* TW) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (lg == 1) {
-    TW[0] = p0.y;
-    TW[1] = 1;
-  } else {
-    TW[0] = p0.y;
-    TW[1] = mneg(p0.y);
-    TW[2] = p0.x;
-    TW[3] = 1;
+  // level t's 2^a entries (a = lg - 2 - t) start at half - 2^(a+1)
+  const uint32_t w = half - off;  // in (2^a, 2^(a+1)]
+  const unsigned a = 31 - __clz(w - 1);
+  const uint32_t r = bitrev((2u << a) - w, a);
+  cpoint pt = padd(j.offset, pmul(j.step, r));
+  for (unsigned t = a; t + 2 < lg; ++t) pt = pdbl(pt);
+  const uint32_t x = pt.x, xi = j.itw ? minv(x) : 0;
+  put(half + off, x, xi);
+  if (a + 2 == lg && lg > 2) {
+    const uint32_t k4 = 2 * (off & ~1u);
+    if (off & 1) {
+      put(k4, x, xi);
+      put(k4 + 1, mneg(x), mneg(xi));
+    } else {
+      put(k4 + 2, mneg(x), mneg(xi));
+      put(k4 + 3, x, xi);
+    }
   }
 }
 
-// Inverse table, stored doubled like the forward one (see mmul2).
-__global__ void k_invert(const uint32_t* in, uint32_t* out, uint32_t n) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) out[k] = minv(in[k]) << 1;
-}
-
-// Forward table doubled in place, after k_invert has read it.
-__global__ void k_double(uint32_t* tw, uint32_t n) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) tw[k] <<= 1;
+static void make_twiddles(const TwJob& j0, const TwJob* j1, cudaStream_t st) {
+  const uint32_t half = 1u << ((j1 ? std::max(j0.lg, j1->lg) : j0.lg) - 1);
+  k_twiddles<<<dim3((half + 255) / 256, j1 ? 2 : 1), 256, 0, st>>>(j0, j1 ? *j1 : j0);
+  ZS_CUDA(cudaGetLastError());
 }
 
 // canonicHalf(lg) (src/m31/circle/coset.zig:59-65): B = generator().neg(),
@@ -108,27 +114,15 @@ CircleDomain::CircleDomain(unsigned lg_, cpoint offset, cpoint step, cudaStream_
   init(offset, step, st);
 }
 
-void CircleDomain::init(cpoint offset, cpoint step, cudaStream_t st) {
+void CircleDomain::init(cpoint offset, cpoint step, cudaStream_t s) {
+  st = s;
   const uint32_t n = 1u << lg;
-  ZS_CUDA(cudaMallocAsync(&tw, n * sizeof(uint32_t), st));
-  ZS_CUDA(cudaMallocAsync(&itw, n * sizeof(uint32_t), st));
-  if (lg <= 2) {
-    k_tw_small<<<1, 32, 0, st>>>(lg, offset, tw);
-  } else {
-    const uint32_t r = 1u << (lg - 2);
-    k_tw_tree<<<(r + 255) / 256, 256, 0, st>>>(lg, offset, step, tw);
-    const uint32_t k = 1u << (lg - 3);
-    k_tw_circle_layer<<<(k + 255) / 256, 256, 0, st>>>(lg, tw);
-  }
-  k_invert<<<(n + 255) / 256, 256, 0, st>>>(tw, itw, n);
-  k_double<<<(n + 255) / 256, 256, 0, st>>>(tw, n);
-  ZS_CUDA(cudaGetLastError());
+  ZS_CUDA(cudaMallocAsync(&tw, 2 * (size_t)n * sizeof(uint32_t), st));
+  itw = tw + n;
+  make_twiddles({lg, offset, step, tw, itw}, nullptr, st);
 }
 
-CircleDomain::~CircleDomain() {
-  cudaFree(tw);
-  cudaFree(itw);
-}
+CircleDomain::~CircleDomain() { cudaFreeAsync(tw, st); }
 
 // ---------------------------------------------------------------------------
 // Butterfly arithmetic
@@ -1027,25 +1021,15 @@ void circle_ifft(const uint32_t* d_evals, uint32_t* d_coeffs, uint32_t C, const 
 
 // ---------------------------------------------------------------------------
 // Table-parameterised variants for callers that own every buffer (the
-// allocation-free entry point in noalloc.cu): the canonic domain's tables are
-// written into caller memory, and the LDE takes the tables directly.
+// allocation-free entry point in noalloc.cu): the two tables of an LDE are written
+// into caller memory, and the LDE takes them directly.
 // ---------------------------------------------------------------------------
 
-void circle_twiddles_into(unsigned lg, uint32_t* tw, uint32_t* itw, cudaStream_t st) {
-  cpoint offset, step;
-  canonic_half(lg, &offset, &step);
-  const uint32_t n = 1u << lg;
-  if (lg <= 2) {
-    k_tw_small<<<1, 32, 0, st>>>(lg, offset, tw);
-  } else {
-    const uint32_t r = 1u << (lg - 2);
-    k_tw_tree<<<(r + 255) / 256, 256, 0, st>>>(lg, offset, step, tw);
-    const uint32_t k = 1u << (lg - 3);
-    k_tw_circle_layer<<<(k + 255) / 256, 256, 0, st>>>(lg, tw);
-  }
-  k_invert<<<(n + 255) / 256, 256, 0, st>>>(tw, itw, n);
-  k_double<<<(n + 255) / 256, 256, 0, st>>>(tw, n);
-  ZS_CUDA(cudaGetLastError());
+void circle_lde_twiddles(unsigned L, unsigned B, uint32_t* itw_small, uint32_t* tw_big, cudaStream_t st) {
+  TwJob small{L, {}, {}, nullptr, itw_small}, big{L + B, {}, {}, tw_big, nullptr};
+  canonic_half(L, &small.offset, &small.step);
+  canonic_half(L + B, &big.offset, &big.step);
+  make_twiddles(small, &big, st);
 }
 
 void circle_lde_tables(const uint32_t* d_in, size_t in_stride, uint32_t* d_out, size_t out_stride, uint32_t C,

@@ -66,6 +66,22 @@ inline void retain_pool_memory() {
   if (dev < 64) done |= 1ull << dev;
 }
 
+// Up to 256 MB of freed blocks stay in the pool (more where retain_pool_memory ran), for
+// entry points that allocate a workspace per call: with none kept, every call's
+// synchronization gives its blocks back to the driver and the next maps them again.
+inline void retain_some_pool_memory() {
+  int dev = 0;
+  ZS_CUDA(cudaGetDevice(&dev));
+  cudaMemPool_t pool;
+  ZS_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
+  uint64_t keep = 0;
+  const uint64_t want = (uint64_t)256 << 20;
+  ZS_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  if (keep < want) {
+    keep = want;
+    ZS_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  }
+}
 
 // Non-blocking streams owned by the calling thread, created on first use per device and
 // slot and kept for the thread's life (creating and destroying streams and events costs

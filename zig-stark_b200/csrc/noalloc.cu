@@ -14,7 +14,7 @@
 //     on the first call on the device (the address lookup below), not when the library
 //     is opened, so a caller that later reserves all free device memory makes one small
 //     call first (or sets CUDA_MODULE_LOADING=EAGER);
-//   - a call needs 2*2^L + 2*2^(L+B) + C*(2^L + 2^(L+B)) words of it, at most
+//   - a call may need up to 2*2^L + 2*2^(L+B) + C*(2^L + 2^(L+B)) words of it, at most
 //     kNoallocWords (2^22 words); larger requests are rejected with -2;
 //   - all calls share the array and it keeps the last call's contents, so calls
 //     whose work overlaps on the GPU (different streams, or several host threads)
@@ -70,15 +70,12 @@ extern "C" int32_t zs_m31_circle_lde_noalloc(const uint32_t* d_in, uint32_t* d_o
   uint32_t* base = nullptr;
   const int32_t rc = scratch_for_current_device(&base);
   if (rc != ZS_OK) return rc;
-  uint32_t* tw_small = base;
-  uint32_t* itw_small = tw_small + n;
+  uint32_t* itw_small = base;
   uint32_t* tw_big = itw_small + n;
-  uint32_t* itw_big = tw_big + N;
-  uint32_t* work = itw_big + N;
+  uint32_t* work = tw_big + N;
   cudaStream_t st = (cudaStream_t)stream;
   try {
-    circle_twiddles_into(log_rows, tw_small, itw_small, st);
-    circle_twiddles_into(log_rows + log_blowup, tw_big, itw_big, st);
+    circle_lde_twiddles(log_rows, log_blowup, itw_small, tw_big, st);
     circle_lde_tables(d_in, n, d_out, N, n_columns, log_rows, log_blowup, itw_small, tw_big, work, st);
   } catch (const Error& e) {
     return e.code;
