@@ -388,30 +388,32 @@ struct DevBuf {
   DevBuf& operator=(const DevBuf&) = delete;
 };
 
-Digest root_of(const DeviceTree& t, cudaStream_t st) {
-  Digest d;
-  d2h_small(d.data(), t.root(), 32, st);
-  return d;
-}
-
 // The trees of a proof's columns (one size), in one allocation with their counters: a wide
 // proof has hundreds, and a stream-ordered allocation and free takes 2-3 us of the host's
 // time each (1.9 ms of a 387-column proof).
 struct OwnedTrees {
   std::vector<DeviceTree> t;
   OwnedTrees(uint32_t count, unsigned log_n, cudaStream_t s)
-      : t(count), words((size_t)count * tree_words(log_n), s), done(count, s) {
+      : t(count), words((size_t)count * tree_words(log_n), s), done(count, s), root_words((size_t)8 * count, s) {
     ZS_CUDA(cudaMemsetAsync(done.p, 0, count * sizeof(uint32_t), s));
     for (uint32_t j = 0; j < count; ++j) {
       t[j].log_n = log_n;
       t[j].words = words.p + (size_t)j * tree_words(log_n);
       t[j].done = done.p + j;
+      t[j].root_out = root_words.p + (size_t)8 * j;
     }
+  }
+  // The roots of trees [a, b), which lie side by side, in one copy.
+  std::vector<Digest> roots(uint32_t a, uint32_t b, cudaStream_t s) const {
+    std::vector<Digest> out(b - a);
+    static_assert(sizeof(Digest) == 32, "digests are copied in a run");
+    d2h_small(out.data(), root_words.p + (size_t)8 * a, (size_t)32 * (b - a), s);
+    return out;
   }
   static size_t tree_words(unsigned log_n) { return (DeviceTree::words_for(log_n) + 63) & ~(size_t)63; }
 
  private:
-  DevBuf<uint32_t> words, done;
+  DevBuf<uint32_t> words, done, root_words;
 };
 
 // The trees of the FRI layers (2^log_n leaves and down), likewise.
@@ -489,15 +491,6 @@ const OffsetTable& offset_table(unsigned log_n, cudaStream_t st, std::unique_ptr
     return *own;
   }
   return cached_table<OffsetTable>(log_n, [&](cudaStream_t s) { return new OffsetTable(log_n, s); });
-}
-
-// The roots of trees[a, b), read back with one wait.
-std::vector<Digest> roots_of(const std::vector<DeviceTree>& trees, uint32_t a, uint32_t b, cudaStream_t st) {
-  std::vector<Digest> out(b - a);
-  std::vector<D2H> c;
-  for (uint32_t j = a; j < b; ++j) c.push_back({out[j - a].data(), trees[j].root(), 32});
-  d2h_many(c.data(), c.size(), st);
-  return out;
 }
 
 // The DeviceTree pointers of trees[a, b).
@@ -735,7 +728,7 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   proof.u8(sp.remainder_log);
   std::vector<Digest> pre_roots, trace_roots, acc_roots;
   {
-    const std::vector<Digest> roots = roots_of(trees, 0, n_pre + m, st);
+    const std::vector<Digest> roots = owned.roots(0, n_pre + m, st);
     pre_roots.assign(roots.begin(), roots.begin() + n_pre);
     trace_roots.assign(roots.begin() + n_pre, roots.end());
   }
@@ -797,7 +790,7 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
              cw.p + (size_t)(n_pre + m) * N, N, n_rel, small, big, offset_pows, st);
     build_qm31_trees(cw.p + (size_t)(n_pre + m) * N, N, tree_ptrs(trees, n_pre + m, n_pre + m + n_rel).data(), n_rel,
                      st);
-    const std::vector<Digest> aroots = roots_of(trees, n_pre + m, n_pre + m + n_rel, st);
+    const std::vector<Digest> aroots = owned.roots(n_pre + m, n_pre + m + n_rel, st);
     for (uint32_t r = 0; r < n_rel; ++r) {
       acc_roots.push_back(aroots[r]);
       ch.absorb(acc_roots.back());
@@ -863,7 +856,7 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   ZS_CUDA(cudaGetLastError());
   DeviceTree& qtree = trees[ncol];
   build_qm31_tree(q.p, qtree, st);
-  const Digest qroot = root_of(qtree, st);
+  const Digest qroot = owned.roots(ncol, ncol + 1, st)[0];
   ch.absorb(qroot);
   proof.digest(qroot);
 
@@ -1111,7 +1104,7 @@ std::vector<uint8_t> commit_columns(const uint8_t* cols_b, size_t cols_len, unsi
   for (uint32_t c0 = 0; c0 < C; c0 += per) {
     const uint32_t c = std::min(per, C - c0);
     build_qm31_trees(cw.p + (size_t)c0 * N, N, tree_ptrs(trees, 0, c).data(), c, st);
-    for (const Digest& d : roots_of(trees, 0, c, st)) out.digest(d);
+    for (const Digest& d : owned.roots(0, c, st)) out.digest(d);
   }
   return out.out;
 }
