@@ -183,6 +183,12 @@ struct Terms {
   alignas(16) uint8_t coef[16 * kMaxTerms];
 };
 
+// A prover's round kernels are launched with programmatic stream serialization: a launch's
+// CTAs come up and load the product table while the kernel before them ends, and take
+// after_previous() before they touch what it wrote.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 __device__ __forceinline__ void load_table(uint8_t* s_T, const uint8_t* __restrict__ gT) {
   const uint4* src = reinterpret_cast<const uint4*>(gT);
   uint4* dst = reinterpret_cast<uint4*>(s_T);
@@ -465,23 +471,50 @@ __device__ __forceinline__ void finish_values(const uint32_t* s_acc, uint32_t wo
   sc_step<WIDE>(s, st, st.round, false, F);
 }
 
+// The fold of the round before, taken by the values kernel that needs its outputs: `cur` holds
+// the tables before it (of 2 len elements), r is its challenge; the folded tables (of len) go
+// to `next`.
+struct Folding {
+  const uint8_t* r;
+  void* next;
+};
+
 // GF(2^8) round; out: (dmax + 1) bytes packed four to a word (little-endian: byte t is
 // values[t]). D > 0: the D = dmax + 1 points in registers, every row once. D = 0: one
 // point per pass, points t = blockIdx.y, blockIdx.y + gridDim.y, ... (a grid of dmax + 1
 // rows of CTAs gives each point its own CTAs when the rows alone cannot fill the GPU).
-template <int D>
+template <int D, bool FOLD>
 __global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* __restrict__ cur, uint32_t len, uint32_t half,
                                                        uint32_t dmax, const __grid_constant__ Terms tm,
                                                        const uint8_t* __restrict__ gT, uint32_t* __restrict__ out,
-                                                       const __grid_constant__ ScStep step) {
+                                                       const __grid_constant__ ScStep step,
+                                                       const __grid_constant__ Folding fold) {
   extern __shared__ uint4 smem_b[];
   uint8_t* s_T = reinterpret_cast<uint8_t*>(smem_b);
   uint32_t* s_acc = reinterpret_cast<uint32_t*>(s_T + 65536);
   const uint32_t words = (dmax + 4) / 4;
+  let_next_start();
   load_table(s_T, gT);
   for (uint32_t k = threadIdx.x; k < words; k += blockDim.x) s_acc[k] = 0;
+  after_previous();
   __syncthreads();
   const Tower F{s_T};
+  // (a, b) of table f's row `row`; with FOLD from the four bytes they are folded from
+  const uint32_t rc = FOLD ? __ldcg(fold.r) : 0;
+  auto pair = [&](uint32_t f, uint32_t row, uint32_t& a, uint32_t& b) {
+    if constexpr (FOLD) {
+      const uint32_t w = __ldcg(reinterpret_cast<const uint32_t*>(cur + 2 * (size_t)f * len) + row);
+      const uint32_t a0 = w & 0xff, a1 = (w >> 16) & 0xff;
+      a = a0 ^ F.m8(rc, a0 ^ ((w >> 8) & 0xff));
+      b = a1 ^ F.m8(rc, a1 ^ (w >> 24));
+      if (D > 0 || blockIdx.y == 0)
+        *reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(fold.next) + (size_t)f * len + 2 * (size_t)row) =
+            (uint16_t)(a | (b << 8));
+    } else {
+      const uint8_t* p = cur + (size_t)f * len + 2 * (size_t)row;
+      a = p[0], b = p[1];
+    }
+  };
   const uint32_t stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
   if constexpr (D > 0) {
     // kRows rows per thread and pass, their loads issued together (the byte loads are
@@ -503,12 +536,11 @@ __global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* __restrict
         }
         uint32_t a[kRows], b[kRows], prod[kRows][D];
         auto load = [&](uint32_t j) {
-          const uint8_t* col = cur + (size_t)tm.idx[j] * len;
 #pragma unroll
           for (int r = 0; r < kRows; ++r) {
             const uint32_t row = base + r * stride;
-            a[r] = row < half ? col[2 * (size_t)row] : 0;
-            b[r] = row < half ? col[2 * (size_t)row + 1] : 0;
+            a[r] = b[r] = 0;
+            if (row < half) pair(tm.idx[j], row, a[r], b[r]);
           }
         };
         load(j0);
@@ -541,8 +573,9 @@ __global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* __restrict
           const uint32_t j0 = tm.off[k], j1 = tm.off[k + 1];
           uint32_t prod = tm.coef[k];
           for (uint32_t j = j0; j < j1; ++j) {
-            const uint8_t* p = cur + (size_t)tm.idx[j] * len + 2 * (size_t)rest;
-            const uint32_t v = at8(F, t, p[0], p[1]);
+            uint32_t a, b;
+            pair(tm.idx[j], rest, a, b);
+            const uint32_t v = at8(F, t, a, b);
             prod = (j == j0 && tm.kind[k] == 0) ? v : F.m8(prod, v);
           }
           acc ^= prod;
@@ -577,8 +610,10 @@ __global__ void __launch_bounds__(kBThreads, (D >= 1 && D <= 4) ? 2 : 1) k_value
   uint8_t* s_T = reinterpret_cast<uint8_t*>(smem_b);
   uint32_t* s_acc = reinterpret_cast<uint32_t*>(s_T + 65536);
   const uint32_t words = 4 * (dmax + 1);
+  let_next_start();
   load_table(s_T, gT);
   for (uint32_t k = threadIdx.x; k < words; k += blockDim.x) s_acc[k] = 0;
+  after_previous();
   __syncthreads();
   const Tower F{s_T};
   const uint32_t stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
@@ -718,6 +753,101 @@ __global__ void __launch_bounds__(kBThreads) k_fold128_direct(const uint4* __res
   }
 }
 
+// A round's values over `half` rows of tables in shared memory (table f's elements at
+// tab + f len), into s_acc (W words a point): a warp takes 32 kRows rows at one point at a time.
+template <bool WIDE, int kRows, typename E>
+__device__ __forceinline__ void values_shared(const Tower& F, const E* tab, uint32_t len, uint32_t half, uint32_t n,
+                                              const Terms& tm, uint32_t* s_acc) {
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const uint32_t groups = (half + 32 * kRows - 1) / (32 * kRows);
+#pragma unroll 1
+  for (uint32_t item = warp; item < groups * n; item += warps) {
+    const uint32_t t = item % n, rest = (item / n) * (32 * kRows) + lane;
+    E acc{};
+    for (uint32_t k = 0; k < tm.nterms; ++k) {
+      const uint32_t j0 = tm.off[k], j1 = tm.off[k + 1], kind = tm.kind[k];
+      if constexpr (WIDE) {
+        const uint64_t* cf = reinterpret_cast<const uint64_t*>(tm.coef + 16 * k);
+        const g128 c{cf[0], cf[1]};
+        if (rest < half) {
+          g128 prod = c;
+          for (uint32_t j = j0; j < j1; ++j) {
+            const g128* p = tab + (size_t)tm.idx[j] * len + 2 * rest;
+            const g128 v = at128(F, t, p[0], p[1]);
+            prod = j == j0 ? times_coef(F, kind, c, v) : F.m128(prod, v);
+          }
+          acc = gxor(acc, prod);
+        }
+      } else {
+        uint32_t prod[kRows];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) prod[r] = tm.coef[k];
+        for (uint32_t j = j0; j < j1; ++j) {
+          const uint8_t* p = tab + (size_t)tm.idx[j] * len + 2 * rest;
+#pragma unroll
+          for (int r = 0; r < kRows; ++r) {
+            const bool in = rest + 32 * r < half;
+            const uint32_t v = at8(F, t, in ? p[64 * r] : 0, in ? p[64 * r + 1] : 0);
+            prod[r] = (j == j0 && kind == 0) ? v : F.m8(prod[r], v);
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < kRows; ++r)
+          if (rest + 32 * r < half) acc ^= (uint8_t)prod[r];
+      }
+    }
+    if constexpr (WIDE)
+      warp_xor_into128(acc, s_acc + 4 * t);
+    else
+      warp_xor_into(acc, s_acc + t);
+  }
+}
+
+// A GF(2^128) round with the fold before it, in chunks of R rows per CTA: the CTA folds the 2R
+// elements of each table that its rows need (products by the challenge in full, 121 lookups)
+// into shared memory and `next`, and takes their values from there. Fold and values were two
+// launches (three with the multiply table), each with a load of the product table.
+// Shared memory: the product table, accumulators, the chunk of m tables.
+__global__ void __launch_bounds__(kBThreads, 2) k_sc_round128(const uint4* __restrict__ cur, uint32_t len, uint32_t m,
+                                                              uint32_t R, const __grid_constant__ Terms tm,
+                                                              const uint8_t* __restrict__ gT,
+                                                              uint32_t* __restrict__ out,
+                                                              const __grid_constant__ ScStep step,
+                                                              const __grid_constant__ Folding fold) {
+  extern __shared__ uint4 smem_b[];
+  uint8_t* s_T = reinterpret_cast<uint8_t*>(smem_b);
+  uint32_t* s_acc = reinterpret_cast<uint32_t*>(s_T + 65536);
+  const uint32_t n = step.n, half = len >> 1;
+  g128* tab = reinterpret_cast<g128*>(s_T + 65536 + 16 * n);
+  let_next_start();
+  load_table(s_T, gT);
+  for (uint32_t k = threadIdx.x; k < 4 * n; k += blockDim.x) s_acc[k] = 0;
+  after_previous();
+  __shared__ uint8_t s_r[16];
+  if (threadIdx.x < 16) s_r[threadIdx.x] = __ldcg(fold.r + threadIdx.x);
+  __syncthreads();
+  const Tower F{s_T};
+  const g128 r = load_challenge(s_r);
+  uint4* next = static_cast<uint4*>(fold.next);
+  for (uint32_t row0 = blockIdx.x * R; row0 < half; row0 += gridDim.x * R) {
+    const uint32_t rows = min(R, half - row0);
+    for (uint32_t e = threadIdx.x; e < m * 2 * rows; e += blockDim.x) {
+      const uint32_t f = e / (2 * rows), i = e % (2 * rows);
+      const uint4* p = cur + (size_t)f * 2 * len + 2 * ((size_t)2 * row0 + i);
+      const uint4 wa = __ldcg(p), wb = __ldcg(p + 1);
+      const g128 a = load_g128(&wa), b = load_g128(&wb);
+      const g128 o = gxor(a, F.m128(r, gxor(a, b)));
+      tab[f * 2 * R + i] = o;
+      next[(size_t)f * len + 2 * (size_t)row0 + i] =
+          make_uint4((uint32_t)o.lo, (uint32_t)(o.lo >> 32), (uint32_t)o.hi, (uint32_t)(o.hi >> 32));
+    }
+    __syncthreads();
+    values_shared<true, 1>(F, tab, 2 * R, rows, n, tm, s_acc);
+    __syncthreads();  // the next chunk overwrites the tables
+  }
+  finish_values<true>(s_acc, 4 * n, out, step, F);
+}
+
 // The last rounds of a proof in one CTA: the tables (m of `len` elements each, in `cur`)
 // come to shared memory and stay there, and each round is its values, the step and the
 // fold, a barrier apart; a round of few rows is otherwise three launches and as many loads
@@ -737,6 +867,7 @@ __global__ void __launch_bounds__(kTailThreads) k_sc_tail(const void* __restrict
   __shared__ uint32_t s_acc[kProveMaxPoints * W];
   uint8_t* s_T = reinterpret_cast<uint8_t*>(smem_b);
   load_table(s_T, gT);
+  after_previous();
   const Tower F{s_T};
   E* tab = reinterpret_cast<E*>(s_T + 65536);
   E* nxt = reinterpret_cast<E*>(s_T + 65536 + (((size_t)m * len * sizeof(E) + 15) & ~(size_t)15));
@@ -750,56 +881,11 @@ __global__ void __launch_bounds__(kTailThreads) k_sc_tail(const void* __restrict
     const uint32_t half = len >> 1;
     for (uint32_t k = threadIdx.x; k < n * W; k += blockDim.x) s_acc[k] = 0;
     __syncthreads();
-    auto values = [&](auto rows_c) {
-      constexpr int kRows = decltype(rows_c)::value;  // rows per lane
-      const uint32_t groups = (half + 32 * kRows - 1) / (32 * kRows);
-#pragma unroll 1
-      for (uint32_t item = warp; item < groups * n; item += warps) {
-        const uint32_t t = item % n, rest = (item / n) * (32 * kRows) + lane;
-        E acc{};
-        for (uint32_t k = 0; k < tm.nterms; ++k) {
-          const uint32_t j0 = tm.off[k], j1 = tm.off[k + 1], kind = tm.kind[k];
-          if constexpr (WIDE) {
-            const uint64_t* cf = reinterpret_cast<const uint64_t*>(tm.coef + 16 * k);
-            const g128 c{cf[0], cf[1]};
-            if (rest < half) {
-              g128 prod = c;
-              for (uint32_t j = j0; j < j1; ++j) {
-                const g128* p = tab + (size_t)tm.idx[j] * len + 2 * rest;
-                const g128 v = at128(F, t, p[0], p[1]);
-                prod = j == j0 ? times_coef(F, kind, c, v) : F.m128(prod, v);
-              }
-              acc = gxor(acc, prod);
-            }
-          } else {
-            uint32_t prod[kRows];
-#pragma unroll
-            for (int r = 0; r < kRows; ++r) prod[r] = tm.coef[k];
-            for (uint32_t j = j0; j < j1; ++j) {
-              const uint8_t* p = tab + (size_t)tm.idx[j] * len + 2 * rest;
-#pragma unroll
-              for (int r = 0; r < kRows; ++r) {
-                const bool in = rest + 32 * r < half;
-                const uint32_t v = at8(F, t, in ? p[64 * r] : 0, in ? p[64 * r + 1] : 0);
-                prod[r] = (j == j0 && kind == 0) ? v : F.m8(prod[r], v);
-              }
-            }
-#pragma unroll
-            for (int r = 0; r < kRows; ++r)
-              if (rest + 32 * r < half) acc ^= (uint8_t)prod[r];
-          }
-        }
-        if constexpr (WIDE)
-          warp_xor_into128(acc, s_acc + 4 * t);
-        else
-          warp_xor_into(acc, s_acc + t);
-      }
-    };
     // over GF(2^8) four rows per lane while there are as many: byte lookups are latency otherwise
     if (!WIDE && half > 64)
-      values(std::integral_constant<int, 4>{});
+      values_shared<WIDE, 4>(F, tab, len, half, n, tm, s_acc);
     else
-      values(std::integral_constant<int, 1>{});
+      values_shared<WIDE, 1>(F, tab, len, half, n, tm, s_acc);
     __syncthreads();
     if (warp == 0) {
       for (uint32_t k = lane; k < n * W; k += 32) {
@@ -870,15 +956,21 @@ void check_rows(size_t len, size_t half, size_t dmax) {
 
 // The values kernels by point count (index D, 0 = one point per pass) and the shared
 // memory they are launched with at most: the table and the largest accumulator.
-const void* const kValues8[kRegPoints + 1] = {
-    (const void*)k_values8<0>, (const void*)k_values8<1>, (const void*)k_values8<2>,
-    (const void*)k_values8<3>, (const void*)k_values8<4>, (const void*)k_values8<5>,
-    (const void*)k_values8<6>, (const void*)k_values8<7>, (const void*)k_values8<8>};
+template <bool FOLD>
+const void* values8(int D) {
+  static const void* const k[kRegPoints + 1] = {
+      (const void*)k_values8<0, FOLD>, (const void*)k_values8<1, FOLD>, (const void*)k_values8<2, FOLD>,
+      (const void*)k_values8<3, FOLD>, (const void*)k_values8<4, FOLD>, (const void*)k_values8<5, FOLD>,
+      (const void*)k_values8<6, FOLD>, (const void*)k_values8<7, FOLD>, (const void*)k_values8<8, FOLD>};
+  return k[D];
+}
 const void* const kValues128[kRegPoints + 1] = {
     (const void*)k_values128<0>, (const void*)k_values128<1>, (const void*)k_values128<2>,
     (const void*)k_values128<3>, (const void*)k_values128<4>, (const void*)k_values128<5>,
     (const void*)k_values128<6>, (const void*)k_values128<7>, (const void*)k_values128<8>};
 constexpr size_t kValuesSmem = 65536 + 16 * (kMaxPoint + 1);
+constexpr size_t kRoundTables = (size_t)40 << 10;  // of a chunk's tables: two CTAs per SM
+constexpr size_t kRoundSmem = 65536 + 16 * kProveMaxPoints + kRoundTables;
 constexpr size_t kTailSmem = 65536 + kTailBytes + kTailBytes / 2 + 32;
 
 // Per device, set up on first use: the product table, the SM count, the kernels' shared
@@ -886,7 +978,7 @@ constexpr size_t kTailSmem = 65536 + kTailBytes + kTailBytes / 2 + 32;
 struct DeviceState {
   uint8_t* table = nullptr;
   int sms = 0;
-  int per_sm8[kRegPoints + 1] = {}, per_sm128[kRegPoints + 1] = {};
+  int per_sm8[kRegPoints + 1] = {}, per_sm128[kRegPoints + 1] = {}, per_sm8f[kRegPoints + 1] = {};
 };
 std::mutex g_dev_mu;
 DeviceState g_dev[64];
@@ -900,9 +992,9 @@ const DeviceState& device_state(cudaStream_t st) {
   if (!d.table) {
     ZS_CUDA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
     for (int D = 0; D <= kRegPoints; ++D) {
-      for (int w = 0; w < 2; ++w) {
-        const void* fn = w ? kValues128[D] : kValues8[D];
-        int* per_sm = w ? &d.per_sm128[D] : &d.per_sm8[D];
+      for (int w = 0; w < 3; ++w) {
+        const void* fn = w == 0 ? values8<false>(D) : w == 1 ? kValues128[D] : values8<true>(D);
+        int* per_sm = w == 0 ? &d.per_sm8[D] : w == 1 ? &d.per_sm128[D] : &d.per_sm8f[D];
         ZS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kValuesSmem));
         ZS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, kBThreads, kValuesSmem));
         *per_sm = std::max(*per_sm, 1);
@@ -911,6 +1003,7 @@ const DeviceState& device_state(cudaStream_t st) {
     ZS_CUDA(cudaFuncSetAttribute(k_mul_table128, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
     ZS_CUDA(cudaFuncSetAttribute(k_fold128, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
     ZS_CUDA(cudaFuncSetAttribute(k_fold128_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
+    ZS_CUDA(cudaFuncSetAttribute(k_sc_round128, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRoundSmem));
     for (const void* fn : {(const void*)k_sc_tail<false>, (const void*)k_sc_tail<true>})
       ZS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));
     uint8_t* t = nullptr;
@@ -922,14 +1015,25 @@ const DeviceState& device_state(cudaStream_t st) {
   return d;
 }
 
+// A launch that may start while the kernel before it on the stream ends (after_previous).
+void launch_overlapped(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t st) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = st;
+  cfg.attrs = &at, cfg.numAttrs = 1;
+  ZS_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
+}
+
 // Accumulates one round's values into d_out, asynchronously on `st`, and takes the round's
 // step when one is given (d_out is zero before and after then; it is zeroed here
-// otherwise). With
+// otherwise); fold (GF(2^8)): d_cur holds the tables before the last fold. With
 // enough rows to give every SM a CTA, each thread takes all points of its rows (up to
 // eight; one point per pass beyond that); with fewer rows, the points get CTAs of their
 // own (a grid of dmax + 1 rows), so that small rounds still spread over the GPU.
 void values_async(bool wide, const void* d_cur, size_t len, size_t half, size_t dmax, const Terms& tm, void* d_out,
-                  const ScStep& step, cudaStream_t st) {
+                  const ScStep& step, const Folding* fold, cudaStream_t st) {
   const size_t words = wide ? 4 * (dmax + 1) : (dmax + 4) / 4;
   if (!step.tx) ZS_CUDA(cudaMemsetAsync(d_out, 0, words * 4, st));
   if (half == 0) return;
@@ -938,7 +1042,7 @@ void values_async(bool wide, const void* d_cur, size_t len, size_t half, size_t 
   const size_t row_blocks = (half + kBThreads - 1) / kBThreads;
   const bool per_row = D > 0 && row_blocks >= (size_t)ds.sms;
   const int kd = per_row ? D : 0;
-  const size_t slots = (size_t)ds.sms * (wide ? ds.per_sm128[kd] : ds.per_sm8[kd]);
+  const size_t slots = (size_t)ds.sms * (wide ? ds.per_sm128[kd] : fold ? ds.per_sm8f[kd] : ds.per_sm8[kd]);
   dim3 grid(1, 1);
   if (per_row) {
     grid.x = (unsigned)std::min(row_blocks, slots);
@@ -950,9 +1054,13 @@ void values_async(bool wide, const void* d_cur, size_t len, size_t half, size_t 
   uint32_t L = (uint32_t)len, H = (uint32_t)half, M = (uint32_t)dmax;
   const uint8_t* T = ds.table;
   uint32_t* out = static_cast<uint32_t*>(d_out);
-  void* args[] = {&cur, &L, &H, &M, const_cast<Terms*>(&tm), &T, &out, const_cast<ScStep*>(&step)};
-  ZS_CUDA(cudaLaunchKernel(wide ? kValues128[kd] : kValues8[kd], grid, dim3(kBThreads), args, 65536 + 4 * words,
-                           st));
+  Folding f = fold ? *fold : Folding{};
+  void* args[] = {&cur, &L, &H, &M, const_cast<Terms*>(&tm), &T, &out, const_cast<ScStep*>(&step), &f};
+  const void* fn = wide ? kValues128[kd] : fold ? values8<true>(kd) : values8<false>(kd);
+  if (step.tx)  // a prover's round
+    launch_overlapped(fn, grid, dim3(kBThreads), args, 65536 + 4 * words, st);
+  else
+    ZS_CUDA(cudaLaunchKernel(fn, grid, dim3(kBThreads), args, 65536 + 4 * words, st));
 }
 
 constexpr size_t kDirectFold = (size_t)1 << 16;  // elements up to which the direct fold is used
@@ -1024,7 +1132,7 @@ int32_t hook_values(bool wide, const uint8_t* cur_flat, size_t len, size_t m, co
     DevMem<uint4> d_cur((m * len * es + 15) / 16, st);
     DevMem<uint32_t> d_out(words, st);
     if (m * len) ZS_CUDA(cudaMemcpyAsync(d_cur.p, cur_flat, m * len * es, cudaMemcpyHostToDevice, st));
-    values_async(wide, d_cur.p, len, half, dmax, tm, d_out.p, {}, st);
+    values_async(wide, d_cur.p, len, half, dmax, tm, d_out.p, {}, nullptr, st);
     std::vector<uint32_t> h(words);
     ZS_CUDA(cudaMemcpyAsync(h.data(), d_out.p, words * 4, cudaMemcpyDeviceToHost, st));
     ZS_CUDA(cudaStreamSynchronize(st));
@@ -1080,6 +1188,7 @@ uint64_t tail_row_cost(bool wide, size_t m, const Terms& tm, size_t pts) {
   return c;
 }
 constexpr uint64_t kTailCost = (uint64_t)3 << 14;
+constexpr size_t kFusedFold = (size_t)3 << 16;  // elements up to which a round's fold is taken in full products
 
 int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, size_t m, const uint8_t* coeffs,
                           size_t nterms, const uint32_t* indices, size_t n_indices, const uint32_t* offsets,
@@ -1153,25 +1262,48 @@ int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, 
     const uint64_t row_cost = tail_row_cost(wide, m, tm, pts);
     void* cur = d_a.p;
     void* nxt = d_b.p;
+    const DeviceState& ds = device_state(st);
+    const uint8_t* d_r = aux + o_tx + offsetof(ScTranscript, r);
+    // rows of a chunk of k_sc_round128: a warp's, or 64 for eight warps at four points
+    const uint32_t chunk = m * 128 * es <= kRoundTables ? 64 : m * 64 * es <= kRoundTables ? 32 : 0;
     size_t len = n;
-    for (size_t i = 0; i < k; ++i) {
+    bool pending = false;  // `cur` awaits the fold of the round before (it has 2 len elements)
+    auto fold_now = [&] {
+      fold_async(wide, cur, 2 * len, m, 0, d_r, nxt, d_rmul.p, st);
+      std::swap(cur, nxt);
+      pending = false;
+    };
+    for (size_t i = 0; i < k; ++i, len /= 2) {
       const size_t half = len / 2;
       step.round = (uint32_t)i;
       if (m * len * es <= kTailBytes && half * row_cost <= kTailCost) {
+        if (pending) fold_now();
         const size_t smem = 65536 + ((m * len * es + 15) & ~(size_t)15) + ((m * half * es + 15) & ~(size_t)15);
-        if (wide)
-          k_sc_tail<true><<<1, kTailThreads, smem, st>>>(cur, (uint32_t)len, (uint32_t)m, (uint32_t)(k - i), tm, T, step);
-        else
-          k_sc_tail<false><<<1, kTailThreads, smem, st>>>(cur, (uint32_t)len, (uint32_t)m, (uint32_t)(k - i), tm, T, step);
-        ZS_CUDA(cudaGetLastError());
+        const void* c = cur;
+        uint32_t l = (uint32_t)len, mm = (uint32_t)m, rounds = (uint32_t)(k - i);
+        void* args[] = {&c, &l, &mm, &rounds, const_cast<Terms*>(&tm), &T, &step};
+        launch_overlapped(wide ? (const void*)k_sc_tail<true> : (const void*)k_sc_tail<false>, dim3(1),
+                          dim3(kTailThreads), args, smem, st);
         break;
       }
-      values_async(wide, cur, len, half, dmax, tm, aux + o_vals, step, st);
-      if (i + 1 < k) {
-        fold_async(wide, cur, len, m, 0, aux + o_tx + offsetof(ScTranscript, r), nxt, d_rmul.p, st);
+      if (pending && wide && m * len <= kFusedFold && chunk) {
+        const void* c = cur;
+        uint32_t l = (uint32_t)len, mm = (uint32_t)m, R = chunk, *o = reinterpret_cast<uint32_t*>(aux + o_vals);
+        Folding f{d_r, nxt};
+        void* args[] = {&c, &l, &mm, &R, const_cast<Terms*>(&tm), &T, &o, &step, &f};
+        const unsigned grid = (unsigned)std::min<size_t>((half + R - 1) / R, (size_t)2 * ds.sms);
+        launch_overlapped((const void*)k_sc_round128, dim3(grid), dim3(kBThreads), args,
+                          65536 + 16 * pts + (size_t)m * 2 * R * es, st);
         std::swap(cur, nxt);
+      } else if (pending && !wide && pts <= (size_t)kRegPoints) {
+        const Folding f{d_r, nxt};
+        values_async(wide, cur, len, half, dmax, tm, aux + o_vals, step, &f, st);
+        std::swap(cur, nxt);
+      } else {
+        if (pending) fold_now();
+        values_async(wide, cur, len, half, dmax, tm, aux + o_vals, step, nullptr, st);
       }
-      len = half;
+      pending = true;
     }
     const D2H back[2] = {{claimed_out, aux + o_claimed, es}, {rounds_out, aux + o_rounds, k * pts * es}};
     d2h_many(back, 2, st);
@@ -1208,7 +1340,7 @@ extern "C" int32_t zs_binius_sumcheck_values_device(uint32_t field_bits, const v
       throw zs::Error(zs::ZS_EMALFORMED, "misaligned buffer");
     zs::check_rows(len, half, dmax);
     const zs::Terms tm = zs::pack_terms(wide, m, coeffs, nterms, indices, n_indices, offsets);
-    zs::values_async(wide, d_cur, len, half, dmax, tm, d_out, {}, (cudaStream_t)stream);
+    zs::values_async(wide, d_cur, len, half, dmax, tm, d_out, {}, nullptr, (cudaStream_t)stream);
   });
 }
 
