@@ -308,77 +308,97 @@ __constant__ uint32_t kSha256K[64] = {
 
 __device__ __forceinline__ uint32_t sha_rotr(uint32_t x, unsigned r) { return __funnelshift_r(x, x, r); }
 
-// One 64-byte block `m` of SHA-256 (FIPS 180-4) into the state `h`, both in shared memory,
-// by a converged warp: every lane computes the rounds (a chain that no other lane could
-// shorten), 16 to a pass of the loop with the message schedule in registers: 4,500 cycles
-// (8,000 with the additions sent to the FMA pipe: they lie on the chain). Unrolled over all 64 rounds and with the message picked
-// together byte by byte in one thread, a step took 26 us, most of it instruction fetches
-// and address arithmetic.
-__device__ __noinline__ void sha_block(uint32_t* h, const uint32_t* m) {
-  uint32_t w[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) w[i] = __byte_perm(m[i], 0, 0x0123);  // big-endian words
-  uint32_t v[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = h[i];
-#pragma unroll 1
-  for (int q = 0; q < 64; q += 16) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      if (q > 0) {
-        const uint32_t x = w[(i + 1) & 15], y = w[(i + 14) & 15];
-        w[i] += (sha_rotr(x, 7) ^ sha_rotr(x, 18) ^ (x >> 3)) + w[(i + 9) & 15] +
-                (sha_rotr(y, 17) ^ sha_rotr(y, 19) ^ (y >> 10));
-      }
-      // v rotates by one word per round: a = v[-i], ..., in place of moving eight words
-      const uint32_t a = v[(0 - i) & 7], bb = v[(1 - i) & 7], c = v[(2 - i) & 7], e = v[(4 - i) & 7],
-                     f = v[(5 - i) & 7], g = v[(6 - i) & 7];
-      const uint32_t t1 = v[(7 - i) & 7] + (sha_rotr(e, 6) ^ sha_rotr(e, 11) ^ sha_rotr(e, 25)) +
-                          ((e & f) ^ (~e & g)) + (kSha256K[q + i] + w[i]);
-      v[(3 - i) & 7] += t1;
-      v[(7 - i) & 7] = t1 + (sha_rotr(a, 2) ^ sha_rotr(a, 13) ^ sha_rotr(a, 22)) + ((a & bb) ^ (a & c) ^ (bb & c));
-    }
-  }
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) h[i] += v[i];
-  }
-  __syncwarp();
-}
-
-// What a step works on, in shared memory: the message to absorb (state || coefficients),
-// a hash block and the hash state.
+// What a step works on, in shared memory: the message to absorb (state || coefficients), the
+// values, the Lagrange matrix, a hash block, two chunks of its schedule and the digest.
 struct StepShared {
   alignas(16) uint8_t msg[32 + kProveMaxPoints * 16];
   alignas(16) uint8_t vals[kProveMaxPoints * 16];
   uint8_t lag[kProveMaxPoints * kProveMaxPoints];
-  uint32_t blk[16], h[8];
+  alignas(16) uint32_t blk[16], wk[2][16];
 };
+__device__ __forceinline__ void two_warps() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
 
-// out[0..32) = SHA-256 of the n bytes at msg (shared or global memory), by a converged warp.
-__device__ __forceinline__ void sha256_warp(StepShared& s, const uint8_t* msg, uint64_t n, uint8_t* out) {
+// out[0..32) = SHA-256 (FIPS 180-4) of the n bytes at msg (shared or global memory), by the
+// first two warps of a CTA, each converged: warp 1 assembles the blocks and expands the
+// message schedule (plus the round constants) 16 words at a time, one chunk ahead of warp 0,
+// which runs the rounds; every lane computes all of its warp's chain. One warp alone takes
+// 4,500 cycles a block (about 26 ALU operations a round at two cycles each), and took 8,000
+// with the additions on the FMA pipe, which lie on the chain; in one thread, with the message
+// picked together byte by byte and all rounds unrolled, a step took 26 us, most of it
+// instruction fetches and address arithmetic.
+__device__ __noinline__ void sha256_two(StepShared& s, const uint8_t* msg, uint64_t n, uint8_t* out) {
   const uint32_t lane = threadIdx.x & 31;
-  constexpr uint32_t iv[8] = {0x6a09e667, 0xbb67ae85, 0x3c6ef372, 0xa54ff53a,
-                              0x510e527f, 0x9b05688c, 0x1f83d9ab, 0x5be0cd19};
-  if (lane == 0)
+  const uint64_t end = 64 * ((n + 9 + 63) / 64);
+  two_warps();  // the message is there
+  if (threadIdx.x >= 32) {
+    uint8_t* b = reinterpret_cast<uint8_t*>(s.blk);
+    uint32_t chunk = 0;
+#pragma unroll 1
+    for (uint64_t at = 0; at < end; at += 64) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s.h[i] = iv[i];
-  const uint64_t blocks = (n + 9 + 63) / 64, end = 64 * blocks;
-  uint8_t* b = reinterpret_cast<uint8_t*>(s.blk);
+      for (uint32_t i = lane; i < 64; i += 32) {
+        const uint64_t o = at + i;
+        uint8_t v = o < n ? msg[o] : o == n ? 0x80 : 0;
+        if (o >= end - 8) v = (uint8_t)((8 * n) >> (8 * (end - 1 - o)));
+        b[i] = v;
+      }
+      __syncwarp();
+      uint32_t w[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) w[i] = __byte_perm(s.blk[i], 0, 0x0123);  // big-endian words
+#pragma unroll 1
+      for (int q = 0; q < 64; q += 16, ++chunk) {
+        if (q > 0) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const uint32_t x = w[(i + 1) & 15], y = w[(i + 14) & 15];
+            w[i] += (sha_rotr(x, 7) ^ sha_rotr(x, 18) ^ (x >> 3)) + w[(i + 9) & 15] +
+                    (sha_rotr(y, 17) ^ sha_rotr(y, 19) ^ (y >> 10));
+          }
+        }
+        if (lane == 0) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) s.wk[chunk & 1][i] = w[i] + kSha256K[q + i];
+        }
+        two_warps();
+      }
+    }
+    return;
+  }
+  uint32_t h[8] = {0x6a09e667, 0xbb67ae85, 0x3c6ef372, 0xa54ff53a, 0x510e527f, 0x9b05688c, 0x1f83d9ab, 0x5be0cd19};
+  uint32_t v[8];
+  uint32_t chunk = 0;
 #pragma unroll 1
   for (uint64_t at = 0; at < end; at += 64) {
 #pragma unroll
-    for (uint32_t i = lane; i < 64; i += 32) {
-      const uint64_t o = at + i;
-      uint8_t v = o < n ? msg[o] : o == n ? 0x80 : 0;
-      if (o >= end - 8) v = (uint8_t)((8 * n) >> (8 * (end - 1 - o)));
-      b[i] = v;
+    for (int i = 0; i < 8; ++i) v[i] = h[i];
+#pragma unroll 1
+    for (int q = 0; q < 64; q += 16, ++chunk) {
+      two_warps();  // chunk `chunk` is there
+      uint32_t wk[16];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint4 x = reinterpret_cast<const uint4*>(s.wk[chunk & 1])[i];
+        wk[4 * i] = x.x, wk[4 * i + 1] = x.y, wk[4 * i + 2] = x.z, wk[4 * i + 3] = x.w;
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        // v rotates by one word per round: a = v[-i], ..., in place of moving eight words
+        const uint32_t a = v[(0 - i) & 7], bb = v[(1 - i) & 7], c = v[(2 - i) & 7], e = v[(4 - i) & 7],
+                       f = v[(5 - i) & 7], g = v[(6 - i) & 7];
+        const uint32_t t1 = v[(7 - i) & 7] + wk[i] + (sha_rotr(e, 6) ^ sha_rotr(e, 11) ^ sha_rotr(e, 25)) +
+                            ((e & f) ^ (~e & g));
+        v[(3 - i) & 7] += t1;
+        v[(7 - i) & 7] = t1 + (sha_rotr(a, 2) ^ sha_rotr(a, 13) ^ sha_rotr(a, 22)) + ((a & bb) ^ (a & c) ^ (bb & c));
+      }
     }
-    __syncwarp();
-    sha_block(s.h, s.blk);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) h[i] += v[i];
   }
-  out[lane] = (uint8_t)(s.h[lane >> 2] >> (24 - 8 * (lane & 3)));
+  if (lane == 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) reinterpret_cast<uint32_t*>(out)[i] = __byte_perm(h[i], 0, 0x0123);
+  }
   __syncwarp();
 }
 
@@ -401,41 +421,45 @@ struct ScStep {
   int has_seed;
 };
 
-// Round `round`'s step by a converged warp, the values in s.vals and the Lagrange matrix in
-// s.lag; the state comes from the round before, in s.msg (`kept`) or device memory. The points 0..n-1 lie in
-// GF(2^8), so the Lagrange matrix does too, and a subfield scalar scales each byte
-// coordinate of a value: byte b of coefficient d is sum_i lag[i][d] * byte b of values[i],
-// one lane per byte. The first round also forms the claimed sum (values[0] + values[1])
-// and starts the transcript (from the seed, or from the claimed sum). The challenge is the
-// digest's last byte over GF(2^8), its last 16 bytes over GF(2^128).
+// Round `round`'s step by the first two warps of a CTA, each converged, the values in s.vals and
+// the Lagrange matrix in s.lag; the state comes from the round before, in s.msg (`kept`) or
+// device memory. The points 0..n-1 lie in GF(2^8), so the Lagrange matrix does too, and a
+// subfield scalar scales each byte coordinate of a value: byte b of coefficient d is
+// sum_i lag[i][d] * byte b of values[i], one lane per byte. The first round also forms the
+// claimed sum (values[0] + values[1]) and starts the transcript (from the seed, or from the
+// claimed sum). The challenge is the digest's last byte over GF(2^8), its last 16 bytes over
+// GF(2^128).
 template <bool WIDE>
 __device__ __forceinline__ void sc_step(StepShared& s, const ScStep& st, uint32_t round, bool kept, const Tower& F) {
   constexpr uint32_t ES = WIDE ? 16 : 1;
   const uint32_t lane = threadIdx.x & 31, n = st.n;
+  const bool first = threadIdx.x < 32;
   if (round == 0) {
-    if (lane < ES) {  // one point: the sum of 2^k copies of a constant is 0
+    if (first && lane < ES) {  // one point: the sum of 2^k copies of a constant is 0
       const uint8_t c = n >= 2 ? s.vals[lane] ^ s.vals[ES + lane] : 0;
       s.msg[32 + lane] = c;
       st.claimed[lane] = c;
     }
-    __syncwarp();
     if (st.has_seed)
-      sha256_warp(s, st.seed, st.seed_len, s.msg);
+      sha256_two(s, st.seed, st.seed_len, s.msg);
     else
-      sha256_warp(s, s.msg + 32, ES, s.msg);
-  } else if (!kept) {
+      sha256_two(s, s.msg + 32, ES, s.msg);
+    two_warps();  // both are done with the message
+  } else if (first && !kept) {
     s.msg[lane] = __ldcg(st.tx->state + lane);
   }
-  for (uint32_t e = lane; e < n * ES; e += 32) {
-    const uint32_t d = e / ES, b = e % ES;
-    uint32_t c = 0;
+  if (first) {
+    for (uint32_t e = lane; e < n * ES; e += 32) {
+      const uint32_t d = e / ES, b = e % ES;
+      uint32_t c = 0;
 #pragma unroll 4
-    for (uint32_t i = 0; i < n; ++i) c ^= F.m8(s.lag[i * n + d], s.vals[ES * i + b]);
-    s.msg[32 + e] = (uint8_t)c;
-    st.rounds_out[(size_t)round * n * ES + e] = (uint8_t)c;
+      for (uint32_t i = 0; i < n; ++i) c ^= F.m8(s.lag[i * n + d], s.vals[ES * i + b]);
+      s.msg[32 + e] = (uint8_t)c;
+      st.rounds_out[(size_t)round * n * ES + e] = (uint8_t)c;
+    }
   }
-  __syncwarp();
-  sha256_warp(s, s.msg, 32 + n * ES, s.msg);
+  sha256_two(s, s.msg, 32 + n * ES, s.msg);
+  if (!first) return;
   st.tx->state[lane] = s.msg[lane];
   if (lane < ES) st.tx->r[lane] = s.msg[32 - ES + lane];
   __syncwarp();
@@ -460,14 +484,14 @@ __device__ __forceinline__ void finish_values(const uint32_t* s_acc, uint32_t wo
     if (s_last) *st.done = 0;
   }
   __syncthreads();
-  if (!s_last || threadIdx.x >= 32) return;
+  if (!s_last || threadIdx.x >= 64) return;
   __threadfence();
-  for (uint32_t k = threadIdx.x; k < words; k += 32) {
+  for (uint32_t k = threadIdx.x; k < words; k += 64) {
     reinterpret_cast<uint32_t*>(s.vals)[k] = __ldcg(out + k);
     out[k] = 0;
   }
-  for (uint32_t k = threadIdx.x; k < st.n * st.n; k += 32) s.lag[k] = __ldg(st.lag + k);
-  __syncwarp();
+  for (uint32_t k = threadIdx.x; k < st.n * st.n; k += 64) s.lag[k] = __ldg(st.lag + k);
+  two_warps();
   sc_step<WIDE>(s, st, st.round, false, F);
 }
 
@@ -887,14 +911,14 @@ __global__ void __launch_bounds__(kTailThreads) k_sc_tail(const void* __restrict
     else
       values_shared<WIDE, 1>(F, tab, len, half, n, tm, s_acc);
     __syncthreads();
-    if (warp == 0) {
-      for (uint32_t k = lane; k < n * W; k += 32) {
+    if (warp < 2) {
+      for (uint32_t k = threadIdx.x; k < n * W; k += 64) {
         if constexpr (WIDE)
           reinterpret_cast<uint32_t*>(s.vals)[k] = s_acc[k];
         else
           s.vals[k] = (uint8_t)s_acc[k];
       }
-      __syncwarp();
+      two_warps();
       sc_step<WIDE>(s, step, step.round + i, i > 0, F);  // leaves the challenge at the digest's end
     }
     __syncthreads();
