@@ -183,12 +183,8 @@ struct Terms {
   alignas(16) uint8_t coef[16 * kMaxTerms];
 };
 
-// A prover's round kernels are launched with programmatic stream serialization: a launch's
-// CTAs come up and load the product table while the kernel before them ends, and take
-// after_previous() before they touch what it wrote.
-__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;"); }
-
+// A prover's round kernels are launched with launch_overlapped: a launch's CTAs come up and
+// load the product table while the kernel before them ends.
 __device__ __forceinline__ void load_table(uint8_t* s_T, const uint8_t* __restrict__ gT) {
   const uint4* src = reinterpret_cast<const uint4*>(gT);
   uint4* dst = reinterpret_cast<uint4*>(s_T);
@@ -1037,17 +1033,6 @@ const DeviceState& device_state(cudaStream_t st) {
     d.table = t;
   }
   return d;
-}
-
-// A launch that may start while the kernel before it on the stream ends (after_previous).
-void launch_overlapped(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t st) {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = st;
-  cfg.attrs = &at, cfg.numAttrs = 1;
-  ZS_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
 }
 
 // Accumulates one round's values into d_out, asynchronously on `st`, and takes the round's

@@ -83,6 +83,24 @@ inline void retain_some_pool_memory() {
   }
 }
 
+// A launch that may start while the kernel before it on the stream ends (programmatic stream
+// serialization). Every thread of such a kernel takes after_previous() before it touches
+// what earlier work wrote or still reads; the kernel before lets it come up early with
+// let_next_start(). Both do nothing in an ordinary launch.
+inline void launch_overlapped(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t st) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = st;
+  cfg.attrs = &at, cfg.numAttrs = 1;
+  ZS_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+#endif
+
 // Non-blocking streams owned by the calling thread, created on first use per device and
 // slot and kept for the thread's life (creating and destroying streams and events costs
 // tens of microseconds per proof otherwise). Slots: 0 the stream of a zs_m31_prove call,

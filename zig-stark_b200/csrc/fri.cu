@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(kTailThreads) k_fri_tail(const FriTail* __rest
   __shared__ wtx::Shared s_tx;
   __shared__ uint4 s_dig[2 * 3 * (kTailMax / 4)];
   __shared__ qm31 s_c;  // the next fold's alpha * off_inv
+  after_previous();
   if (threadIdx.x < 32) wtx::load(s_tx, ch);
   if (threadIdx.x == 0 && ft.layer[0]) s_c = qmul(ft.alphas[-1], ft.off_inv[0]);
   __syncthreads();
@@ -114,8 +115,8 @@ __global__ void __launch_bounds__(kTailThreads) k_fri_tail(const FriTail* __rest
 }
 
 void fri_tail(const FriTail* ft, Channel* ch, cudaStream_t st) {
-  k_fri_tail<<<1, kTailThreads, 0, st>>>(ft, ch);
-  ZS_CUDA(cudaGetLastError());
+  void* args[] = {&ft, &ch};
+  launch_overlapped((const void*)k_fri_tail, dim3(1), dim3(kTailThreads), args, 0, st);
 }
 
 }  // namespace zs

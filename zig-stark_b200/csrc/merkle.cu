@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(kTreeThreads, SRC == kValues ? 4 : 3)
     k_tree(const __grid_constant__ TreeSet ts, unsigned level0, unsigned span, unsigned levels, unsigned top,
            const __grid_constant__ FoldSource f, const __grid_constant__ TranscriptStep tx) {
   extern __shared__ uint4 s_dig[];
+  let_next_start();
+  after_previous();
   uint32_t* words = ts.words[blockIdx.y];
   const unsigned log_n = ts.log_n[blockIdx.y];
   if (level0 + span > log_n) span = levels = log_n - level0;
@@ -222,8 +224,14 @@ void finish_set(const TreeSet& ts, uint32_t count, unsigned log_n, unsigned leve
     auto* k = from == kFold     ? (with_tx ? k_tree<kFold, true> : k_tree<kFold, false>)
               : from == kValues ? (with_tx ? k_tree<kValues, true> : k_tree<kValues, false>)
                                 : (with_tx ? k_tree<kDigests, true> : k_tree<kDigests, false>);
-    k<<<grid, t.threads, t.smem(), st>>>(ts, t.level0, t.span, t.levels, t.top_levels > 0, f,
-                                         tx ? *tx : TranscriptStep{});
+    if (tx) {  // a chain of launches that wait for one another
+      unsigned level0 = t.level0, span = t.span, levels = t.levels, top = t.top_levels > 0;
+      void* args[] = {const_cast<TreeSet*>(&ts), &level0, &span, &levels, &top, const_cast<FoldSource*>(&f),
+                      const_cast<TranscriptStep*>(tx)};
+      launch_overlapped((const void*)k, grid, dim3(t.threads), args, t.smem(), st);
+    } else {
+      k<<<grid, t.threads, t.smem(), st>>>(ts, t.level0, t.span, t.levels, t.top_levels > 0, f, {});
+    }
   }
   ZS_CUDA(cudaGetLastError());
 }

@@ -265,6 +265,8 @@ __device__ __forceinline__ uint32_t slot_of(uint32_t e, uint32_t c) {
 template <bool DIF>
 __global__ void __launch_bounds__(1 << (kTileLog - 2), 2) k_ntt_pass(const __grid_constant__ NttPass p) {
   extern __shared__ uint2 s_el[];
+  let_next_start();
+  after_previous();
   const unsigned E = p.lgG + p.M + p.lgH, lo = p.lo, M = p.M;
   const uint32_t c = threadIdx.x & 1, q = threadIdx.x >> 1;
   // the tile: l0 = the first l, hi0 = the first hi
@@ -468,7 +470,9 @@ static void run_transform(const NttPass& t, unsigned from, uint32_t count, cudaS
     for (uint32_t c0 = 0; c0 < count; c0 += 65535) {  // grid.y is at most 65535
       NttPass g = p;
       g.a += c0 * g.stride, g.src += c0 * g.src_stride, g.wbuf += g.wbuf ? c0 * g.w_stride : 0;
-      k_ntt_pass<DIF><<<dim3(1u << (p.logN - E), std::min(65535u, count - c0)), 1u << (E - 2), smem, st>>>(g);
+      void* args[] = {&g};
+      launch_overlapped((const void*)k_ntt_pass<DIF>, dim3(1u << (p.logN - E), std::min(65535u, count - c0)),
+                        dim3(1u << (E - 2)), args, smem, st);
     }
   }
   ZS_CUDA(cudaGetLastError());

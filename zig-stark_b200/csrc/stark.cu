@@ -928,17 +928,6 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
     h2d_small(d_ch.p, &ch, sizeof(Channel), st);
     DevBuf<qm31> d_alpha(L, st);
     DevBuf<uint32_t> d_roots((size_t)8 * L, st);
-    for (unsigned i = 0; i < tail; ++i) {
-      const TranscriptStep tx{d_ch.p, d_alpha.p + i};
-      ftrees[i].root_out = d_roots.p + 8 * i;
-      if (i == 0) {
-        build_qm31_tree(layers[0], ftrees[0], st, &tx);
-      } else {
-        const FoldSource f{layers[i - 1], layers[i], d_alpha.p + i - 1, ftabs.tables, ftabs.offset_inv(i - 1),
-                           N >> i, i - 1};
-        build_fold_tree(f, ftrees[i], st, &tx);
-      }
-    }
     DevBuf<FriTail> d_tail(1, st);
     if (tail < L) {
       FriTail ft{};
@@ -951,6 +940,19 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
       ft.roots = d_roots.p + 8 * tail;
       ft.alphas = d_alpha.p + tail;
       h2d_small(d_tail.p, &ft, sizeof(ft), st);
+    }
+    for (unsigned i = 0; i < tail; ++i) {
+      const TranscriptStep tx{d_ch.p, d_alpha.p + i};
+      ftrees[i].root_out = d_roots.p + 8 * i;
+      if (i == 0) {
+        build_qm31_tree(layers[0], ftrees[0], st, &tx);
+      } else {
+        const FoldSource f{layers[i - 1], layers[i], d_alpha.p + i - 1, ftabs.tables, ftabs.offset_inv(i - 1),
+                           N >> i, i - 1};
+        build_fold_tree(f, ftrees[i], st, &tx);
+      }
+    }
+    if (tail < L) {
       fri_tail(d_tail.p, d_ch.p, st);
     } else {
       fri_fold(layers[L - 1], layers[L], N >> L, qzero(), d_alpha.p + L - 1, L - 1, ftabs, st);

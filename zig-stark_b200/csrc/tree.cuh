@@ -38,7 +38,7 @@ __device__ __forceinline__ qm31 fold_value(const qm31& y0, const qm31& y1, uint3
 
 // Levels level0 + 1 .. level0 + levels of a tree of 2^log_n leaves over the 2^span digests
 // [cta 2^span, (cta + 1) 2^span) of level `level0`, one node per thread, a barrier between
-// levels (and one at the end); kValues and kFold (level0 = 0) hash those digests first, two
+// levels (of the warp where one suffices) and one at the end; kValues and kFold (level0 = 0) hash those digests first, two
 // leaves to a node. All levels run through one loop with one copy of hash2: a copy is 26 KB
 // of instructions, and the seven copies of an earlier kernel (a 3-level subtree per thread)
 // ran at the rate of the instruction cache, not of the ALU.
@@ -52,6 +52,7 @@ __device__ __forceinline__ void cta_levels(uint32_t* words, unsigned log_n, unsi
 #pragma unroll 1
   for (unsigned l = 1; l <= levels; ++l) {
     const uint32_t cnt = 1u << (span - l);
+    if (cnt < 32 && threadIdx.x >= 32) break;  // the last levels are the first warp's alone
     const size_t dst = (N2 - (N2 >> (level0 + l))) + (cta << (span - l));
     const bool leaves = SRC != kDigests && level0 == 0 && l == 1;
     // The children's digests (or their leaves' values) in `q`, loaded one node ahead: warps
@@ -105,10 +106,14 @@ __device__ __forceinline__ void cta_levels(uint32_t* words, unsigned log_n, unsi
       put_digest(words, dst + e, o);
       if (l < levels) put_digest(reinterpret_cast<uint32_t*>(s_dig), to + e, o);
     }
-    __syncthreads();
+    if (cnt < 32)
+      __syncwarp();
+    else
+      __syncthreads();
     from = to;
     to = to == 0 ? 1u << (span - 1) : 0;
   }
+  __syncthreads();
 }
 
 }  // namespace zs
