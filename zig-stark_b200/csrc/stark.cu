@@ -129,18 +129,19 @@ __global__ void __launch_bounds__(kT) k_quotient_rescue(const qm31* __restrict__
   for (int j = 0; j < 5; ++j) per[j] = ldq(per_tab + (size_t)5 * (i & k.per_mask) + j);
   const qm31 x = domain_point(k, wpow, i);
   rescue_stacked_eval(per, cur, next, res);
-  qm31 tsum = qzero();
+  QAcc tsum;
 #pragma unroll
-  for (int t = 0; t < 12; ++t) tsum = qadd(tsum, qmul(rq.alphas[t], res[t]));
-  qm31 h = qmul(tsum, qsub(x, k.last_point));
+  for (int t = 0; t < 12; ++t) tsum.mul_add(rq.alphas[t], res[t]);
+  qm31 h = qmul(tsum.value(), qsub(x, k.last_point));
   const qm31 d0 = qsub(x, rq.bp[0]), d1 = qsub(x, rq.bp[1]);
   const qm31 inv = qinv(qmul(d0, d1));  // every x - p is a unit on the evaluation domain
-  qm31 acc0 = qneg(rq.be[0]), acc1 = qneg(rq.be[1]);
+  QAcc sum0, sum1;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    acc0 = qadd(acc0, qmul(rq.bc[0][j], cur[j]));
-    acc1 = qadd(acc1, qmul(rq.bc[1][j], cur[j]));
+    sum0.mul_add(rq.bc[0][j], cur[j]);
+    sum1.mul_add(rq.bc[1][j], cur[j]);
   }
+  const qm31 acc0 = qsub(sum0.value(), rq.be[0]), acc1 = qsub(sum1.value(), rq.be[1]);
   const qm31 bsum = qadd(qmul(acc0, qmul(inv, d1)), qmul(acc1, qmul(inv, d0)));
   const uint32_t zi = i & ((1u << k.log_blowup) - 1);
   h = qadd(h, qmul(bsum, ldq(zh_tab + 2 * (size_t)zi)));
@@ -186,17 +187,33 @@ __global__ void k_logup_rows(const qm31* __restrict__ vals, uint32_t n, const Qu
 }
 
 // The linear-layer AIR's LogUp row contributions (stark.zig:283-297) on H, its key and
-// table columns streamed from the column-major values [P_0..P_127 | x, y, sel, mult].
+// table columns streamed from the column-major values [P_0..P_127 | x, y, sel, mult]. A CTA
+// takes kLogupRows rows, kLogupParts threads to a row (each a part of the 128 columns, lanes
+// along the rows): one thread per row left most SMs with one CTA and a chain of 256 loads.
+constexpr uint32_t kLogupRows = 32, kLogupParts = kT / kLogupRows;
 __global__ void __launch_bounds__(kT) k_ml_logup_rows(const qm31* __restrict__ vals, uint32_t n,
                                                       const MlConsts* __restrict__ kp, qm31* __restrict__ out) {
+  __shared__ qm31 s_key[kT], s_tkey[kT];
   const MlConsts& k = *kp;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const uint32_t lane = threadIdx.x % kLogupRows, part = threadIdx.x / kLogupRows;
+  const uint32_t i = blockIdx.x * kLogupRows + lane;
   const qm31* main = vals + (size_t)kMlDim * n;
-  qm31 key = qzero(), tkey = qzero();
-  for (uint32_t l = 0; l < kMlDim; ++l) {
-    key = qadd(key, qmul(k.ac[l], ldq(main + (size_t)l * n + i)));
-    tkey = qadd(tkey, qmul(k.ac[l], ldq(vals + (size_t)l * n + i)));
+  if (i < n) {
+    QAcc ksum, tsum;
+#pragma unroll 4
+    for (uint32_t l = part; l < kMlDim; l += kLogupParts) {
+      ksum.mul_add(k.ac[l], ldq(main + (size_t)l * n + i));
+      tsum.mul_add(k.ac[l], ldq(vals + (size_t)l * n + i));
+    }
+    s_key[threadIdx.x] = ksum.value();
+    s_tkey[threadIdx.x] = tsum.value();
+  }
+  __syncthreads();
+  if (part != 0 || i >= n) return;
+  qm31 key = s_key[lane], tkey = s_tkey[lane];
+  for (uint32_t p = 1; p < kLogupParts; ++p) {
+    key = qadd(key, s_key[p * kLogupRows + lane]);
+    tkey = qadd(tkey, s_tkey[p * kLogupRows + lane]);
   }
   const qm31 sel = ldq(main + (size_t)kMlSel * n + i), mult = ldq(main + (size_t)kMlMult * n + i);
   const qm31 lt = qmul(sel, qmul(mult, qinv(qsub(k.ar, key))));
@@ -217,14 +234,15 @@ __global__ void __launch_bounds__(kT) k_ml_quotient(const qm31* __restrict__ cw,
   const uint32_t half = N >> 1;
   const qm31 x = qmul(k.offset, i < half ? ldq(wpow + i) : qneg(ldq(wpow + (i - half))));
   const qm31* main = cw + (size_t)kMlDim * N;
-  qm31 ty = qzero(), tx = qzero(), key = qzero(), tkey = qzero();
+  QAcc sum_y, sum_x, sum_k, sum_t;
   for (uint32_t l = 0; l < kMlDim; ++l) {
     const qm31 xl = ldq(main + (size_t)l * N + i);
-    ty = qadd(ty, qmul(k.alpha_y[l], ldq(main + (size_t)(kMlDim + l) * N + i)));
-    tx = qadd(tx, qmul(k.beta_x[l], xl));
-    key = qadd(key, qmul(k.ac[l], xl));
-    tkey = qadd(tkey, qmul(k.ac[l], ldq(cw + (size_t)l * N + i)));
+    sum_y.mul_add(k.alpha_y[l], ldq(main + (size_t)(kMlDim + l) * N + i));
+    sum_x.mul_add(k.beta_x[l], xl);
+    sum_k.mul_add(k.ac[l], xl);
+    sum_t.mul_add(k.ac[l], ldq(cw + (size_t)l * N + i));
   }
+  const qm31 ty = sum_y.value(), tx = sum_x.value(), key = sum_k.value(), tkey = sum_t.value();
   const uint32_t in = (i + k.shift) & (N - 1);
   const qm31 sel = ldq(main + (size_t)kMlSel * N + i), mult = ldq(main + (size_t)kMlMult * N + i);
   const qm31 acc = ldq(main + (size_t)kMlCols * N + i), accn = ldq(main + (size_t)kMlCols * N + in);
@@ -279,22 +297,44 @@ __device__ __forceinline__ qm31 block_sum(qm31 v, qm31* s) {
   return s[0];
 }
 
-// partial[pt][col][blk] = sum over the block's j of coeffs[col][j] * zpow[pt][bitrev(j)]
-// (the coefficients are stored in bit-reversed order, log_n = log2 n).
-__global__ void __launch_bounds__(kT) k_eval_partial(const qm31* __restrict__ coeffs, uint32_t n, unsigned log_n,
-                                                     const qm31* __restrict__ zpow, uint32_t npt, qm31* partial) {
+// out[pt][bitrev(k)] = x_pt^k, k < 2^log_n: the powers of both points in the coefficients'
+// (bit-reversed) order, so that every column's sums read them in rows.
+constexpr uint32_t kPowRun = 16;
+__global__ void k_eval_powers(qm31 x0, qm31 x1, qm31* __restrict__ out, unsigned log_n) {
+  const uint32_t n = 1u << log_n, k0 = (blockIdx.x * blockDim.x + threadIdx.x) * kPowRun;
+  if (k0 >= n) return;
+  const qm31 x = blockIdx.y ? x1 : x0;
+  qm31* dst = out + (size_t)blockIdx.y * n;
+  qm31 v = qpow(x, k0);
+  for (uint32_t k = k0; k < n && k < k0 + kPowRun; ++k) {
+    stq(dst + bitrev(k, log_n), v);
+    v = qmul(v, x);
+  }
+}
+
+// partial[pt][col][blk] = sum over the block's j of coeffs[col][j] * zpow[pt][j], both points
+// from one read of the coefficients.
+__global__ void __launch_bounds__(kT) k_eval_partial(const qm31* __restrict__ coeffs, uint32_t n,
+                                                     const qm31* __restrict__ zpow, qm31* partial) {
   __shared__ qm31 s[kT];
-  const uint32_t col = blockIdx.y, pt = blockIdx.z;
+  const uint32_t col = blockIdx.y;
   const qm31* c = coeffs + (size_t)col * n;
-  const qm31* zp = zpow + (size_t)pt * n;
-  qm31 acc = qzero();
+  QAcc acc0, acc1;
 #pragma unroll
   for (uint32_t k = 0; k < kEvalPer; ++k) {
     const uint32_t j = (blockIdx.x * kEvalPer + k) * blockDim.x + threadIdx.x;
-    if (j < n) acc = qadd(acc, qmul(ldq(c + j), ldq(zp + bitrev(j, log_n))));
+    if (j >= n) break;
+    const qm31 x = ldq(c + j);
+    acc0.mul_add(x, ldq(zpow + j));
+    acc1.mul_add(x, ldq(zpow + n + j));
   }
-  const qm31 sum = block_sum(acc, s);
-  if (threadIdx.x == 0) stq(partial + ((size_t)pt * gridDim.y + col) * gridDim.x + blockIdx.x, sum);
+  const qm31 sum0 = block_sum(acc0.value(), s);
+  __syncthreads();  // the sums share `s`
+  const qm31 sum1 = block_sum(acc1.value(), s);
+  if (threadIdx.x == 0) {
+    stq(partial + (size_t)col * gridDim.x + blockIdx.x, sum0);
+    stq(partial + ((size_t)gridDim.y + col) * gridDim.x + blockIdx.x, sum1);
+  }
 }
 
 // out[idx] = the sum of the `nblk` partials of (pt, col) = idx, one CTA each.
@@ -307,20 +347,19 @@ __global__ void __launch_bounds__(kT) k_eval_sum(const qm31* partial, uint32_t n
   if (threadIdx.x == 0) stq(out + blockIdx.x, sum);
 }
 
-// DEEP codeword (stark.zig:577-588), with 1/(d_i - z) factored out of the sum.
-// ge: the 2 m_total + 1 weights gamma_j, then the 2 m_total evaluations f_j(z), f_j(wz).
+// DEEP codeword (stark.zig:577-588), with 1/(d_i - z) factored out of the sum and the
+// evaluations' part of it, at_z = sum_j gamma_j f_j(z) + gamma_(m+j) f_j(wz) + gamma_2m q(z),
+// taken off at the end. gammas: the 2 m_total + 1 weights.
 struct DeepConsts {
   uint32_t m_total, n_pre, shift;
   unsigned log_N;
-  qm31 offset, z, qz;
+  qm31 offset, z, at_z;
 };
 
 __global__ void __launch_bounds__(kT) k_deep(const qm31* __restrict__ cw, const qm31* __restrict__ q,
                                              const qm31* __restrict__ wpow, const DeepConsts* __restrict__ kp,
-                                             const qm31* __restrict__ ge, qm31* __restrict__ g) {
+                                             const qm31* __restrict__ gammas, qm31* __restrict__ g) {
   const DeepConsts& k = *kp;
-  const qm31* gammas = ge;
-  const qm31* evals = ge + 2 * k.m_total + 1;
   const uint32_t N = 1u << k.log_N;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -329,14 +368,14 @@ __global__ void __launch_bounds__(kT) k_deep(const qm31* __restrict__ cw, const 
   const qm31 w = i < half ? ldq(wpow + i) : qneg(ldq(wpow + (i - half)));
   const qm31 x = qmul(k.offset, w);
   const qm31 inv_dz = qinv(qsub(x, k.z));
-  qm31 acc = qzero();
+  QAcc acc;
   for (uint32_t j = 0; j < k.m_total; ++j) {
     const qm31* c = cw + (size_t)(k.n_pre + j) * N;
-    acc = qadd(acc, qmul(ldq(gammas + j), qsub(ldq(c + i), ldq(evals + j))));
-    acc = qadd(acc, qmul(ldq(gammas + k.m_total + j), qsub(ldq(c + in), ldq(evals + k.m_total + j))));
+    acc.mul_add(ldq(gammas + j), ldq(c + i));
+    acc.mul_add(ldq(gammas + k.m_total + j), ldq(c + in));
   }
-  acc = qadd(acc, qmul(ldq(gammas + 2 * k.m_total), qsub(ldq(q + i), k.qz)));
-  stq(g + i, qmul(acc, inv_dz));
+  acc.mul_add(ldq(gammas + 2 * k.m_total), ldq(q + i));
+  stq(g + i, qmul(qsub(acc.value(), k.at_z), inv_dz));
 }
 
 // Gather: out[r] = words [idx * w, (idx + 1) * w) of src[r] (requests prepared on the host).
@@ -774,7 +813,7 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
     for (uint32_t r = 0; r < n_rel; ++r) {
       qm31* acc_vals = vals.p + (size_t)(n_pre + m + r) * n;
       if (wide)
-        k_ml_logup_rows<<<(n + kT - 1) / kT, kT, 0, st>>>(vals.p, n, d_ml->p, contrib.p);
+        k_ml_logup_rows<<<(n + kLogupRows - 1) / kLogupRows, kT, 0, st>>>(vals.p, n, d_ml->p, contrib.p);
       else
         k_logup_rows<<<(n + kT - 1) / kT, kT, 0, st>>>(vals.p, n, d_kc.p, r, contrib.p);
       // acc[i] = sum_{k < i} contrib[k] (stark.zig:438-446)
@@ -867,11 +906,10 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   std::vector<qm31> pre_z(n_pre);
   {
     DevBuf<qm31> zpow((size_t)2 * n, st);
-    qm31_powers(z, zpow.p, n, st);
-    qm31_powers(wz, zpow.p + n, n, st);
+    k_eval_powers<<<dim3((n + kT * kPowRun - 1) / (kT * kPowRun), 2), kT, 0, st>>>(z, wz, zpow.p, tl);
     const uint32_t nblk = (n + kT * kEvalPer - 1) / (kT * kEvalPer);
     DevBuf<qm31> partial((size_t)2 * ncol * nblk, st), sums((size_t)2 * ncol, st);
-    k_eval_partial<<<dim3(nblk, ncol, 2), kT, 0, st>>>(coeffs.p, n, tl, zpow.p, 2, partial.p);
+    k_eval_partial<<<dim3(nblk, ncol), kT, 0, st>>>(coeffs.p, n, zpow.p, partial.p);
     k_eval_sum<<<2 * ncol, kT, 0, st>>>(partial.p, nblk, sums.p);
     ZS_CUDA(cudaGetLastError());
     std::vector<qm31> hs(2 * ncol);
@@ -893,10 +931,14 @@ std::vector<uint8_t> stark_prove(uint32_t air_id, const uint8_t* params_b, size_
   // ---- DEEP codeword and FRI ---------------------------------------------------
   DeepConsts dc{};
   dc.m_total = m_total, dc.n_pre = n_pre, dc.shift = shift, dc.log_N = lN;
-  dc.offset = offset, dc.z = z, dc.qz = deep[2 * m_total];
-  std::vector<qm31> ge(n_deep + 2 * m_total);  // gammas, then f_j(z), f_j(wz)
-  for (uint32_t j = 0; j < n_deep; ++j) ge[j] = ch.sample_q();
-  for (uint32_t j = 0; j < 2 * m_total; ++j) ge[n_deep + j] = deep[j];
+  dc.offset = offset, dc.z = z;
+  std::vector<qm31> ge(n_deep);  // the weights
+  QAcc at_z;
+  for (uint32_t j = 0; j < n_deep; ++j) {
+    ge[j] = ch.sample_q();
+    at_z.mul_add(ge[j], deep[j]);
+  }
+  dc.at_z = at_z.value();
   DevBuf<DeepConsts> d_dc(1, st);
   h2d_small(d_dc.p, &dc, sizeof(dc), st);
   DevBuf<qm31> d_ge(ge.size(), st);
