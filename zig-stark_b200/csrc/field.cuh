@@ -53,8 +53,18 @@ ZS_HD uint32_t mpow(uint32_t a, uint32_t e) {
   }
   return r;
 }
-// a^(p-2); 0 maps to 0 exactly as the reference's release build does.
-ZS_HD uint32_t minv(uint32_t a) { return mpow(a, P - 2); }
+// a^(p-2); 0 maps to 0 exactly as the reference's release build does. By the addition chain
+// 1, 2, 3, 6, 7, 14, 28, 29 on the exponents 2^k - 1, and p - 2 = 4 (2^29 - 1) + 1: 38
+// products in place of binary exponentiation's 60.
+ZS_HD uint32_t minv(uint32_t a) {
+  auto up = [](uint32_t x, int k) {  // x^(2^k)
+    for (int i = 0; i < k; ++i) x = mmul(x, x);
+    return x;
+  };
+  const uint32_t x2 = mmul(up(a, 1), a), x3 = mmul(up(x2, 1), a), x6 = mmul(up(x3, 3), x3);
+  const uint32_t x7 = mmul(up(x6, 1), a), x14 = mmul(up(x7, 7), x7), x28 = mmul(up(x14, 14), x14);
+  return mmul(up(mmul(up(x28, 1), a), 2), a);
+}
 
 struct cm31 {
   uint32_t a, b;  // a + b i
