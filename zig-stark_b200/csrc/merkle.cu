@@ -47,44 +47,65 @@ __global__ void __launch_bounds__(kThreads) k_row_leaves(const uint32_t* __restr
   __syncthreads();
   const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
+  const uint32_t row_bytes = (uint32_t)r * 4;  // fits: a plan has at most 2^28 rows
   uint64_t acc0 = 0, acc1 = 0, acc2 = 0, acc3 = 0;
   uint32_t cv[8];
   b3::iv(cv);
   const uint32_t nblocks = C * 4 <= 64 ? 1 : (C * 4 + 63) / 64;
   // The next block's 16 column loads are issued before the current block is
-  // compressed, so their latency hides behind ~700 integer instructions.
+  // compressed, so their latency hides behind ~700 integer instructions. Only a row's last
+  // block can be a part of one: the others take their loads and products without a
+  // comparison of the column, from column addresses that are the same in every thread.
+  // Bound by the ALU pipe and the issue slots at once: 64 columns x 2^22 rows 761 -> 650 us,
+  // 4950 -> 4230 instructions a row, 2460 -> 2150 of them on the ALU (1792 in the four
+  // compressions). With one copy of the product code for whole and partial blocks (a test
+  // every four columns) 663-687 us.
   uint32_t nxt[16];
+  auto load_block = [&](uint32_t blk) {
+    const char* col = reinterpret_cast<const char*>(cols) + (size_t)blk * 64 * col_stride;
+    const uint32_t left = C - blk * 16;
+    if (left >= 16) {
 #pragma unroll
-  for (int k = 0; k < 16; ++k) nxt[k] = (uint32_t)k < C ? __ldg(cols + (size_t)k * col_stride + r) : 0u;
+      for (int k = 0; k < 16; ++k)
+        nxt[k] = __ldg(reinterpret_cast<const uint32_t*>(col + (size_t)k * 4 * col_stride + row_bytes));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        nxt[k] = (uint32_t)k < left
+                     ? __ldg(reinterpret_cast<const uint32_t*>(col + (size_t)k * 4 * col_stride + row_bytes))
+                     : 0u;
+    }
+  };
+  auto add_product = [&](uint32_t w, uint32_t v) {
+    const uint4 g = sg[w];
+    acc0 += (uint64_t)g.x * v;
+    acc1 += (uint64_t)g.y * v;
+    acc2 += (uint64_t)g.z * v;
+    acc3 += (uint64_t)g.w * v;
+  };
+  auto fold_sums = [&] {
+    acc0 = fold_high(acc0);
+    acc1 = fold_high(acc1);
+    acc2 = fold_high(acc2);
+    acc3 = fold_high(acc3);
+  };
+  load_block(0);
   for (uint32_t blk = 0; blk < nblocks; ++blk) {
     uint32_t m[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) m[k] = nxt[k];
-    if (blk + 1 < nblocks) {
+    if (blk + 1 < nblocks) load_block(blk + 1);
+    if (comb && blk * 16 + 16 <= C) {
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
-        const uint32_t w = (blk + 1) * 16 + k;
-        nxt[k] = w < C ? __ldg(cols + (size_t)w * col_stride + r) : 0u;
+        add_product(blk * 16 + k, m[k]);
+        if (k & 1) fold_sums();
       }
-    }
-    if (comb) {
+    } else if (comb) {
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
-        const uint32_t w = blk * 16 + k;
-        if (w < C) {
-          const uint4 g = sg[w];
-          const uint32_t v = m[k];
-          acc0 += (uint64_t)g.x * v;
-          acc1 += (uint64_t)g.y * v;
-          acc2 += (uint64_t)g.z * v;
-          acc3 += (uint64_t)g.w * v;
-        }
-        if (k & 1) {
-          acc0 = fold_high(acc0);
-          acc1 = fold_high(acc1);
-          acc2 = fold_high(acc2);
-          acc3 = fold_high(acc3);
-        }
+        if (blk * 16 + k < C) add_product(blk * 16 + k, m[k]);
+        if (k & 1) fold_sums();
       }
     }
     const int rem = (int)(C * 4) - (int)(blk * 64);
