@@ -35,3 +35,26 @@ def test_fold128_either_way_matches_oracle(orc, m, length):
     native.binius_fold_device(128, d_cur.data_ptr(), length, m, r, d_next.data_ptr(), d_scratch.data_ptr())
     torch.cuda.synchronize()
     assert bytes(d_next.cpu().numpy()) == orc.binius_fold(7, cur, length, m, r)
+
+
+@pytest.mark.parametrize("over", [1, 2, 257])
+def test_fold128_table_equals_direct(orc, over):
+    """The most elements that the direct fold takes, and `over` more, which go through the
+    multiply table: equal rows, and the rows past the line as the oracle has them."""
+    import torch
+    from zs_b200 import native
+    half = 1 << 18
+    rng = np.random.default_rng(over)
+    cur = rng.bytes((half + over) * 32)
+    r = int.from_bytes(rng.bytes(16), "little")
+    d_cur = torch.frombuffer(bytearray(cur), dtype=torch.uint8).to("cuda")
+    d_scratch = torch.zeros(65536, dtype=torch.uint8, device="cuda")
+    outs = []
+    for rows in (half, half + over):
+        d_next = torch.zeros(rows * 16, dtype=torch.uint8, device="cuda")
+        native.binius_fold_device(128, d_cur.data_ptr(), 2 * rows, 1, r, d_next.data_ptr(), d_scratch.data_ptr())
+        torch.cuda.synchronize()
+        outs.append(bytes(d_next.cpu().numpy()))
+    assert outs[0] == outs[1][:16 * half]
+    for lo, hi in ((0, 512), (half, half + over)):
+        assert outs[1][16 * lo:16 * hi] == orc.binius_fold(7, cur[32 * lo:32 * hi], 2 * (hi - lo), 1, r)

@@ -1072,7 +1072,10 @@ void values_async(bool wide, const void* d_cur, size_t len, size_t half, size_t 
     ZS_CUDA(cudaLaunchKernel(fn, grid, dim3(kBThreads), args, 65536 + 4 * words, st));
 }
 
-constexpr size_t kDirectFold = (size_t)1 << 16;  // elements up to which the direct fold is used
+// Elements up to which the direct fold is used: two tables folded to 2^16 elements in all 6.2 us
+// (10.6 with the multiply table's launch), to 2^17 10.3 (16.4), to 2^18 17.3 (20.5); from there
+// on the lookups outweigh the launch.
+constexpr size_t kDirectFold = (size_t)1 << 18;
 // next (m tables of len / 2) = fold of cur (m tables of len) at r, asynchronously on `st`.
 // r_mul: a 64 KB device buffer for the GF(2^128) multiply table.
 void fold_async(bool wide, const void* d_cur, size_t len, size_t m, u128 r, const uint8_t* d_r, void* d_next,
