@@ -493,7 +493,8 @@ __device__ __forceinline__ void finish_values(const uint32_t* s_acc, uint32_t wo
 
 // The fold of the round before, taken by the values kernel that needs its outputs: `cur` holds
 // the tables before it (of 2 len elements), r is its challenge; the folded tables (of len) go
-// to `next`.
+// to `next`. The fold's own launch, its load of the challenge's row and its pass over the tables
+// go: with the launches overlapped, a GF(2^8) proof of 2^22 rows 574 -> 522 us.
 struct Folding {
   const uint8_t* r;
   void* next;
@@ -826,7 +827,8 @@ __device__ __forceinline__ void values_shared(const Tower& F, const E* tab, uint
 // A GF(2^128) round with the fold before it, in chunks of R rows per CTA: the CTA folds the 2R
 // elements of each table that its rows need (products by the challenge in full, 121 lookups)
 // into shared memory and `next`, and takes their values from there. Fold and values were two
-// launches (three with the multiply table), each with a load of the product table.
+// launches (three with the multiply table), each with a load of the product table: a proof of
+// 2^16 rows 447 -> 393 us with the launches overlapped.
 // Shared memory: the product table, accumulators, the chunk of m tables.
 __global__ void __launch_bounds__(kBThreads, 2) k_sc_round128(const uint4* __restrict__ cur, uint32_t len, uint32_t m,
                                                               uint32_t R, const __grid_constant__ Terms tm,
@@ -871,7 +873,9 @@ __global__ void __launch_bounds__(kBThreads, 2) k_sc_round128(const uint4* __res
 // The last rounds of a proof in one CTA: the tables (m of `len` elements each, in `cur`)
 // come to shared memory and stay there, and each round is its values, the step and the
 // fold, a barrier apart; a round of few rows is otherwise three launches and as many loads
-// of the product table. A warp takes 32 rows (or 128) at one point at a time.
+// of the product table: 20-24 us a round, here 6-10 us (a GF(2^8) proof of 2^22 rows 780 ->
+// 574 us with the step in the values kernel). A warp takes 32 rows (or 128) at one point at a
+// time. Bound by the step, a chain of SHA-256 blocks.
 // Shared memory: the product table, the tables, half as much for their folds.
 constexpr unsigned kTailThreads = 512;
 constexpr size_t kTailBytes = (size_t)64 << 10;  // of tables
@@ -1165,7 +1169,7 @@ void store_elem(uint8_t* p, size_t es, u128 v) {
 
 // Lagrange interpolation through the points 0..n-1 (sumcheck.zig:124-162) as a matrix:
 // row i holds the low-first coefficients of prod_{j != i} (x + j) / (i + j), so a round's
-// coefficients are coeffs[d] = sum_i values[i] * lag[i][d] (k_sc_step). The matrix
+// coefficients are coeffs[d] = sum_i values[i] * lag[i][d] (sc_step). The matrix
 // depends on the points only and is built once per proof, on the host.
 std::vector<std::vector<u128>> lagrange_matrix(const HostTower& ht, unsigned level, size_t n) {
   std::vector<std::vector<u128>> lag(n, std::vector<u128>(n, 0));
@@ -1199,8 +1203,14 @@ uint64_t tail_row_cost(bool wide, size_t m, const Terms& tm, size_t pts) {
   }
   return c;
 }
+// Lookups of a round up to which one CTA takes it and the rest: a launched round costs about
+// 10 us of launches and tables, the CTA that much for this many lookups. Half as many: GF(2^128)
+// 2^13 rows 241 -> 255 us, GF(2^8) equal; twice as many: GF(2^8) 2^16 rows 185 -> 201 us.
 constexpr uint64_t kTailCost = (uint64_t)3 << 14;
-constexpr size_t kFusedFold = (size_t)3 << 16;  // elements up to which a round's fold is taken in full products
+// Elements up to which a GF(2^128) round's fold is taken in full products with its values, in
+// place of two more launches (the multiply table's and the fold's, 10 us): 2^13 rows 241 us,
+// 248 with half as many; twice as many changes less than the runs differ.
+constexpr size_t kFusedFold = (size_t)3 << 16;
 
 int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, size_t m, const uint8_t* coeffs,
                           size_t nterms, const uint32_t* indices, size_t n_indices, const uint32_t* offsets,

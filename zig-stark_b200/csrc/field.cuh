@@ -55,7 +55,8 @@ ZS_HD uint32_t mpow(uint32_t a, uint32_t e) {
 }
 // a^(p-2); 0 maps to 0 exactly as the reference's release build does. By the addition chain
 // 1, 2, 3, 6, 7, 14, 28, 29 on the exponents 2^k - 1, and p - 2 = 4 (2^29 - 1) + 1: 38
-// products in place of binary exponentiation's 60.
+// products in place of binary exponentiation's 60 (stacked Rescue 2^18: quotient 197 -> 190 us,
+// DEEP 110 -> 107 us, proof 3.88 -> 3.84 ms).
 ZS_HD uint32_t minv(uint32_t a) {
   auto up = [](uint32_t x, int k) {  // x^(2^k)
     for (int i = 0; i < k; ++i) x = mmul(x, x);
@@ -104,6 +105,8 @@ ZS_HD qm31 qneg(qm31 x) { return {cneg(x.a), cneg(x.b)}; }
 // the high word takes it off; then the high word is at most p + 1 and two more products of
 // words <= p keep the sum below 2^64. A term is 16 wide multiply-adds and 8 minima, against 9
 // reduced products and 27 reduced sums (63 ALU operations) for qmul's Karatsuba form and its sum.
+// stacked Rescue 2^18: quotient 230 -> 197 us, DEEP 165 -> 110 us; the linear layer's proof 12.2 ->
+// 12.0 ms.
 struct QAcc {
   uint64_t v[4] = {0, 0, 0, 0};
   ZS_HD static uint64_t fold(uint64_t x) {

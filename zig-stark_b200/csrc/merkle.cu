@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(kThreads) k_row_leaves(const uint32_t* __restr
   // compressed, so their latency hides behind ~700 integer instructions. Only a row's last
   // block can be a part of one: the others take their loads and products without a
   // comparison of the column, from column addresses that are the same in every thread.
-  // Bound by the ALU pipe and the issue slots at once: 64 columns x 2^22 rows 761 -> 650 us,
+  // Bound by the ALU pipe and the issue slots at once: 64 columns x 2^22 rows 761 -> 644 us,
   // 4950 -> 4230 instructions a row, 2460 -> 2150 of them on the ALU (1792 in the four
   // compressions). With one copy of the product code for whole and partial blocks (a test
   // every four columns) 663-687 us.

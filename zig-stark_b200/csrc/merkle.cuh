@@ -56,7 +56,10 @@ constexpr uint32_t kTreeBatch = 64;
 void build_qm31_trees(const qm31* d_values, size_t v_stride, DeviceTree* const* trees, uint32_t count,
                       cudaStream_t st);
 // Trees of several sizes up to 2^kSmallTreeLog, each over its own values: small trees are
-// chains of levels, so one launch takes the time of its largest.
+// chains of levels, so one launch takes the time of its largest; but it waits for the last
+// layer's fold, and trees of more leaves take their levels faster in launches of their own.
+// From 2^13 down: a commit of 8 x 2^18 520 us against 511, of 37 x 2^15 247 against 243; from
+// 2^15 down: 499 and 246, but 16 x 2^13 115 against 105 (8 x 2^10: equal).
 constexpr unsigned kSmallTreeLog = 14;
 void build_small_trees(const qm31* const* d_values, DeviceTree* const* trees, uint32_t count, cudaStream_t st);
 // Completes the levels above `from_level` (levels <= from_level must be written).
