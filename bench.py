@@ -882,10 +882,10 @@ def main():
     # DRAM read + write bytes per launch of each phase's kernels from ncu, scaled by the
     # rows. LDE: its three kernels at 32 columns x 2^20 rows (1.945 GB; the intermediate
     # buffers are larger than L2 there too) scaled to 64 columns. Row leaves + trees: the
-    # row leaves and the row and g trees of this workload (1381.5 MB read, 443.0 MB
+    # row leaves and the row and g trees of this workload (1294.8 MB read, 468.6 MB
     # written; one pass per launch, checked on the 32-column case first).
     traffic = {"lde": 1.9454e9 * (N_COLS / 32) * 2.0 ** (log_rows - 20),
-               "row_tree": 1.8245e9 * 2.0 ** (log_rows - 20)}.get(dom)
+               "row_tree": 1.7634e9 * 2.0 ** (log_rows - 20)}.get(dom)
     # Integer co-roof. The path is exact integer work, so next to the HBM roof each phase
     # is set against the SMs' issue rate (148 SMs x 4 schedulers x 1 warp instruction per
     # cycle at the sampled SM clock) and against the ALU pipe's (a warp instruction every
@@ -894,7 +894,7 @@ def main():
     # sm__inst_executed_pipe_alu.sum of one captured step at 64 x 2^20, summed over each
     # phase's kernels), over the CUDA-event phase time of this run. Other row counts
     # scale the counts by the rows (marked).
-    counted = {"lde": (946.8e6, 488.4e6), "row_tree": (1059.4e6, 735.3e6), "folds": (342.0e6, 237.1e6)}
+    counted = {"lde": (946.8e6, 488.4e6), "row_tree": (1077.6e6, 588.0e6), "folds": (369.2e6, 212.0e6)}
     cs = clocks.summary()
     sm_mhz = cs.get("sm_mhz") or cs.get("sm_max_mhz") or 1965.0
     n_sm = torch.cuda.get_device_properties(local).multi_processor_count
