@@ -92,7 +92,10 @@ inline void retain_some_pool_memory() {
 // A launch that may start while the kernel before it on the stream ends (programmatic stream
 // serialization). Every thread of such a kernel takes after_previous() before it touches
 // what earlier work wrote or still reads; the kernel before lets it come up early with
-// let_next_start(). Both do nothing in an ordinary launch.
+// let_next_start(). Both do nothing in an ordinary launch. What the launches before it on the
+// stream write changes during the kernel's life, so the kernel reads it with plain or __ldcg
+// loads: __ldg, and loads through const __restrict__ parameters, which the compiler may turn
+// into the same, are for what was there before the first launch of the chain.
 inline void launch_overlapped(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t st) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;

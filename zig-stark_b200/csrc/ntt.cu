@@ -179,8 +179,15 @@ struct NttPass {
   unsigned in_mode, out_mode, logN, lo, M, lgG, lgH;
 };
 
+// Component c of a table's entry: the tables are written before any pass is launched.
 __device__ __forceinline__ cm31 ldc(const qm31* p, uint32_t c) {
   const uint2 r = __ldg(reinterpret_cast<const uint2*>(p) + c);
+  return {r.x, r.y};
+}
+// Component c of what an earlier pass wrote, which may end while this one's CTAs are up: a
+// plain load, never the read-only path (launch_overlapped).
+__device__ __forceinline__ cm31 ld_pass(const qm31* p, uint32_t c) {
+  const uint2 r = reinterpret_cast<const uint2*>(p)[c];
   return {r.x, r.y};
 }
 
@@ -321,10 +328,9 @@ __global__ void __launch_bounds__(1 << (kTileLog - 2), 2) k_ntt_pass(const __gri
           const qm31 x = to_crt(ldq(src + j));
           v[m] = c ? x.b : x.a;
         } else if (p.in_mode == kExpand) {
-          v[m] = ldc(src + (j >> lo), c);
+          v[m] = ld_pass(src + (j >> lo), c);
         } else {
-          const uint2 r = reinterpret_cast<const uint2*>(col + j)[c];
-          v[m] = {r.x, r.y};
+          v[m] = ld_pass(col + j, c);
         }
       }
     } else {
