@@ -504,8 +504,10 @@ struct Folding {
 // values[t]). D > 0: the D = dmax + 1 points in registers, every row once. D = 0: one
 // point per pass, points t = blockIdx.y, blockIdx.y + gridDim.y, ... (a grid of dmax + 1
 // rows of CTAs gives each point its own CTAs when the rows alone cannot fill the GPU).
+// `cur` is not __restrict__: in a prover's overlapped rounds the launch before may still be
+// writing it when this one's CTAs come up, so its loads must not take the read-only path.
 template <int D, bool FOLD>
-__global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* __restrict__ cur, uint32_t len, uint32_t half,
+__global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* cur, uint32_t len, uint32_t half,
                                                        uint32_t dmax, const __grid_constant__ Terms tm,
                                                        const uint8_t* __restrict__ gT, uint32_t* __restrict__ out,
                                                        const __grid_constant__ ScStep step,
@@ -621,9 +623,9 @@ __device__ __forceinline__ g128 load_g128(const uint4* p) {
   return {(uint64_t)v.y << 32 | v.x, (uint64_t)v.w << 32 | v.z};
 }
 
-// GF(2^128) round; out: (dmax + 1) values of four little-endian words. D as k_values8.
+// GF(2^128) round; out: (dmax + 1) values of four little-endian words. D and `cur` as k_values8.
 template <int D>
-__global__ void __launch_bounds__(kBThreads, (D >= 1 && D <= 4) ? 2 : 1) k_values128(const uint4* __restrict__ cur, uint32_t len, uint32_t half,
+__global__ void __launch_bounds__(kBThreads, (D >= 1 && D <= 4) ? 2 : 1) k_values128(const uint4* cur, uint32_t len, uint32_t half,
                                                          uint32_t dmax, const __grid_constant__ Terms tm,
                                                          const uint8_t* __restrict__ gT, uint32_t* __restrict__ out,
                                                          const __grid_constant__ ScStep step) {
@@ -830,7 +832,7 @@ __device__ __forceinline__ void values_shared(const Tower& F, const E* tab, uint
 // launches (three with the multiply table), each with a load of the product table: a proof of
 // 2^16 rows 447 -> 393 us with the launches overlapped.
 // Shared memory: the product table, accumulators, the chunk of m tables.
-__global__ void __launch_bounds__(kBThreads, 2) k_sc_round128(const uint4* __restrict__ cur, uint32_t len, uint32_t m,
+__global__ void __launch_bounds__(kBThreads, 2) k_sc_round128(const uint4* cur, uint32_t len, uint32_t m,
                                                               uint32_t R, const __grid_constant__ Terms tm,
                                                               const uint8_t* __restrict__ gT,
                                                               uint32_t* __restrict__ out,
@@ -880,7 +882,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_sc_round128(const uint4* __res
 constexpr unsigned kTailThreads = 512;
 constexpr size_t kTailBytes = (size_t)64 << 10;  // of tables
 template <bool WIDE>
-__global__ void __launch_bounds__(kTailThreads) k_sc_tail(const void* __restrict__ cur, uint32_t len, uint32_t m,
+__global__ void __launch_bounds__(kTailThreads) k_sc_tail(const void* cur, uint32_t len, uint32_t m,
                                                           uint32_t rounds, const __grid_constant__ Terms tm,
                                                           const uint8_t* __restrict__ gT,
                                                           const __grid_constant__ ScStep step) {
