@@ -47,10 +47,12 @@ int32_t circle_transform(const uint32_t* in, uint32_t n_columns, uint32_t ox, ui
     ensure_device();
     const unsigned lg = log_half + 1;
     const size_t n = (size_t)1 << lg;
+    // The legacy default stream and plain copies: the call is ordered after what the caller
+    // has queued on that stream and on every blocking one, an asynchronous copy into `in`
+    // among it. (On a stream of the thread's own, with `in` staged by host threads, a copy
+    // still in flight was overtaken.)
     cudaStream_t st = nullptr;
-    thread_stream(0, &st);  // the calling thread's stream on the current device
     retain_some_pool_memory();
-    PinnedScope pinned(st);
     const size_t words = n * n_columns;
     struct Buffers {  // input, output, scratch
       uint32_t* p = nullptr;
@@ -59,13 +61,12 @@ int32_t circle_transform(const uint32_t* in, uint32_t n_columns, uint32_t ox, ui
       ~Buffers() { cudaFreeAsync(p, st); }
     } buf(words, st);
     CircleDomain dom(lg, cpoint{ox, oy}, cpoint{sx, sy}, st);
-    upload_bytes(buf.p, in, words * 4, st);
+    ZS_CUDA(cudaMemcpy(buf.p, in, words * 4, cudaMemcpyHostToDevice));
     if (inverse)
       circle_ifft(buf.p, buf.p + words, n_columns, dom, buf.p + 2 * words, st);
     else
       circle_fft(buf.p, buf.p + words, n_columns, dom, buf.p + 2 * words, st);
-    ZS_CUDA(cudaMemcpyAsync(out, buf.p + words, words * 4, cudaMemcpyDeviceToHost, st));
-    ZS_CUDA(cudaStreamSynchronize(st));
+    ZS_CUDA(cudaMemcpy(out, buf.p + words, words * 4, cudaMemcpyDeviceToHost));
   });
 }
 
