@@ -193,7 +193,11 @@ int32_t zs_m31_commit_columns(zs_host_allocator host, uint8_t trace_log, uint8_t
  * half_coset ++ conjugate, coefficients use the A-then-B layout, evaluations are in
  * natural domain order. n = 2^(log_half + 1) words, n_columns transforms in a row
  * (column c at offset c * n). Host buffers. Bit-identical to the CPU transform for
- * every size (the reference falls back to the CPU below 8 points; this does not). */
+ * every size (the reference falls back to the CPU below 8 points; this does not).
+ * Ordered after the work queued on the default stream and on blocking streams (an
+ * asynchronous copy into pinned input among it); returns when the output is there. A
+ * workspace of up to 64 MB stays in the device's stream-ordered pool until the program's
+ * next synchronization with the device; a larger one is given back before the return. */
 int32_t zs_m31_circle_fft(const uint32_t *coeffs, uint32_t n_columns, uint32_t offset_x, uint32_t offset_y,
                           uint32_t step_x, uint32_t step_y, uint32_t log_half, uint32_t *evals);
 int32_t zs_m31_circle_ifft(const uint32_t *evals, uint32_t n_columns, uint32_t offset_x, uint32_t offset_y,

@@ -17,7 +17,6 @@ CommitPlan::CommitPlan(uint32_t C_, unsigned L_, unsigned B_, unsigned F_) : C(C
   if (C == 0 || C > 256) throw Error(ZS_EMALFORMED, "n_columns must be in [1, 256]");
   if (L < 1 || L + B > 28) throw Error(ZS_EMALFORMED, "log_rows + log_blowup must be in [1, 28]");
   if (F > L + B) throw Error(ZS_EMALFORMED, "more folds than domain bits");
-  retain_some_pool_memory();  // plans of small configurations come and go
   ZS_CUDA(cudaStreamCreateWithFlags(&setup, cudaStreamNonBlocking));
   ZS_CUDA(cudaStreamCreateWithFlags(&copy, cudaStreamNonBlocking));
   for (auto& s : sides) ZS_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -76,10 +75,11 @@ CommitPlan::CommitPlan(uint32_t C_, unsigned L_, unsigned B_, unsigned F_) : C(C
 CommitPlan::~CommitPlan() {
   cudaDeviceSynchronize();
   drop_graph();
-  cudaFree(base);
   small.reset();
   big.reset();
   tabs.reset();
+  cudaFreeAsync(base, setup);
+  cudaStreamSynchronize(setup);  // the pool gives back what it does not keep
   for (auto& e : events) cudaEventDestroy(e);
   for (auto& e : up_events) cudaEventDestroy(e);
   cudaStreamDestroy(copy);

@@ -46,19 +46,14 @@ ZS_HD uint32_t bitrev(uint32_t x, unsigned bits) {
 #endif
 }
 
-// Held by whoever changes a device's pool setting.
-inline std::mutex& pool_settings_mutex() {
-  static std::mutex mu;
-  return mu;
-}
-
 // Freed blocks stay in the device's stream-ordered pool instead of going back to the
 // driver at every synchronization, so repeated proofs do not map their memory again.
 inline void retain_pool_memory() {
+  static std::mutex mu;
   static uint64_t done = 0;
   int dev = 0;
   ZS_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(pool_settings_mutex());
+  std::lock_guard<std::mutex> lk(mu);
   if (dev < 64 && (done >> dev & 1)) return;
   cudaMemPool_t pool;
   ZS_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
@@ -69,24 +64,6 @@ inline void retain_pool_memory() {
   int no = 0;
   ZS_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no));
   if (dev < 64) done |= 1ull << dev;
-}
-
-// Up to 256 MB of freed blocks stay in the pool (more where retain_pool_memory ran), for
-// entry points that allocate a workspace per call: with none kept, every call's
-// synchronization gives its blocks back to the driver and the next maps them again.
-inline void retain_some_pool_memory() {
-  int dev = 0;
-  ZS_CUDA(cudaGetDevice(&dev));
-  cudaMemPool_t pool;
-  ZS_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
-  uint64_t keep = 0;
-  const uint64_t want = (uint64_t)256 << 20;
-  std::lock_guard<std::mutex> lk(pool_settings_mutex());
-  ZS_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-  if (keep < want) {
-    keep = want;
-    ZS_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-  }
 }
 
 // A launch that may start while the kernel before it on the stream ends (programmatic stream
