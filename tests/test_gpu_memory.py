@@ -47,3 +47,27 @@ def test_memory_is_given_back(call, sync):
     out = subprocess.run([sys.executable, "-c", SCRIPT.format(call=call, sync=sync)], env=env, capture_output=True,
                          text=True, timeout=300)
     assert out.returncode == 0, out.stderr[-2000:]
+
+
+PINNED = """
+import numpy as np, torch
+from zs_b200 import native
+
+def pinned():  # the driver's pinned blocks are shared memory
+    return next(line.split()[1] for line in open("/proc/self/status") if line.startswith("RssShmem"))
+
+p = native.CommitPlan(8, 10, 2, 6)
+p.set_challenges(np.ones((8, 4), dtype=np.uint32), np.ones((6, 4), dtype=np.uint32))
+p.upload(np.ones((8, 1 << 10), dtype=np.uint32))
+p.run()
+torch.cuda.synchronize()
+before = pinned()
+p.results()
+assert pinned() == before, f"{before} -> {pinned()} kB"
+"""
+
+
+def test_results_leave_no_pinned_memory():
+    env = {**os.environ, "PYTHONPATH": os.path.join(ROOT, "zig-stark_b200")}
+    out = subprocess.run([sys.executable, "-c", PINNED], env=env, capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]

@@ -6,12 +6,10 @@
 #include <mutex>
 #include <new>
 #include <thread>
-#include <vector>
 
 #include "../../include/zs_m31.h"
 #include "circle.cuh"
 #include "commit.cuh"
-#include "staging.cuh"
 #include "stark.cuh"
 #include "verify.cuh"
 
@@ -154,21 +152,7 @@ int32_t zs_m31_commit_plan_results(zs_commit_plan* plan, void* stream, uint8_t* 
                                    uint32_t* final_layer) {
   return guarded([&] {
     if (!plan) throw Error(ZS_EMALFORMED, "null plan");
-    CommitPlan& p = *plan->plan;
-    cudaStream_t st = (cudaStream_t)stream;
-    // The roots lie in one buffer; with a small final layer they come back through pinned
-    // memory with one wait (a pageable copy is a wait of its own, about 8 us each).
-    const size_t final_bytes = ((size_t)1 << (p.L + p.B - p.F)) * sizeof(qm31);
-    const bool final_small = final_bytes <= ((size_t)256 << 10);
-    if (final_layer && !final_small)
-      ZS_CUDA(cudaMemcpyAsync(final_layer, p.layers[p.F], final_bytes, cudaMemcpyDeviceToHost, st));
-    PinnedScope pinned(st);
-    std::vector<D2H> back;
-    if (lde_root) back.push_back({lde_root, p.roots, 32});
-    if (layer_roots && p.F > 0) back.push_back({layer_roots, p.roots + 8, (size_t)32 * p.F});
-    if (final_layer && final_small) back.push_back({final_layer, p.layers[p.F], final_bytes});
-    d2h_many(back.data(), back.size(), st);
-    ZS_CUDA(cudaStreamSynchronize(st));
+    plan->plan->results((cudaStream_t)stream, lde_root, layer_roots, final_layer);
   });
 }
 

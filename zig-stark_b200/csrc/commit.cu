@@ -3,6 +3,7 @@
 // FRI commitment, then the fold chain with one fused fold+commit launch per layer.
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 #include <functional>
 #include <memory>
 #include <vector>
@@ -50,11 +51,13 @@ CommitPlan::CommitPlan(uint32_t C_, unsigned L_, unsigned B_, unsigned F_) : C(C
                              {(void**)&scratch, lde_scratch_words(L, B, C) * sizeof(uint32_t)},
                              {(void**)&gammas, C * sizeof(qm31)},
                              {(void**)&row_tree.words, DeviceTree::words_for(L + B) * sizeof(uint32_t)},
-                             {(void**)&done, (F + 1) * sizeof(uint32_t)},
-                             {(void**)&roots, (F + 1) * 32}};
-  for (unsigned i = 0; i <= F; ++i) parts.push_back({(void**)&layers[i], (N >> i) * sizeof(qm31)});
-  for (unsigned i = 0; i < F; ++i)
+                             {(void**)&done, (F + 1) * sizeof(uint32_t)}};
+  for (unsigned i = 0; i < F; ++i) {
+    parts.push_back({(void**)&layers[i], (N >> i) * sizeof(qm31)});
     parts.push_back({(void**)&layer_trees[i].words, DeviceTree::words_for(L + B - i) * sizeof(uint32_t)});
+  }
+  parts.push_back({(void**)&roots, (F + 1) * 32});  // side by side: results() takes both in one copy
+  parts.push_back({(void**)&layers[F], (N >> F) * sizeof(qm31)});
   size_t total = 0;
   for (const Part& q : parts) total += (q.bytes + 255) & ~(size_t)255;
   ZS_CUDA(cudaMallocAsync((void**)&base, total, setup));
@@ -197,6 +200,28 @@ void CommitPlan::run_host(const uint32_t* h_trace, cudaStream_t st) {
     host_trace = h_trace;
   }
   ZS_CUDA(cudaGraphLaunch(host_exec, st));
+}
+
+// The roots lie just before the final layer: one copy brings both back where the layer is
+// small. A copy into pageable memory is a wait of its own (15 us for a kilobyte, 20 for 64 KB,
+// 33 for 256), three through pinned memory with one wait 18; but pinning takes over a
+// millisecond, so a call that pins has to keep the memory when it returns.
+void CommitPlan::results(cudaStream_t st, uint8_t* lde_root, uint8_t* layer_roots, uint32_t* final_layer) {
+  constexpr size_t kTogether = (size_t)64 << 10;
+  const size_t final_bytes = ((size_t)1 << (L + B - F)) * sizeof(qm31), roots_bytes = (F + 1) * 32;
+  const size_t at = reinterpret_cast<unsigned char*>(layers[F]) - reinterpret_cast<unsigned char*>(roots);
+  const bool together = final_layer && final_bytes <= kTogether;
+  if (final_layer && !together)
+    ZS_CUDA(cudaMemcpyAsync(final_layer, layers[F], final_bytes, cudaMemcpyDeviceToHost, st));
+  if (lde_root || layer_roots || together) {
+    std::vector<uint8_t> back(together ? at + final_bytes : roots_bytes);
+    ZS_CUDA(cudaMemcpyAsync(back.data(), roots, back.size(), cudaMemcpyDeviceToHost, st));
+    ZS_CUDA(cudaStreamSynchronize(st));
+    if (lde_root) std::memcpy(lde_root, back.data(), 32);
+    if (layer_roots) std::memcpy(layer_roots, back.data() + 32, roots_bytes - 32);
+    if (together) std::memcpy(final_layer, back.data() + at, final_bytes);
+  }
+  ZS_CUDA(cudaStreamSynchronize(st));
 }
 
 // Everything after the LDE: row leaves with the gamma combination, the trees, the folds.

@@ -27,7 +27,7 @@ struct CommitPlan {
   DeviceTree row_tree;
   std::vector<DeviceTree> layer_trees;  // trees of layers 0 .. F-1
   uint32_t* done = nullptr;   // the trees' counters: row tree, then the layers
-  uint32_t* roots = nullptr;  // their roots, 8 words each, in the same order
+  uint32_t* roots = nullptr;  // their roots, 8 words each, in the same order; before layers[F]
 
   CommitPlan(uint32_t C, unsigned L, unsigned B, unsigned F);
   ~CommitPlan();
@@ -46,6 +46,8 @@ struct CommitPlan {
   // the step; replayed as one captured graph per host pointer.
   void run_host(const uint32_t* h_trace, cudaStream_t st);
   void run_host_direct(const uint32_t* h_trace, cudaStream_t st);
+  // The roots and the final layer on the host, after what is queued on `st`; any may be null.
+  void results(cudaStream_t st, uint8_t* lde_root, uint8_t* layer_roots, uint32_t* final_layer);
   // Column counts of the upload groups, largest first: after the last copy only the
   // last (smallest) group's LDE precedes the rest of the step.
   std::vector<uint32_t> upload_groups;
