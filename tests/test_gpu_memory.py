@@ -62,12 +62,15 @@ p.upload(np.ones((8, 1 << 10), dtype=np.uint32))
 p.run()
 torch.cuda.synchronize()
 before = pinned()
-p.results()
-assert pinned() == before, f"{before} -> {pinned()} kB"
+{call}
+assert pinned() == before, f"{{before}} -> {{pinned()}} kB"
 """
 
 
-def test_results_leave_no_pinned_memory():
+@pytest.mark.parametrize("call", ["p.results()", "native.circle_fft(np.ones((4, 1 << 18), dtype=np.uint32))",
+                                  "native.binius_prove_combination(8, bytes(3 << 12), 12, 3, [([0, 1, 2], 1)])"])
+def test_no_pinned_memory_stays(call):
     env = {**os.environ, "PYTHONPATH": os.path.join(ROOT, "zig-stark_b200")}
-    out = subprocess.run([sys.executable, "-c", PINNED], env=env, capture_output=True, text=True, timeout=300)
+    out = subprocess.run([sys.executable, "-c", PINNED.format(call=call)], env=env, capture_output=True, text=True,
+                         timeout=300)
     assert out.returncode == 0, out.stderr[-2000:]

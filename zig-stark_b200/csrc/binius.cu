@@ -47,7 +47,6 @@
 
 #include "../../include/zs_binius.h"
 #include "common.cuh"
-#include "staging.cuh"
 
 namespace zs {
 namespace {
@@ -1248,7 +1247,6 @@ int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, 
 
     cudaStream_t st = (cudaStream_t)stream;
     retain_pool_memory();
-    PinnedScope pinned(st);
     const size_t words = wide ? 4 * (dmax + 1) : (dmax + 4) / 4;
     DevMem<uint4> d_a((m * n * es + 15) / 16, st), d_b((m * (n / 2) * es + 15) / 16, st);
     DevMem<uint4> d_rmul(wide && m * (n / 2) > kDirectFold ? 4096 : 0, st);
@@ -1258,7 +1256,7 @@ int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, 
       for (size_t d = 0; d < pts; ++d) lag_b[a * pts + d] = (uint8_t)lag[a][d];
     // One block for the device transcript's inputs and outputs: the values' accumulators and
     // the counter (zero between rounds), the state and challenge, the Lagrange matrix, the
-    // seed, the claimed sum and every round's coefficients.
+    // seed, then, for one copy back, the claimed sum and every round's coefficients.
     size_t at = 0;
     auto part = [&](size_t bytes) {
       const size_t o = at;
@@ -1271,7 +1269,7 @@ int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, 
     DevMem<uint4> d_aux(at / 16, st);
     uint8_t* const aux = reinterpret_cast<uint8_t*>(d_aux.p);
     ZS_CUDA(cudaMemsetAsync(aux, 0, o_tx, st));
-    h2d_small(aux + o_lag, lag_b.data(), lag_b.size(), st);
+    ZS_CUDA(cudaMemcpyAsync(aux + o_lag, lag_b.data(), lag_b.size(), cudaMemcpyHostToDevice, st));
     if (has_seed && seed_len) ZS_CUDA(cudaMemcpyAsync(aux + o_seed, seed, seed_len, cudaMemcpyHostToDevice, st));
     ZS_CUDA(cudaMemcpyAsync(d_a.p, tables, m * n * es, cudaMemcpyHostToDevice, st));
     const uint8_t* T = device_state(st).table;
@@ -1329,8 +1327,11 @@ int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, 
       }
       pending = true;
     }
-    const D2H back[2] = {{claimed_out, aux + o_claimed, es}, {rounds_out, aux + o_rounds, k * pts * es}};
-    d2h_many(back, 2, st);
+    std::vector<uint8_t> back(o_rounds - o_claimed + k * pts * es);
+    ZS_CUDA(cudaMemcpyAsync(back.data(), aux + o_claimed, back.size(), cudaMemcpyDeviceToHost, st));
+    ZS_CUDA(cudaStreamSynchronize(st));
+    std::memcpy(claimed_out, back.data(), es);
+    std::memcpy(rounds_out, back.data() + (o_rounds - o_claimed), k * pts * es);
   });
 }
 
