@@ -58,3 +58,48 @@ def test_fold128_table_equals_direct(orc, over):
     assert outs[0] == outs[1][:16 * half]
     for lo, hi in ((0, 512), (half, half + over)):
         assert outs[1][16 * lo:16 * hi] == orc.binius_fold(7, cur[32 * lo:32 * hi], 2 * (hi - lo), 1, r)
+
+
+@pytest.mark.parametrize("points", range(1, 9))
+def test_fold_fused_round_at_every_point_count(orc, points):
+    """2^18 rows over GF(2^8): the second round folds and takes its values with all points in
+    registers. Four tables, one of which no term names."""
+    from zs_b200 import native
+    terms = [([0, 3, 1, 0, 3, 1, 0][:points - 1], 3)]
+    if points > 1:
+        terms.append(([1], 1))
+    rng = np.random.default_rng(1100 + points)
+    tables = rng.bytes(4 << 18)
+    got = native.binius_prove_combination(8, tables, 18, 4, terms)
+    assert got == orc.binius_prove(3, tables, 18, 4, terms)
+
+
+@pytest.mark.parametrize("k,m", [(8, 20), (8, 21), (8, 40), (8, 41)])
+def test_chunks_of_gf128_rounds(orc, k, m):
+    """Chunks of 64 rows (up to 20 tables), of 32 (up to 40), and a launch of its own for the
+    fold beyond: two tables are named by terms."""
+    from zs_b200 import native
+    rng = np.random.default_rng(1200 + m)
+    tables = rng.bytes(m * 16 << k)
+    terms = [([0, m - 1], 5), ([0], 1)]
+    got = native.binius_prove_combination(128, tables, k, m, terms)
+    named = tables[:16 << k] + tables[(m - 1) * 16 << k:]  # the others change nothing
+    assert got == orc.binius_prove(7, named, k, 2, [([0, 1], 5), ([0], 1)])
+
+
+@pytest.mark.parametrize("k,m,terms", [(18, 5, [([4, 4], 1 << 90)]), (14, 33, [([32], 3), ([0, 32], 7)])])
+def test_gf128_fold_by_the_table(orc, k, m, terms):
+    """More than 2^18 elements to fold: the multiply table's launch, with the challenge in device
+    memory, before values with the points in registers (2^18 rows) or in CTAs of their own, and
+    the fused rounds after. Verified over the tables that the terms name."""
+    from zs_b200 import native
+    rng = np.random.default_rng(1300 + k)
+    tables = rng.bytes(m * 16 << k)
+    claimed, rounds = native.binius_prove_combination(128, tables, k, m, terms)
+    names = sorted({f for fs, _ in terms for f in fs})
+    named = b"".join(tables[f * 16 << k:(f + 1) * 16 << k] for f in names)
+    renamed = [([names.index(f) for f in fs], c) for fs, c in terms]
+    assert orc.binius_verify(7, named, k, len(names), renamed, claimed, rounds)
+    bad = bytearray(rounds)
+    bad[len(bad) // 2] ^= 1
+    assert not orc.binius_verify(7, named, k, len(names), renamed, claimed, bytes(bad))
