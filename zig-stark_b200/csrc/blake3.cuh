@@ -84,13 +84,17 @@ static __constant__ uint32_t kPairPrefix[3] = {0x2d67697au, 0x72617473u, 0x61703
 // additions, which the FMA pipe (64 integer lanes too) executes as well when they have two
 // operands. Written plainly, a + b + m becomes one three-operand add on the ALU: 10 ALU
 // operations per G against 2 on the FMA pipe, and the hash kernels ran the ALU at 83-94 %.
-// add_fma keeps a + m out of it, as a * 1 + m with a 1 that the compiler cannot see (the
-// block's z extent: every launch of this library is one-dimensional), and the sum with b
-// is then a two-operand add: 8 ALU and 6 FMA operations per G. Measured on
+// add_fma keeps a + m out of it, as a * 1 + m with a 1 that the compiler cannot see, the
+// block's z extent, and the sum with b is then a two-operand add: 8 ALU and 6 FMA operations per G. Measured on
 // one B200 over 148 x 16 CTAs of chained hashes: a compression of 16 unknown words 31.8 ->
 // 38.9 G/s, hash2 34.5 -> 38.9 G compressions/s (ALU bound of the 8: 41.6). Sending more
 // over (rotations as the halves of a wide product, c + d as a product) was slower in every
 // combination: a wide product takes two FMA slots and its halves an extra add.
+// PRECONDITION of every device hash (compress_cv, hash_qm31, hash2, hash_words, the
+// transcript's compress): the kernel is launched with a block of z extent 1; with another,
+// every digest is wrong. launch_overlapped refuses such a block, and the other launches give
+// their block as one number. (The 1 from a __constant__ word needs no such rule but measured
+// slower: commits of 64 x 2^20 3192 -> 3230 us, 37 x 2^15 230.4 -> 234.6, 8 x 2^10 82.1 -> 85.5.)
 __device__ __forceinline__ uint32_t add_fma(uint32_t a, uint32_t m) {
   uint32_t r;
   asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(blockDim.z), "r"(m));

@@ -74,6 +74,7 @@ inline void retain_pool_memory() {
 // loads: __ldg, and loads through const __restrict__ parameters, which the compiler may turn
 // into the same, are for what was there before the first launch of the chain.
 inline void launch_overlapped(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t st) {
+  if (block.z != 1) throw Error(ZS_EGENERIC, "a block's z extent is 1 (b3::add_fma)");
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
