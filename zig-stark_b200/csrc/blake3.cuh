@@ -90,7 +90,7 @@ static __constant__ uint32_t kPairPrefix[3] = {0x2d67697au, 0x72617473u, 0x61703
 // 38.9 G/s, hash2 34.5 -> 38.9 G compressions/s (ALU bound of the 8: 41.6). Sending more
 // over (rotations as the halves of a wide product, c + d as a product) was slower in every
 // combination: a wide product takes two FMA slots and its halves an extra add.
-// PRECONDITION of every device hash (compress_cv, hash_qm31, hash2, hash_words, the
+// PRECONDITION of every device hash (compress_cv, hash_qm31, hash2, the
 // transcript's compress): the kernel is launched with a block of z extent 1; with another,
 // every digest is wrong. launch_overlapped refuses such a block, and the other launches give
 // their block as one number. (The 1 from a __constant__ word needs no such rule but measured
@@ -252,27 +252,6 @@ ZS_HD void hash2(const uint32_t l[8], const uint32_t r[8], uint32_t out[8]) {
 #pragma unroll
   for (int k = 4; k < 16; ++k) m2[k] = 0;
   compress_cv<0xfff0u>(out, m2, 14, CHUNK_END | ROOT);
-}
-
-// Blake3 of a single-chunk message given as `nwords` little-endian u32 words
-// (nwords * 4 <= 1024), e.g. hashM31s over a row (src/m31/hash.zig:15-25).
-template <typename Loader>
-ZS_HD void hash_words(int nwords, Loader load, uint32_t out[8]) {
-  iv(out);
-  int nblocks = (nwords * 4 + 63) / 64;
-  if (nblocks == 0) nblocks = 1;
-  for (int blk = 0; blk < nblocks; ++blk) {
-    uint32_t m[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      int w = blk * 16 + k;
-      m[k] = w < nwords ? load(w) : 0u;
-    }
-    int rem = nwords * 4 - blk * 64;
-    uint32_t len = rem >= 64 ? 64u : (uint32_t)rem;
-    uint32_t flags = (blk == 0 ? CHUNK_START : 0) | (blk == nblocks - 1 ? (CHUNK_END | ROOT) : 0);
-    compress_cv(out, m, len, flags);
-  }
 }
 
 }  // namespace b3

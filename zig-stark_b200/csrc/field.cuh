@@ -44,15 +44,6 @@ ZS_HD uint32_t mshl(uint32_t x, unsigned k) {
   uint32_t r = ((x << k) | (x >> (31 - k))) & P;
   return r == P ? 0 : r;
 }
-ZS_HD uint32_t mpow(uint32_t a, uint32_t e) {
-  uint32_t r = 1;
-  while (e) {
-    if (e & 1) r = mmul(r, a);
-    a = mmul(a, a);
-    e >>= 1;
-  }
-  return r;
-}
 // a^(p-2); 0 maps to 0 exactly as the reference's release build does. By the addition chain
 // 1, 2, 3, 6, 7, 14, 28, 29 on the exponents 2^k - 1, and p - 2 = 4 (2^29 - 1) + 1: 38
 // products in place of binary exponentiation's 60 (stacked Rescue 2^18: quotient 197 -> 190 us,
@@ -146,7 +137,6 @@ ZS_HD qm31 qmul(qm31 x, qm31 y) {
 #endif
 }
 ZS_HD qm31 qmul_m(qm31 x, uint32_t s) { return {cmul_m(x.a, s), cmul_m(x.b, s)}; }
-ZS_HD qm31 qmul_c(qm31 x, cm31 s) { return {cmul(x.a, s), cmul(x.b, s)}; }
 // Norm a^2 + i b^2 in CM31; inverse = (a - b j) / norm (qm31.zig:39-48).
 ZS_HD cm31 qnorm(qm31 x) { return cadd(cmul(x.a, x.a), cmul_i(cmul(x.b, x.b))); }
 ZS_HD qm31 qinv(qm31 x) {
@@ -180,7 +170,6 @@ ZS_HD cpoint padd(cpoint p, cpoint q) {
   return {msub(mmul(p.x, q.x), mmul(p.y, q.y)), madd(mmul(p.x, q.y), mmul(p.y, q.x))};
 }
 ZS_HD cpoint pdbl(cpoint p) { return {msub(mmul(p.x, p.x), mmul(p.y, p.y)), mmul(mmul(p.x, p.y), 2)}; }
-ZS_HD cpoint pneg(cpoint p) { return {p.x, mneg(p.y)}; }
 ZS_HD cpoint pmul(cpoint p, uint64_t k) {
   cpoint r = {1, 0};
   while (k) {

@@ -325,35 +325,4 @@ void build_row_leaves(const uint32_t* d_cols, size_t col_stride, uint32_t C, Dev
   ZS_CUDA(cudaGetLastError());
 }
 
-// out[q * log_n * 8 ...] = siblings of indices[q], bottom-up.
-__global__ void k_open_many(const uint32_t* tree_words, unsigned log_n, const uint64_t* indices, uint32_t count,
-                            uint32_t* out) {
-  const uint32_t q = blockIdx.x;
-  if (q >= count) return;
-  const size_t N2 = (size_t)2 << log_n;
-  uint64_t idx = indices[q];
-  for (unsigned lvl = threadIdx.x; lvl < log_n; lvl += blockDim.x) {
-    const uint64_t sib = (idx >> lvl) ^ 1;
-    const uint32_t* s = tree_words + 8 * (N2 - (N2 >> lvl) + sib);
-    uint32_t* o = out + ((size_t)q * log_n + lvl) * 8;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) o[w] = s[w];
-  }
-}
-
-void tree_open_many(const DeviceTree& tree, const uint64_t* d_indices, uint32_t count, uint32_t* d_out,
-                    cudaStream_t st) {
-  if (count == 0 || tree.log_n == 0) return;
-  k_open_many<<<count, 32, 0, st>>>(tree.words, tree.log_n, d_indices, count, d_out);
-  ZS_CUDA(cudaGetLastError());
-}
-
-void tree_open_host(const DeviceTree& tree, uint64_t index, uint8_t* out, cudaStream_t st) {
-  for (unsigned lvl = 0; lvl < tree.log_n; ++lvl) {
-    const uint64_t sib = (index >> lvl) ^ 1;
-    ZS_CUDA(cudaMemcpyAsync(out + 32 * lvl, tree.level(lvl) + 8 * sib, 32, cudaMemcpyDeviceToHost, st));
-  }
-  ZS_CUDA(cudaStreamSynchronize(st));
-}
-
 }  // namespace zs

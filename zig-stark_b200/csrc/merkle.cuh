@@ -67,14 +67,6 @@ void tree_finish(DeviceTree& tree, unsigned from_level, cudaStream_t st);
 // Number of launches that a tree from its leaves' digests or values takes.
 uint32_t tree_launches(unsigned log_n);
 
-// Opening path of leaf `index` (siblings bottom-up, merkle.zig:57-68), read back to
-// the host from a device tree. `out` receives log_n digests of 32 bytes.
-void tree_open_host(const DeviceTree& tree, uint64_t index, uint8_t* out, cudaStream_t st);
-
-// Gathers `count` opening paths at once: out[q] = path of indices[q] (log_n * 32 bytes each).
-void tree_open_many(const DeviceTree& tree, const uint64_t* d_indices, uint32_t count, uint32_t* d_out,
-                    cudaStream_t st);
-
 // Row leaves of C columns x 2^log_n M31 values (column c at d_cols + c * col_stride):
 // leaf r = hashM31s(col_0[r], ..., col_{C-1}[r]) (src/m31/hash.zig:15-25), C <= 256.
 // Also writes g[r] = sum_c gammas[c] * col_c[r] when `d_gammas` is not null. The leaf level
