@@ -366,7 +366,8 @@ struct Hasher {
   // finalize() of the state followed by `n` <= 64 more bytes, state unchanged, without
   // a snapshot: the chunk state is copied into words, the stack read in place, and a
   // chunk finished by the suffix (at most one) becomes a virtual top of the stack.
-  // The plain statement that the tests hold the incremental hasher against.
+  // The plain statement that the tests hold the incremental hasher against; the library's
+  // samples are drawn from a snapshot on the host and by one warp on the device.
   ZS_HD void finalize_suffix(const uint8_t* suf, unsigned n, uint32_t o[8]) const {
     uint32_t c[8], m[16], out[16], top[8];
     for (int i = 0; i < 8; ++i) c[i] = cv[i];

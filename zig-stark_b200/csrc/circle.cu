@@ -77,7 +77,7 @@ __global__ void k_twiddles(const __grid_constant__ TwJob j0, const __grid_consta
   for (unsigned t = a; t + 2 < lg; ++t) pt = pdbl(pt);
   const uint32_t x = pt.x, xi = j.itw ? minv(x) : 0;
   put(half + off, x, xi);
-  if (a + 2 == lg && lg > 2) {
+  if (a + 2 == lg && lg > 2) {  // the pattern that circle_layer32 relies on, in both tables
     const uint32_t k4 = 2 * (off & ~1u);
     if (off & 1) {
       put(k4, x, xi);
@@ -228,7 +228,8 @@ __device__ __forceinline__ void chunk_dispatch(unsigned r, uint32_t* s, uint32_t
 
 // C consecutive twiddles from T into registers, as 16- or 8-byte loads where C allows
 // (a chunk's twiddle run for layer i starts at TW[n - (n >> i) + Vh * C], a multiple of
-// C words from a 256-byte-aligned table, so the vector loads are aligned).
+// C words from the table; the tables of the sizes that take this path, 2^10 points and more,
+// lie at multiples of 4 KB from a 256-byte-aligned block, so the vector loads are aligned).
 template <int C>
 __device__ __forceinline__ void load_twiddles(uint32_t* dst, const uint32_t* __restrict__ T) {
   if constexpr (C >= 4) {
@@ -286,8 +287,8 @@ __device__ __forceinline__ void chunk_layers(uint32_t* v, const uint32_t* __rest
 // The circle layer (global layer 0) on 32 values in registers whose twiddles at layer 0
 // start at block 16 Vh, with the first line layer's eight twiddles t1 = T_1[8 Vh ..]. A
 // table of lg >= 3 holds at layer-0 entries 4k .. 4k + 3 the values f1, -f1, -f0, f0 of
-// its layer-1 entries f0 = T_1[2k], f1 = T_1[2k + 1] (k_tw_circle_layer; the inverse
-// table, elementwise inverses, keeps the pattern), so layer 0 needs no loads of its own:
+// its layer-1 entries f0 = T_1[2k], f1 = T_1[2k + 1] (k_twiddles; the inverse table,
+// elementwise inverses, keeps the pattern), so layer 0 needs no loads of its own:
 // a butterfly with the negated twiddle swaps its two outputs (forward) or the operands
 // of its subtraction (inverse), and gives the same canonical values.
 template <bool INV>

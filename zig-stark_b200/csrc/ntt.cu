@@ -48,8 +48,6 @@ ZS_HD qm31 to_crt(const qm31& x) {
   const cm31 bs = {mshl(madd(x.b.a, x.b.b), 15), mshl(msub(x.b.b, x.b.a), 15)};
   return {cadd(x.a, bs), cconj(csub(x.a, bs))};
 }
-// Products with the 4th root i and its inverse, and with the 8th root (1 + i) 2^15 and its
-// inverse (1 - i) 2^15 (the first component's; the second's have the other sign).
 // x t for a twiddle held doubled, T = 2 t (both words below 2^32): the sums of two products
 // are 2 v < 2^64, whose high word is at >> 31 and at most 2p, and whose low word is 2 (v & p).
 // Three ALU operations a word against seven for three reduced products and their sums.
@@ -65,6 +63,8 @@ __device__ __forceinline__ cm31 mul_tw(cm31 x, cm31 T) {
   return {fold2((uint64_t)x.a * T.a + (uint64_t)nb * T.b), fold2((uint64_t)x.a * T.b + (uint64_t)x.b * T.a)};
 }
 __device__ __forceinline__ qm31 twice(const qm31& v) { return qmake(v.a.a << 1, v.a.b << 1, v.b.a << 1, v.b.b << 1); }
+// Products with the 4th root i and its inverse, and with the 8th root (1 + i) 2^15 and its
+// inverse (1 - i) 2^15 (the first component's; the second's have the other sign).
 __device__ __forceinline__ cm31 mul_w4(cm31 x) { return {P - x.b, x.a}; }
 __device__ __forceinline__ cm31 mul_w4i(cm31 x) { return {x.b, P - x.a}; }
 __device__ __forceinline__ uint32_t rot15(uint32_t x) { return ((x << 15) | (x >> 16)) & P; }  // x 2^15

@@ -6,8 +6,8 @@
 
 namespace zs {
 
-// Powers of a primitive 2^log_n-th root w (qm31.zig:86-89): fwd[k] = w^k and
-// inv[k] = w^-k for k < 2^(log_n-1).
+// Powers of a primitive 2^log_n-th root w (qm31.zig:86-89) and of its inverse, for
+// k < 2^(log_n-1).
 struct NttTables {
   unsigned log_n = 0;
   qm31* fwd = nullptr;      // w^k, k < n/2 (QM31; the domain points of D)
