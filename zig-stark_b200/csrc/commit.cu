@@ -263,7 +263,7 @@ void CommitPlan::drop_graph() {
 }
 
 // The whole step is one CUDA graph (35 launches for 64 columns of 2^20 at blowup 4 with 16
-// folds, 8 for 8 of 2^10 with 6), captured on the plan's own stream and replayed on the
+// folds, 7 for 8 of 2^10 with 6), captured on the plan's own stream and replayed on the
 // caller's; it is recaptured when the trace pointer or the challenges change.
 void CommitPlan::run(const uint32_t* d_trace, cudaStream_t st) {
   if (!d_trace) d_trace = trace;
