@@ -463,12 +463,15 @@ __device__ __forceinline__ void sc_step(StepShared& s, const ScStep& st, uint32_
 // The end of a values kernel: the CTA's accumulators (`words` words in shared memory) go to
 // `out`; with a step to take, the CTA that is the last to do so takes it and clears `out`
 // for the next round.
-template <bool WIDE>
-__device__ __forceinline__ void finish_values(const uint32_t* s_acc, uint32_t words, uint32_t* out, const ScStep& st,
-                                              const Tower& F) {
+__device__ __forceinline__ void add_values(const uint32_t* s_acc, uint32_t words, uint32_t* out) {
   __syncthreads();
   for (uint32_t k = threadIdx.x; k < words; k += blockDim.x)
     if (s_acc[k]) atomicXor(out + k, s_acc[k]);
+}
+template <bool WIDE>
+__device__ __forceinline__ void finish_values(const uint32_t* s_acc, uint32_t words, uint32_t* out, const ScStep& st,
+                                              const Tower& F) {
+  add_values(s_acc, words, out);
   if (!st.tx) return;
   __shared__ StepShared s;
   __shared__ bool s_last;
@@ -503,9 +506,14 @@ struct Folding {
 // values[t]). D > 0: the D = dmax + 1 points in registers, every row once. D = 0: one
 // point per pass, points t = blockIdx.y, blockIdx.y + gridDim.y, ... (a grid of dmax + 1
 // rows of CTAs gives each point its own CTAs when the rows alone cannot fill the GPU).
+// PROVER: a proof's round, overlapped with its neighbours and with the step at its end. The
+// values alone (the hook and the round on tables in device memory) are instances without it:
+// the step's registers, shared memory and code cost them a microsecond a call otherwise (2^12
+// rows at four points 8.5 against 7.5 us, 2^20 rows 14.6 against 13.1).
 // `cur` is not __restrict__: in a prover's overlapped rounds the launch before may still be
 // writing it when this one's CTAs come up, so its loads must not take the read-only path.
-template <int D, bool FOLD>
+enum Round : int { kValuesOnly = 0, kRound = 1, kFoldRound = 2 };
+template <int D, int ROUND>
 __global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* cur, uint32_t len, uint32_t half,
                                                        uint32_t dmax, const __grid_constant__ Terms tm,
                                                        const uint8_t* __restrict__ gT, uint32_t* __restrict__ out,
@@ -515,10 +523,11 @@ __global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* cur, uint3
   uint8_t* s_T = reinterpret_cast<uint8_t*>(smem_b);
   uint32_t* s_acc = reinterpret_cast<uint32_t*>(s_T + 65536);
   const uint32_t words = (dmax + 4) / 4;
-  let_next_start();
+  constexpr bool PROVER = ROUND != kValuesOnly, FOLD = ROUND == kFoldRound;
+  if (PROVER) let_next_start();
   load_table(s_T, gT);
   for (uint32_t k = threadIdx.x; k < words; k += blockDim.x) s_acc[k] = 0;
-  after_previous();
+  if (PROVER) after_previous();
   __syncthreads();
   const Tower F{s_T};
   // (a, b) of table f's row `row`; with FOLD from the four bytes they are folded from
@@ -606,7 +615,10 @@ __global__ void __launch_bounds__(kBThreads) k_values8(const uint8_t* cur, uint3
       warp_xor_into(acc << (8 * (t & 3)), s_acc + (t >> 2));
     }
   }
-  finish_values<false>(s_acc, words, out, step, F);
+  if constexpr (PROVER)
+    finish_values<false>(s_acc, words, out, step, F);
+  else
+    add_values(s_acc, words, out);
 }
 
 // 16 little-endian bytes
@@ -622,7 +634,10 @@ __device__ __forceinline__ g128 load_g128(const uint4* p) {
   return {(uint64_t)v.y << 32 | v.x, (uint64_t)v.w << 32 | v.z};
 }
 
-// GF(2^128) round; out: (dmax + 1) values of four little-endian words. D and `cur` as k_values8.
+// GF(2^128) round; out: (dmax + 1) values of four little-endian words. D and `cur` as k_values8. One
+// instance serves a prover's rounds and the values alone (step.tx null): without the step's code the
+// compiler's schedule is slower from six points on (2^20 rows at seven points 920 against 803 us)
+// and equal or up to 3 % faster below, and each instance adds a millisecond to the first call.
 template <int D>
 __global__ void __launch_bounds__(kBThreads, (D >= 1 && D <= 4) ? 2 : 1) k_values128(const uint4* cur, uint32_t len, uint32_t half,
                                                          uint32_t dmax, const __grid_constant__ Terms tm,
@@ -979,20 +994,25 @@ void check_rows(size_t len, size_t half, size_t dmax) {
   if (dmax > kMaxPoint) throw Error(ZS_EMALFORMED, "more than 256 points");
 }
 
-// The values kernels by point count (index D, 0 = one point per pass) and the shared
-// memory they are launched with at most: the table and the largest accumulator.
-template <bool FOLD>
+// The values kernels by point count (index D, 0 = one point per pass) and kind of round.
+template <int ROUND>
 const void* values8(int D) {
   static const void* const k[kRegPoints + 1] = {
-      (const void*)k_values8<0, FOLD>, (const void*)k_values8<1, FOLD>, (const void*)k_values8<2, FOLD>,
-      (const void*)k_values8<3, FOLD>, (const void*)k_values8<4, FOLD>, (const void*)k_values8<5, FOLD>,
-      (const void*)k_values8<6, FOLD>, (const void*)k_values8<7, FOLD>, (const void*)k_values8<8, FOLD>};
+      (const void*)k_values8<0, ROUND>, (const void*)k_values8<1, ROUND>, (const void*)k_values8<2, ROUND>,
+      (const void*)k_values8<3, ROUND>, (const void*)k_values8<4, ROUND>, (const void*)k_values8<5, ROUND>,
+      (const void*)k_values8<6, ROUND>, (const void*)k_values8<7, ROUND>, (const void*)k_values8<8, ROUND>};
   return k[D];
 }
 const void* const kValues128[kRegPoints + 1] = {
     (const void*)k_values128<0>, (const void*)k_values128<1>, (const void*)k_values128<2>,
     (const void*)k_values128<3>, (const void*)k_values128<4>, (const void*)k_values128<5>,
     (const void*)k_values128<6>, (const void*)k_values128<7>, (const void*)k_values128<8>};
+// The kernel of a round (GF(2^128): one for all, its folds are launches of their own).
+const void* values_kernel(bool wide, Round round, int D) {
+  if (wide) return kValues128[D];
+  return round == kValuesOnly ? values8<kValuesOnly>(D) : round == kRound ? values8<kRound>(D) : values8<kFoldRound>(D);
+}
+// The shared memory that they are launched with at most: the table and the largest accumulator.
 constexpr size_t kValuesSmem = 65536 + 16 * (kMaxPoint + 1);
 constexpr size_t kRoundTables = (size_t)40 << 10;  // of a chunk's tables: two CTAs per SM
 constexpr size_t kRoundSmem = 65536 + 16 * kProveMaxPoints + kRoundTables;
@@ -1003,7 +1023,7 @@ constexpr size_t kTailSmem = 65536 + kTailBytes + kTailBytes / 2 + 32;
 struct DeviceState {
   uint8_t* table = nullptr;
   int sms = 0;
-  int per_sm8[kRegPoints + 1] = {}, per_sm128[kRegPoints + 1] = {}, per_sm8f[kRegPoints + 1] = {};
+  int per_sm[2][3][kRegPoints + 1] = {};  // of values_kernel(wide, round, D)
 };
 std::mutex g_dev_mu;
 DeviceState g_dev[64];
@@ -1016,15 +1036,15 @@ const DeviceState& device_state(cudaStream_t st) {
   DeviceState& d = g_dev[dev];
   if (!d.table) {
     ZS_CUDA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
-    for (int D = 0; D <= kRegPoints; ++D) {
-      for (int w = 0; w < 3; ++w) {
-        const void* fn = w == 0 ? values8<false>(D) : w == 1 ? kValues128[D] : values8<true>(D);
-        int* per_sm = w == 0 ? &d.per_sm8[D] : w == 1 ? &d.per_sm128[D] : &d.per_sm8f[D];
-        ZS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kValuesSmem));
-        ZS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, kBThreads, kValuesSmem));
-        *per_sm = std::max(*per_sm, 1);
-      }
-    }
+    for (int wide = 0; wide < 2; ++wide)
+      for (Round round : {kValuesOnly, kRound, kFoldRound})
+        for (int D = 0; D <= kRegPoints; ++D) {
+          const void* fn = values_kernel(wide, round, D);
+          int* per_sm = &d.per_sm[wide][round][D];
+          ZS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kValuesSmem));
+          ZS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, kBThreads, kValuesSmem));
+          *per_sm = std::max(*per_sm, 1);
+        }
     ZS_CUDA(cudaFuncSetAttribute(k_mul_table128, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
     ZS_CUDA(cudaFuncSetAttribute(k_fold128, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
     ZS_CUDA(cudaFuncSetAttribute(k_fold128_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));
@@ -1056,7 +1076,8 @@ void values_async(bool wide, const void* d_cur, size_t len, size_t half, size_t 
   const size_t row_blocks = (half + kBThreads - 1) / kBThreads;
   const bool per_row = D > 0 && row_blocks >= (size_t)ds.sms;
   const int kd = per_row ? D : 0;
-  const size_t slots = (size_t)ds.sms * (wide ? ds.per_sm128[kd] : fold ? ds.per_sm8f[kd] : ds.per_sm8[kd]);
+  const Round round = !step.tx ? kValuesOnly : fold ? kFoldRound : kRound;
+  const size_t slots = (size_t)ds.sms * ds.per_sm[wide][round][kd];
   dim3 grid(1, 1);
   if (per_row) {
     grid.x = (unsigned)std::min(row_blocks, slots);
@@ -1070,7 +1091,7 @@ void values_async(bool wide, const void* d_cur, size_t len, size_t half, size_t 
   uint32_t* out = static_cast<uint32_t*>(d_out);
   Folding f = fold ? *fold : Folding{};
   void* args[] = {&cur, &L, &H, &M, const_cast<Terms*>(&tm), &T, &out, const_cast<ScStep*>(&step), &f};
-  const void* fn = wide ? kValues128[kd] : fold ? values8<true>(kd) : values8<false>(kd);
+  const void* fn = values_kernel(wide, round, kd);
   if (step.tx)  // a prover's round
     launch_overlapped(fn, grid, dim3(kBThreads), args, 65536 + 4 * words, st);
   else
