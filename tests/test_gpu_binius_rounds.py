@@ -103,3 +103,26 @@ def test_gf128_fold_by_the_table(orc, k, m, terms):
     bad = bytearray(rounds)
     bad[len(bad) // 2] ^= 1
     assert not orc.binius_verify(7, named, k, len(names), renamed, claimed, bytes(bad))
+
+
+@pytest.mark.parametrize("k,points", [(8, 5), (9, 8), (8, 9), (8, 17)])
+def test_gf128_rounds_of_many_points(orc, k, points):
+    """More than four points over GF(2^128): the fold has a launch of its own while the chunks of
+    a fused round would not fill the SMs."""
+    from zs_b200 import native
+    rng = np.random.default_rng(1400 + points)
+    tables = rng.bytes(2 * 16 << k)
+    terms = [([(j * j) % 2 for j in range(points - 1)], 77), ([1], 1 << 70), ([], 5)]
+    assert native.binius_prove_combination(128, tables, k, 2, terms) == orc.binius_prove(7, tables, k, 2, terms)
+
+
+def test_gf128_fused_rounds_of_many_points(orc):
+    """2^16 rows at six points: fused while the chunks fill the SMs, then not."""
+    from zs_b200 import native
+    tables = np.random.default_rng(1500).bytes(16 << 16)
+    terms = [([0] * 5, 9), ([0], 1)]
+    claimed, rounds = native.binius_prove_combination(128, tables, 16, 1, terms)
+    assert orc.binius_verify(7, tables, 16, 1, terms, claimed, rounds)
+    bad = bytearray(rounds)
+    bad[16 * 6 + 3] ^= 1
+    assert not orc.binius_verify(7, tables, 16, 1, terms, claimed, bytes(bad))

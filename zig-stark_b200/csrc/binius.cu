@@ -1309,6 +1309,14 @@ int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, 
     const uint8_t* d_r = aux + o_tx + offsetof(ScTranscript, r);
     // rows of a chunk of k_sc_round128: a warp's, or 64 for eight warps at four points
     const uint32_t chunk = m * 128 * es <= kRoundTables ? 64 : m * 64 * es <= kRoundTables ? 32 : 0;
+    // More points than four take their turns in a chunk's eight warps, where the values kernel
+    // gives each its own CTAs: while the chunks do not fill the SMs the latter is faster (three
+    // tables of 2^12 rows at 8 points 316 us against 373 fused, at 16 points 507 against 1034, at
+    // 21 points 648 against 2271; four points: equal, 194 us), and from there on the fused one
+    // (2^16 rows at 6 points 526 us against 562).
+    auto fused = [&](size_t l) {
+      return wide && chunk && m * l <= kFusedFold && (pts <= 4 || l / 2 >= (size_t)ds.sms * chunk);
+    };
     size_t len = n;
     bool pending = false;  // `cur` awaits the fold of the round before (it has 2 len elements)
     auto fold_now = [&] {
@@ -1329,7 +1337,7 @@ int32_t prove_combination(uint32_t field_bits, const uint8_t* tables, size_t k, 
                           dim3(kTailThreads), args, smem, st);
         break;
       }
-      if (pending && wide && m * len <= kFusedFold && chunk) {
+      if (pending && fused(len)) {
         const void* c = cur;
         uint32_t l = (uint32_t)len, mm = (uint32_t)m, R = chunk, *o = reinterpret_cast<uint32_t*>(aux + o_vals);
         Folding f{d_r, nxt};
