@@ -72,7 +72,7 @@ int32_t zs_binius_sumcheck_fold_device(uint32_t field_bits, const void *d_cur, s
  * transcript step, fold) runs on the device, and the host waits once, for the proof.
  * claimed_out: one element (the hypercube sum). rounds_out: k * (dmax + 1) elements, round
  * i's low-first coefficients at i * (dmax + 1), dmax = the longest term (dmax + 1 <= 64).
- * Synchronous. */
+ * Synchronous. The tables' device memory stays in the device's pool (zs_m31_prove). */
 int32_t zs_binius_sumcheck_prove_combination(uint32_t field_bits, const uint8_t *tables, size_t k, size_t m,
                                              const uint8_t *coeffs, size_t nterms, const uint32_t *indices,
                                              size_t n_indices, const uint32_t *offsets, const uint8_t *seed,

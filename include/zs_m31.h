@@ -76,7 +76,14 @@ enum {
  * (stark.zig:107-122), allocated with `host` and released with zs_free. The proof is
  * byte-identical to the reference prover's for the same inputs. Parameters the
  * reference asserts on (stark.zig:230-232, fri.zig:228) return -4; a domain above 2^26
- * points (trace_log + log_blowup > 26) or more than 2^24 queries returns -2. */
+ * points (trace_log + log_blowup > 26) or more than 2^24 queries returns -2.
+ *
+ * Memory: the first proof, column commitment or sum-check proof on a device sets the release
+ * threshold of its default stream-ordered pool to the maximum, so that what proofs free stays
+ * there for the next (cudaMemPoolTrimTo gives it back), and a proof's pinned staging buffers
+ * (32 MB for uploads of a megabyte and more, a few megabytes for small transfers) stay for the
+ * life of the process, one set for each proof that ran at the same time. The transforms and
+ * the commit plans keep neither. */
 int32_t zs_m31_prove(zs_host_allocator host, uint32_t air_id, const uint8_t *params, size_t params_len,
                      const uint8_t *public_inputs, size_t public_inputs_len, const uint8_t *preprocessed,
                      size_t preprocessed_len, const uint8_t *trace, size_t trace_len, const uint8_t *channel_sep,
@@ -212,7 +219,8 @@ int32_t zs_m31_circle_ifft(const uint32_t *evals, uint32_t n_columns, uint32_t o
  * of size 2^(log_rows + log_blowup) with the given fold challenges, each layer
  * committed with hashQM31 leaves before it is folded (fri.zig:195-220).
  *
- * A plan owns every device buffer of one configuration. Typical use:
+ * A plan owns every device buffer of one configuration, in use by one run at a time: order
+ * a plan's runs (one stream, or events). destroy gives its memory back. Typical use:
  *   create -> set_challenges -> (upload | run_device)* -> results -> destroy. */
 typedef struct zs_commit_plan zs_commit_plan;
 
