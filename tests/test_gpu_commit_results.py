@@ -1,4 +1,4 @@
-"""A commit plan's results where their copies change: final layers of up to 64 KB come back in
+"""A commit plan's results where their copies change: final layers of up to 256 KB come back in
 one copy with the roots, larger ones in their own; without folds; and with any output left out.
 Against the oracle."""
 import ctypes
@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n_cols,log_rows,log_blowup,n_folds", [
-    (3, 9, 2, 0), (3, 11, 2, 0), (2, 12, 1, 1), (2, 12, 2, 1), (5, 10, 2, 12), (1, 16, 1, 16)])
+    (3, 9, 2, 0), (2, 12, 1, 1), (2, 13, 1, 0), (1, 14, 1, 0), (2, 13, 2, 1), (5, 10, 2, 12), (1, 16, 1, 16)])
 def test_results_at_every_copy(orc, n_cols, log_rows, log_blowup, n_folds):
     from zs_b200 import native
     rng = np.random.default_rng(71 * log_rows + n_folds)
